@@ -188,7 +188,7 @@ __device__ __forceinline__ void bltc_near64_body(const TreeGeom& tg, int f, int 
     tz[r] = z[i];
     ax[r] = ay[r] = az[r] = 0;
   }
-  const double eps = tg.eps;
+  const double eps2 = twice_eps(tg.eps);
   for (int e = tg.near_start[f] + split; e < tg.near_start[f + 1]; e += nsplit) {
     const long sb = (long)tg.near_src[e] * npl;
     __syncthreads();
@@ -197,16 +197,7 @@ __device__ __forceinline__ void bltc_near64_body(const TreeGeom& tg, int f, int 
 #pragma unroll 8
     for (int k = 0; k < npl; k++) {
       const double4 s = tile[k];
-#pragma unroll
-      for (int r = 0; r < TPT; r++) {
-        double dx = s.x - tx[r], dy = s.y - ty[r], dz = s.z - tz[r];
-        double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-        double g = s.w * recip_nr(fma(0.5, r2, eps));
-        if (GUARD) g = r2 > 0.0 ? g : 0.0;
-        ax[r] = fma(g, dx, ax[r]);
-        ay[r] = fma(g, dy, ay[r]);
-        az[r] = fma(g, dz, az[r]);
-      }
+      pairs64<GUARD>(tx, ty, tz, s.x, s.y, s.z, s.w, eps2, ax, ay, az);
     }
   }
 #pragma unroll
@@ -214,9 +205,9 @@ __device__ __forceinline__ void bltc_near64_body(const TreeGeom& tg, int f, int 
     int k = threadIdx.x + r * NT;
     if (k >= npl) continue;
     long i = (long)f * npl + k;
-    v[i] = kBiotSavart * (ty[r] * az[r] - tz[r] * ay[r]);
-    v[tg.N + i] = kBiotSavart * (tz[r] * ax[r] - tx[r] * az[r]);
-    v[2 * tg.N + i] = kBiotSavart * (tx[r] * ay[r] - ty[r] * ax[r]);
+    v[i] = kBiotSavartTwice * (ty[r] * az[r] - tz[r] * ay[r]);
+    v[tg.N + i] = kBiotSavartTwice * (tz[r] * ax[r] - tx[r] * az[r]);
+    v[2 * tg.N + i] = kBiotSavartTwice * (tx[r] * ay[r] - ty[r] * ax[r]);
   }
 }
 

@@ -223,6 +223,7 @@ __global__ void __launch_bounds__(NT)
     }
     ax[r] = ay[r] = az[r] = bx[r] = by[r] = bz[r] = 0;
   }
+  const double deps2 = twice_eps(tg.eps);
   const float feps = (float)tg.eps;
   const int hq = (gq + 1) / 2, ngl = npl / gq, np2 = ngl * hq;
   for (int e = tg.near_start[f] + split; e < tg.near_start[f + 1]; e += nsplit) {
@@ -311,15 +312,12 @@ __global__ void __launch_bounds__(NT)
 #pragma unroll 4
       for (int k = 0; k < npl; k++) {
         const double4 s1 = t1[k], s2 = t2[k];
-#pragma unroll
-        for (int r = 0; r < TPT; r++) {
-          pair64<GUARD>(tx[r], ty[r], tz[r], s1, tg.eps, ax[r], ay[r], az[r]);
-          pair64<GUARD>(tx[r], ty[r], tz[r], s2, tg.eps, bx[r], by[r], bz[r]);
-        }
+        pairs64<GUARD>(tx, ty, tz, s1.x, s1.y, s1.z, s1.w, deps2, ax, ay, az);
+        pairs64<GUARD>(tx, ty, tz, s2.x, s2.y, s2.z, s2.w, deps2, bx, by, bz);
       }
     }
   }
-  constexpr double K = MIXED ? kBiotSavartPacked : kBiotSavart;
+  constexpr double K = MIXED ? kBiotSavartPacked : kBiotSavartTwice;
 #pragma unroll
   for (int r = 0; r < TPT; r++) {
     const int k = threadIdx.x + r * NT;

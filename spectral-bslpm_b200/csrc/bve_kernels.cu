@@ -17,6 +17,7 @@
 #include "../../include/sbslpm.h"
 #include "bve_kernels.cuh"
 #include "device_common.cuh"
+#include "list64.cuh"
 
 namespace sbslpm {
 
@@ -365,149 +366,27 @@ __global__ void k_downward_subtree_batch(const BatchMember* __restrict__ mem, in
 template <int Q>
 struct WarpShape {
   static constexpr int S = Q <= 16 ? 32 / Q : 1;          // source splits per warp
-  static constexpr int STAGE = (S * Q > Q ? S * Q : Q);    // staged points per warp
   static constexpr int Q2 = (Q + 1) / 2;                    // source pairs per panel
   static constexpr int STAGE2 = (S > 1 ? S : 1) * 2 * Q2;   // float4 slots per warp, paired layout
 };
 
-template <int Q, bool ALL_LEAVES, bool GUARD>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock) k_interact64(StepGeom g, const double4* __restrict__ src,
-                                                                    double* __restrict__ out, long out_stride) {
-  using W = WarpShape<Q>;
-  __shared__ double4 stage[kWarpsPerBlock][W::STAGE];
-  __shared__ double red[kWarpsPerBlock][3][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tp_first = ALL_LEAVES ? g.offset : 0;
-  const int tp_count = ALL_LEAVES ? g.leaves : g.panels;
-  const int tix = blockIdx.x * kWarpsPerBlock + warp;
-  if (tix >= tp_count) return;
-  const int t = tp_first + tix;
-  const long pn = (long)g.panels * g.q;
-
-  int e0, e1;
-  if (ALL_LEAVES) {
-    int per = (g.leaves + gridDim.y - 1) / gridDim.y;
-    e0 = blockIdx.y * per;
-    e1 = min(g.leaves, e0 + per);
-  } else {
-    e0 = g.tgt_start[t];
-    e1 = g.tgt_start[t + 1];
-  }
-  auto source_of = [&](int e) { return ALL_LEAVES ? g.offset + e : __ldg(g.src_panel + e); };
-
-  if constexpr (Q <= 32) {
-    const int h = lane / Q, j = lane % Q;
-    const bool active = h < W::S;
-    double tx = 0, ty = 0, tz = 0;
-    if (active) {
-      long o = (long)t * Q + j;
-      tx = g.px[o];
-      ty = g.px[pn + o];
-      tz = g.px[2 * pn + o];
-    }
-    double ax = 0, ay = 0, az = 0;
-    if constexpr (ALL_LEAVES) {
-      for (int e = e0; e < e1; e += W::S) {
-        if (active && e + h < e1) stage[warp][h * Q + j] = src[(long)source_of(e + h) * Q + j];
-        __syncwarp();
-        if (active && e + h < e1) {
-          const double4* sp = &stage[warp][h * Q];
-#pragma unroll
-          for (int k = 0; k < Q; k++) pair64<GUARD>(tx, ty, tz, sp[k], g.eps, ax, ay, az);
-        }
-        __syncwarp();
-      }
-    } else {
-      // the list in batches of 32 entries, one source index per lane, handed
-      // to the splits by shuffles; the next entry's sources are loaded while
-      // the current ones are evaluated
-      for (int eb = e0; eb < e1; eb += 32) {
-        const int nb = min(32, e1 - eb);
-        const int idx = lane < nb ? __ldg(g.src_panel + eb + lane) : 0;
-        const int iters = (nb + W::S - 1) / W::S;
-        double4 sv = make_double4(0, 0, 0, 0);
-        {
-          const int sp = __shfl_sync(0xffffffffu, idx, h & 31);
-          if (active && h < nb) sv = src[(long)sp * Q + j];
-        }
-        for (int it = 0; it < iters; it++) {
-          const bool on = active && it * W::S + h < nb;
-          const int ns = (it + 1) * W::S + h;
-          const int sp_n = __shfl_sync(0xffffffffu, idx, ns & 31);
-          double4 sv_n = make_double4(0, 0, 0, 0);
-          if (active && ns < nb) sv_n = src[(long)sp_n * Q + j];
-          if (on) stage[warp][h * Q + j] = sv;
-          __syncwarp();
-          if (on) {
-            const double4* sp = &stage[warp][h * Q];
-#pragma unroll
-            for (int k = 0; k < Q; k++) pair64<GUARD>(tx, ty, tz, sp[k], g.eps, ax, ay, az);
-          }
-          __syncwarp();
-          sv = sv_n;
-        }
-      }
-    }
-    if (W::S > 1) {
-      red[warp][0][lane] = ax;
-      red[warp][1][lane] = ay;
-      red[warp][2][lane] = az;
-      __syncwarp();
-      if (h == 0) {
-        for (int hh = 1; hh < W::S; hh++) {
-          ax += red[warp][0][hh * Q + j];
-          ay += red[warp][1][hh * Q + j];
-          az += red[warp][2][hh * Q + j];
-        }
-      }
-    }
-    if (h == 0) {
-      double ux = kBiotSavart * (ty * az - tz * ay);
-      double uy = kBiotSavart * (tz * ax - tx * az);
-      double uz = kBiotSavart * (tx * ay - ty * ax);
-      long o = ALL_LEAVES ? (long)blockIdx.y * 3 * out_stride + (long)tix * Q + j : (long)t * Q + j;
-      long s = ALL_LEAVES ? out_stride : pn;
-      out[o] = ux;
-      out[s + o] = uy;
-      out[2 * s + o] = uz;
-    }
-  } else {
-    constexpr int TPL = Q <= 32 ? 1 : (Q + 31) / 32;  // target nodes per lane
-    double tx[TPL], ty[TPL], tz[TPL], ax[TPL], ay[TPL], az[TPL];
-#pragma unroll
-    for (int r = 0; r < TPL; r++) {
-      int j = lane + 32 * r;
-      long o = (long)t * Q + (j < Q ? j : 0);
-      tx[r] = g.px[o];
-      ty[r] = g.px[pn + o];
-      tz[r] = g.px[2 * pn + o];
-      ax[r] = ay[r] = az[r] = 0;
-    }
-    for (int e = e0; e < e1; e++) {
-      const long sb = (long)source_of(e) * Q;
-      for (int k = lane; k < Q; k += 32) stage[warp][k] = src[sb + k];
-      __syncwarp();
-      for (int k = 0; k < Q; k++) {
-        const double4 s = stage[warp][k];
-#pragma unroll
-        for (int r = 0; r < TPL; r++) pair64<GUARD>(tx[r], ty[r], tz[r], s, g.eps, ax[r], ay[r], az[r]);
-      }
-      __syncwarp();
-    }
-#pragma unroll
-    for (int r = 0; r < TPL; r++) {
-      int j = lane + 32 * r;
-      if (j >= Q) continue;
-      double ux = kBiotSavart * (ty[r] * az[r] - tz[r] * ay[r]);
-      double uy = kBiotSavart * (tz[r] * ax[r] - tx[r] * az[r]);
-      double uz = kBiotSavart * (tx[r] * ay[r] - ty[r] * ax[r]);
-      long o = ALL_LEAVES ? (long)blockIdx.y * 3 * out_stride + (long)tix * Q + j : (long)t * Q + j;
-      long s = ALL_LEAVES ? out_stride : pn;
-      out[o] = ux;
-      out[s + o] = uy;
-      out[2 * s + o] = uz;
-    }
-  }
+// Float64, q <= 25 (list64.cuh).
+template <int Q, int WPT, bool ALL_LEAVES, bool GUARD>
+__global__ void __launch_bounds__(32 * ListShape<Q, 1>::NW)
+    k_interact64(StepGeom g, const double4* __restrict__ src, double* __restrict__ out, long out_stride) {
+  using W = ListShape<Q, 1>;
+  __shared__ __align__(16) double2 tiles[W::NW * W::WARP];
+  const long pn = (long)g.panels * Q;
+  list64_sweep<Q, 1, WPT, ALL_LEAVES, GUARD>(
+      g, src, nullptr, tiles, [&](int t, int tix, int j, const double* a) {
+        const long i = (long)t * Q + j;
+        const double x = g.px[i], y = g.px[pn + i], z = g.px[2 * pn + i];
+        const long o = ALL_LEAVES ? (long)blockIdx.y * 3 * out_stride + (long)tix * Q + j : i;
+        const long s = ALL_LEAVES ? out_stride : pn;
+        out[o] = kBiotSavartTwice * (y * a[2] - z * a[1]);
+        out[s + o] = kBiotSavartTwice * (z * a[0] - x * a[2]);
+        out[2 * s + o] = kBiotSavartTwice * (x * a[1] - y * a[0]);
+      });
 }
 
 // Mixed precision: positions relative to panel centres in float, pair
@@ -696,61 +575,6 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_interact32(StepGeom g, 
       out[s + o] = kBiotSavartPacked * (tz * ax - tx * az);
       out[2 * s + o] = kBiotSavartPacked * (tx * ay - ty * ax);
     }
-  } else {
-    constexpr int TPL = Q <= 32 ? 1 : (Q + 31) / 32;  // target nodes per lane
-    double tx[TPL], ty[TPL], tz[TPL], ax[TPL], ay[TPL], az[TPL];
-    float dtx[TPL], dty[TPL], dtz[TPL];
-#pragma unroll
-    for (int r = 0; r < TPL; r++) {
-      int j = lane + 32 * r;
-      long o = (long)t * Q + (j < Q ? j : 0);
-      tx[r] = g.px[o];
-      ty[r] = g.px[pn + o];
-      tz[r] = g.px[2 * pn + o];
-      dtx[r] = (float)((tx[r] - ctx) * kPackScale);
-      dty[r] = (float)((ty[r] - cty) * kPackScale);
-      dtz[r] = (float)((tz[r] - ctz) * kPackScale);
-      ax[r] = ay[r] = az[r] = 0;
-    }
-    for (int e = e0; e < e1; e++) {
-      const int sp = ALL_LEAVES ? g.offset + e : __ldg(g.src_panel + e);
-      const long sb = (long)sp * Q;
-      for (int k = lane; k < Q; k += 32) stage[warp][k] = srcf[sb + k];
-      const double* cs = g.pd_centre + 4 * (long)sp;
-      const float bx0 = (float)((cs[0] - ctx) * kPackScale), by0 = (float)((cs[1] - cty) * kPackScale),
-                  bz0 = (float)((cs[2] - ctz) * kPackScale);
-      float fx[TPL], fy[TPL], fz[TPL], bx[TPL], by[TPL], bz[TPL];
-#pragma unroll
-      for (int r = 0; r < TPL; r++) {
-        fx[r] = fy[r] = fz[r] = 0.f;
-        bx[r] = bx0 - dtx[r];
-        by[r] = by0 - dty[r];
-        bz[r] = bz0 - dtz[r];
-      }
-      __syncwarp();
-      for (int k = 0; k < Q; k++) {
-        const float4 s = stage[warp][k];
-#pragma unroll
-        for (int r = 0; r < TPL; r++) pair32<GUARD>(bx[r], by[r], bz[r], s, eps, fx[r], fy[r], fz[r]);
-      }
-#pragma unroll
-      for (int r = 0; r < TPL; r++) {
-        ax[r] += fx[r];
-        ay[r] += fy[r];
-        az[r] += fz[r];
-      }
-      __syncwarp();
-    }
-#pragma unroll
-    for (int r = 0; r < TPL; r++) {
-      int j = lane + 32 * r;
-      if (j >= Q) continue;
-      long o = ALL_LEAVES ? (long)blockIdx.y * 3 * out_stride + (long)tix * Q + j : (long)t * Q + j;
-      long s = ALL_LEAVES ? out_stride : pn;
-      out[o] = kBiotSavartPacked * (ty[r] * az[r] - tz[r] * ay[r]);
-      out[s + o] = kBiotSavartPacked * (tz[r] * ax[r] - tx[r] * az[r]);
-      out[2 * s + o] = kBiotSavartPacked * (tx[r] * ay[r] - ty[r] * ax[r]);
-    }
   }
 }
 
@@ -923,6 +747,7 @@ __device__ __forceinline__ void interact_wide_body(const StepGeom& g, int tix, i
     ax[r] = ay[r] = az[r] = 0;
   }
   const float feps = (float)g.eps;
+  const double eps2 = twice_eps(g.eps);
   for (int e = e0 + warp; e < e1; e += NW) {
     const int sp = ALL_LEAVES ? g.offset + e : __ldg(g.src_panel + e);
     const long sb = (long)sp * Q;
@@ -970,8 +795,7 @@ __device__ __forceinline__ void interact_wide_body(const StepGeom& g, int tix, i
 #pragma unroll 3
       for (int k = 0; k < Q; k++) {
         const double4 s = stage[warp][k];
-#pragma unroll
-        for (int r = 0; r < TPL; r++) pair64<GUARD>(tx[r], ty[r], tz[r], s, g.eps, ax[r], ay[r], az[r]);
+        pairs64<GUARD>(tx, ty, tz, s.x, s.y, s.z, s.w, eps2, ax, ay, az);
       }
     }
     __syncwarp();
@@ -986,7 +810,7 @@ __device__ __forceinline__ void interact_wide_body(const StepGeom& g, int tix, i
     }
   }
   __syncthreads();
-  const double cb = MIXED ? kBiotSavartPacked : kBiotSavart;
+  const double cb = MIXED ? kBiotSavartPacked : kBiotSavartTwice;
   for (int j = threadIdx.x; j < Q; j += blockDim.x) {
     double sx = red[0][0][j], sy = red[0][1][j], sz = red[0][2][j];
     for (int w = 1; w < NW; w++) {
@@ -1161,19 +985,20 @@ __global__ void __launch_bounds__(kDirectThreads)
   long per = (ns + gridDim.y - 1) / gridDim.y;
   long s0 = blockIdx.y * per, s1 = min(ns, s0 + per);
   double ax = 0, ay = 0, az = 0;
+  const double eps2 = twice_eps(eps);
   for (long b = s0; b < s1; b += kDirectThreads) {
     long k = b + threadIdx.x;
     tile[threadIdx.x] = k < s1 ? make_double4(sx[k], sy[k], sz[k], sw[k]) : make_double4(0, 0, 0, 0);
     __syncthreads();
     int cnt = (int)min((long)kDirectThreads, s1 - b);
-    for (int m = 0; m < cnt; m++) pair64<true>(x, y, z, tile[m], eps, ax, ay, az);
+    for (int m = 0; m < cnt; m++) pair64<true>(x, y, z, tile[m], eps2, ax, ay, az);
     __syncthreads();
   }
   if (i < nt) {
     long o = (long)blockIdx.y * 3 * nt + i;
-    partial[o] = kBiotSavart * (y * az - z * ay);
-    partial[nt + o] = kBiotSavart * (z * ax - x * az);
-    partial[2 * nt + o] = kBiotSavart * (x * ay - y * ax);
+    partial[o] = kBiotSavartTwice * (y * az - z * ay);
+    partial[nt + o] = kBiotSavartTwice * (z * ax - x * az);
+    partial[2 * nt + o] = kBiotSavartTwice * (x * ay - y * ax);
   }
 }
 
@@ -1428,24 +1253,31 @@ void interact_qg(const StepGeom& g, int precision, const double4* src, double* o
       if (all_leaves) SB_LAUNCH((k_interact_wide<Q, true, GUARD, false>), wgrid, 128, 0, st, g, src, g.srcf, out, out_stride);
       else SB_LAUNCH((k_interact_wide<Q, false, GUARD, false>), wgrid, 128, 0, st, g, src, g.srcf, out, out_stride);
     }
-    return;
+  } else {
+    const int threads = 32 * kWarpsPerBlock;
+    if (precision == SBSLPM_MIXED) {
+      const dim3 grid(blocks_for(tp, kWarpsPerBlock), all_leaves ? groups : 1);
+      if (pack) SB_LAUNCH(k_pack_mixed, blocks_for((long)g.panels * g.q, 256), 256, 0, st, g, src, g.srcf);
+      if (all_leaves)
+        SB_LAUNCH((k_interact32<Q, true, GUARD>), grid, threads, 0, st, g, g.srcf, out, out_stride);
+      else if constexpr (Q == 16)
+        SB_LAUNCH((k_interact32_q16<GUARD>), grid, threads, 0, st, g, g.srcf, out);
+      else
+        SB_LAUNCH((k_interact32<Q, false, GUARD>), grid, threads, 0, st, g, g.srcf, out, out_stride);
+    } else {
+      constexpr int NW = dev::ListShape<Q, 1>::NW, threads64 = 32 * NW;
+      const int wpt = dev::list_warps<Q, 1>(tp);
+      if (all_leaves)
+        SB_LAUNCH((k_interact64<Q, 1, true, GUARD>), dim3(blocks_for(tp, NW), groups), threads64, 0, st, g, src, out,
+                  out_stride);
+      else if (wpt == NW)
+        SB_LAUNCH((k_interact64<Q, NW, false, GUARD>), tp, threads64, 0, st, g, src, out, out_stride);
+      else if (wpt == 2)
+        SB_LAUNCH((k_interact64<Q, 2, false, GUARD>), blocks_for(tp, NW / 2), threads64, 0, st, g, src, out, out_stride);
+      else
+        SB_LAUNCH((k_interact64<Q, 1, false, GUARD>), blocks_for(tp, NW), threads64, 0, st, g, src, out, out_stride);
+    }
   }
-  dim3 grid(blocks_for(tp, kWarpsPerBlock), all_leaves ? groups : 1);
-  if (precision == SBSLPM_MIXED) {
-    long pn = (long)g.panels * g.q;
-    if (pack) SB_LAUNCH(k_pack_mixed, blocks_for(pn, 256), 256, 0, st, g, src, g.srcf);
-    if (all_leaves)
-      SB_LAUNCH((k_interact32<Q, true, GUARD>), grid, 32 * kWarpsPerBlock, 0, st, g, g.srcf, out, out_stride);
-    else if constexpr (Q == 16)
-      SB_LAUNCH((k_interact32_q16<GUARD>), grid, 32 * kWarpsPerBlock, 0, st, g, g.srcf, out);
-    else
-      SB_LAUNCH((k_interact32<Q, false, GUARD>), grid, 32 * kWarpsPerBlock, 0, st, g, g.srcf, out, out_stride);
-    return;
-  }
-  if (all_leaves)
-    SB_LAUNCH((k_interact64<Q, true, GUARD>), grid, 32 * kWarpsPerBlock, 0, st, g, src, out, out_stride);
-  else
-    SB_LAUNCH((k_interact64<Q, false, GUARD>), grid, 32 * kWarpsPerBlock, 0, st, g, src, out, out_stride);
 }
 
 // The coincident-point guard is compiled in only when kernel_eps = 0.

@@ -475,6 +475,7 @@ __global__ void __launch_bounds__(CcShape<Q, S>::NT)
     tz = g.px[2 * pn + o];
   }
   double ax = 0, ay = 0, az = 0;
+  const double eps2 = dev::twice_eps(g.eps);
   for (int e = 0; e < nmax; e++) {
     const bool act = live && e < n;
     __syncthreads();
@@ -483,7 +484,7 @@ __global__ void __launch_bounds__(CcShape<Q, S>::NT)
     if (act) {
       const double4* tb = tile[h];
 #pragma unroll 3
-      for (int k = 0; k < Q; k++) pair64<GUARD>(tx, ty, tz, tb[k], g.eps, ax, ay, az);
+      for (int k = 0; k < Q; k++) pair64<GUARD>(tx, ty, tz, tb[k], eps2, ax, ay, az);
     }
   }
   if (live) {
@@ -828,7 +829,7 @@ void launch_cc_chunks(const StepGeom& g, int precision, int slots, const int4* c
   }
   const long pn = (long)g.panels * g.q;
   SB_LAUNCH(k_cc_reduce, blocks_for(pn, 256), 256, 0, st, g, cstart, partial,
-            mixed ? kBiotSavartPacked : kBiotSavart, out);
+            mixed ? kBiotSavartPacked : kBiotSavartTwice, out);
 }
 
 void launch_cc_multi(const CcTcGroup& g, cudaStream_t st) {

@@ -21,6 +21,8 @@ constexpr int kMaxDegree = 10;
 constexpr int kMaxQ = (kMaxDegree + 1) * (kMaxDegree + 1);
 // -1/(4 pi), the Biot-Savart constant (src/fmm_interactions/bve_vel_impl.hpp:115)
 constexpr double kBiotSavart = -0.07957747154594767;
+// its double, for sums taken with the denominator |d|^2 + 2 eps
+constexpr double kBiotSavartTwice = 2.0 * kBiotSavart;
 
 // Error bits reported by device code through the context's error word.
 enum : unsigned { kErrOutOfPanel = 1u, kErrNonFinite = 2u, kErrBadFace = 4u, kErrTimeout = 8u };

@@ -18,6 +18,7 @@
 
 #include "../../include/sbslpm.h"
 #include "device_common.cuh"
+#include "list64.cuh"
 #include "swe_kernels.cuh"
 
 namespace sbslpm {
@@ -300,7 +301,8 @@ __global__ void __launch_bounds__(32 * kWarps)
   }
   const double* ct = g.pd_centre + 4 * (long)t;
   const float eps32 = (float)g.eps;
-  constexpr double K = MIXED ? kBiotSavartPacked : kBiotSavart;
+  const double deps2 = twice_eps(g.eps);
+  constexpr double K = MIXED ? kBiotSavartPacked : kBiotSavartTwice;
   constexpr int TPL = W::TPL;
   const int h = Q <= 32 ? lane / Q : 0;
   const bool active = Q <= 32 ? h < W::S : true;
@@ -392,11 +394,8 @@ __global__ void __launch_bounds__(32 * kWarps)
 #pragma unroll 4
         for (int k = 0; k < Q; k++) {
           const double4 v1 = st1[k], v2 = st2[k];
-#pragma unroll
-          for (int r = 0; r < TPL; r++) {
-            pair64<GUARD>(tx[r], ty[r], tz[r], v1, g.eps, ax[r], ay[r], az[r]);
-            pair64<GUARD>(tx[r], ty[r], tz[r], v2, g.eps, bx[r], by[r], bz[r]);
-          }
+          pairs64<GUARD>(tx, ty, tz, v1.x, v1.y, v1.z, v1.w, deps2, ax, ay, az);
+          pairs64<GUARD>(tx, ty, tz, v2.x, v2.y, v2.z, v2.w, deps2, bx, by, bz);
         }
       }
     }
@@ -436,6 +435,28 @@ __global__ void __launch_bounds__(32 * kWarps)
     out[s + o] = uy;
     out[2 * s + o] = uz;
   }
+}
+
+// Float64, q <= 25: both fields by list64.cuh.
+template <int Q, int WPT, bool ALL_LEAVES, bool GUARD>
+__global__ void __launch_bounds__(32 * ListShape<Q, 2>::NW)
+    k_swe_interact64(StepGeom g, const double4* __restrict__ src, const double4* __restrict__ src2,
+                     double* __restrict__ out, long out_stride) {
+  using W = ListShape<Q, 2>;
+  __shared__ __align__(16) double2 tiles[W::NW * W::WARP];
+  const long pn = (long)g.panels * Q;
+  list64_sweep<Q, 2, WPT, ALL_LEAVES, GUARD>(
+      g, src, src2, tiles, [&](int t, int tix, int j, const double* a) {
+        const long i = (long)t * Q + j;
+        double ux, uy, uz;
+        swe_epilogue(kBiotSavartTwice, g.px[i], g.px[pn + i], g.px[2 * pn + i], a[0], a[1], a[2], a[3], a[4], a[5],
+                     ux, uy, uz);
+        const long o = ALL_LEAVES ? (long)blockIdx.y * 3 * out_stride + (long)tix * Q + j : i;
+        const long s = ALL_LEAVES ? out_stride : pn;
+        out[o] = ux;
+        out[s + o] = uy;
+        out[2 * s + o] = uz;
+      });
 }
 
 // Mixed precision, q <= 32, list mode: the BVE list kernel's organisation
@@ -601,17 +622,31 @@ void swe_interact_qg(const StepGeom& g, const SweGeom& s, int precision, const d
   const bool mixed = precision == SBSLPM_MIXED;
 #define SB_SWE_K(AL, MX) \
   SB_LAUNCH((k_swe_interact<Q, AL, GUARD, MX>), grid, 32 * kWarps, 0, st, g, s, src, src2, out, out_stride)
-  if (all_leaves) {
-    if (mixed) SB_SWE_K(true, true);
-    else SB_SWE_K(true, false);
-  } else {
+  if (mixed) {
     if constexpr (Q <= 32) {
-      if (mixed && g.entry) {
+      if (!all_leaves && g.entry) {
         SB_LAUNCH((k_swe_interact32_list<Q, GUARD>), grid, 32 * kWarps, 0, st, g, s, out);
         return;
       }
     }
-    if (mixed) SB_SWE_K(false, true);
+    if (all_leaves) SB_SWE_K(true, true);
+    else SB_SWE_K(false, true);
+  } else if constexpr (Q <= 32) {
+    constexpr int NW = ListShape<Q, 2>::NW, threads = 32 * NW;
+    const int wpt = dev::list_warps<Q, 2>(tp);
+    if (all_leaves)
+      SB_LAUNCH((k_swe_interact64<Q, 1, true, GUARD>), dim3(blocks_for(tp, NW), groups), threads, 0, st, g, src, src2,
+                out, out_stride);
+    else if (wpt == NW)
+      SB_LAUNCH((k_swe_interact64<Q, NW, false, GUARD>), tp, threads, 0, st, g, src, src2, out, out_stride);
+    else if (wpt == 2)
+      SB_LAUNCH((k_swe_interact64<Q, 2, false, GUARD>), blocks_for(tp, NW / 2), threads, 0, st, g, src, src2, out,
+                out_stride);
+    else
+      SB_LAUNCH((k_swe_interact64<Q, 1, false, GUARD>), blocks_for(tp, NW), threads, 0, st, g, src, src2, out,
+                out_stride);
+  } else {
+    if (all_leaves) SB_SWE_K(true, false);
     else SB_SWE_K(false, false);
   }
 #undef SB_SWE_K
