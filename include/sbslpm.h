@@ -549,22 +549,13 @@ sbslpm_status sbslpm_direct_sum_inv_lap(long n, const double* x, const double* y
 /* No counterpart in the reference.  The same Biot-Savart direct sum as
  * sbslpm_direct_sum_bve, for callers that cannot let a library allocate
  * device memory: a host model that fixes its device footprint at start-up, or
- * that routes every device allocation through its own allocator, cannot
- * accept the cudaMallocAsync/cudaFreeAsync of scratch that
- * sbslpm_direct_sum_bve makes on every call.  This entry point allocates
- * nothing: its scratch is one fixed 16 MiB array compiled into the library,
- * which each GPU that loads the library holds until the process exits.
- * Limit: n_targets <= 699,050 (3 * n_targets doubles of scratch); larger
- * calls return SBSLPM_ERR_ARG with a message and do nothing.  Results equal
- * sbslpm_direct_sum_bve's up to summation order: from about 100,000 targets
- * the scratch holds fewer source groups than that entry point would use.
- * The first call on each device looks the array's device address up
- * (cudaGetSymbolAddress, with that device current) and keeps it, so make
- * that first call before any stream capture, and do not reset the device
- * (cudaDeviceReset) while the library is in use.  Every call on a device shares the one array and each call
- * overwrites the parts it uses, so calls whose kernels overlap on the GPU
- * (different streams or host threads) race: serialise them.  Synchronises
- * the stream before returning. */
+ * that routes every device allocation through its own allocator.  Neither
+ * entry point allocates device memory (their partial sums stay in shared
+ * memory); this one promises it.
+ * Limit: n_targets <= 699,050; larger calls return SBSLPM_ERR_ARG with a
+ * message and do nothing.  Results equal sbslpm_direct_sum_bve's; in mixed
+ * precision from about 100,000 targets up to the order of the sources'
+ * grouping.  Synchronises the stream before returning. */
 sbslpm_status sbslpm_direct_sum_bve_noalloc(long n_targets, const double* tx, const double* ty, const double* tz,
                                             long n_sources, const double* sx, const double* sy, const double* sz,
                                             const double* strength, double eps, int precision, double* u_x,

@@ -9,8 +9,10 @@
 //   tgt   : double  [3][panels*q] proxy-target velocities.
 //   v_k   : double  [3][leaves*q] stage velocities (x, y, z blocks).
 // Every kernel is owner-computes (no atomics), so results are deterministic.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <type_traits>
 
@@ -963,100 +965,188 @@ __global__ void k_depart_remap_batch(StepGeom g, BliTable tab, const double* __r
 }
 
 // ---------------------------------------------------------------------------
-// Stand-alone direct sums over arbitrary points: blocks own 128 targets and
-// stage 128 sources at a time in shared memory; gridDim.y source groups write
-// partials reduced by k_reduce_groups.
+// Stand-alone direct sums over arbitrary points.  A cluster of kDirectRanks
+// blocks owns a tile of targets; its blocks, and the warps (float64) or
+// 64-thread groups (mixed) within a block, split the sources, and the partial
+// sums are added in a fixed order over shared memory and distributed shared
+// memory.  Nothing goes through device memory: with partial sums there, a call
+// of 10,007 x 24,577 points spent 450 of its 790 us allocating and freeing
+// them, and three more launches adding them.
 
-constexpr int kDirectThreads = 128;
+constexpr int kDirectThreads = 256, kDirectRanks = 8;
+constexpr int kInvLapThreads = 128;
 
-__global__ void __launch_bounds__(kDirectThreads)
+// Adds the partial sums red[PARTS][3][TB] of the cluster's blocks, part by
+// part and rank by rank, and writes u = cb x cross a for the targets.
+template <int PARTS, int TB>
+__device__ __forceinline__ void direct_reduce(double* red, double* bsum, long nt, const double* __restrict__ tx,
+                                              const double* __restrict__ ty, const double* __restrict__ tz, double cb,
+                                              double* __restrict__ ux, double* __restrict__ uy,
+                                              double* __restrict__ uz) {
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  __syncthreads();
+  for (int k = threadIdx.x; k < 3 * TB; k += kDirectThreads) {
+    double a = red[k];
+#pragma unroll
+    for (int p = 1; p < PARTS; p++) a += red[p * 3 * TB + k];
+    bsum[k] = a;
+  }
+  cl.sync();
+  constexpr int SHARE = TB / kDirectRanks;  // each rank finishes its share of the targets
+  if (threadIdx.x < SHARE) {
+    const int k = (int)cl.block_rank() * SHARE + threadIdx.x;
+    const long i = (long)blockIdx.x * TB + k;
+    if (i < nt) {
+      double a[3] = {0, 0, 0};
+      for (int r = 0; r < kDirectRanks; r++) {
+        const double* b = cl.map_shared_rank(bsum, r);
+#pragma unroll
+        for (int c = 0; c < 3; c++) a[c] += b[c * TB + k];
+      }
+      const double x = tx[i], y = ty[i], z = tz[i];
+      ux[i] = cb * (y * a[2] - z * a[1]);
+      uy[i] = cb * (z * a[0] - x * a[2]);
+      uz[i] = cb * (x * a[1] - y * a[0]);
+    }
+  }
+  cl.sync();  // the blocks' sums stay until every rank has read them
+}
+
+// float64: two targets per lane (64 per block), each warp sweeping its own
+// `per` sources 32 at a time through its own tile, the next 32 loaded during
+// the current ones.
+template <bool GUARD>
+__global__ void __cluster_dims__(1, kDirectRanks, 1) __launch_bounds__(kDirectThreads, 4)
     k_direct_bve64(long nt, const double* __restrict__ tx, const double* __restrict__ ty,
                    const double* __restrict__ tz, long ns, const double* __restrict__ sx,
                    const double* __restrict__ sy, const double* __restrict__ sz, const double* __restrict__ sw,
-                   double eps, double* __restrict__ partial) {
-  __shared__ double4 tile[kDirectThreads];
-  long i = blockIdx.x * (long)kDirectThreads + threadIdx.x;
-  double x = 0, y = 0, z = 0;
-  if (i < nt) {
-    x = tx[i];
-    y = ty[i];
-    z = tz[i];
+                   long per, double eps, double* __restrict__ ux, double* __restrict__ uy, double* __restrict__ uz) {
+  constexpr int TPT = 2, TB = 32 * TPT, PARTS = kDirectThreads / 32;
+  __shared__ __align__(16) double2 tile[PARTS][64];
+  __shared__ double red[PARTS * 3 * TB], bsum[3 * TB];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double x[TPT], y[TPT], z[TPT], ax[TPT], ay[TPT], az[TPT];
+#pragma unroll
+  for (int r = 0; r < TPT; r++) {
+    const long i = min(nt - 1, (long)blockIdx.x * TB + lane + 32 * r);
+    x[r] = tx[i];
+    y[r] = ty[i];
+    z[r] = tz[i];
+    ax[r] = ay[r] = az[r] = 0;
   }
-  long per = (ns + gridDim.y - 1) / gridDim.y;
-  long s0 = blockIdx.y * per, s1 = min(ns, s0 + per);
-  double ax = 0, ay = 0, az = 0;
   const double eps2 = twice_eps(eps);
-  for (long b = s0; b < s1; b += kDirectThreads) {
-    long k = b + threadIdx.x;
-    tile[threadIdx.x] = k < s1 ? make_double4(sx[k], sy[k], sz[k], sw[k]) : make_double4(0, 0, 0, 0);
-    __syncthreads();
-    int cnt = (int)min((long)kDirectThreads, s1 - b);
-    for (int m = 0; m < cnt; m++) pair64<true>(x, y, z, tile[m], eps2, ax, ay, az);
-    __syncthreads();
+  const long s0 = (blockIdx.y * PARTS + warp) * per, s1 = min(ns, s0 + per);
+  double2 a = make_double2(0, 0), b = a;
+  auto load = [&](long k) {
+    if (k < s1) {
+      a = make_double2(sx[k], sy[k]);
+      b = make_double2(sz[k], sw[k]);
+    }
+  };
+  load(s0 + lane);
+  for (long k = s0; k < s1; k += 32) {
+    __syncwarp();
+    tile[warp][2 * lane] = a;
+    tile[warp][2 * lane + 1] = b;
+    __syncwarp();
+    load(k + 32 + lane);
+    const int cnt = (int)min(32L, s1 - k);
+#pragma unroll 8
+    for (int m = 0; m < cnt; m++) {
+      const double2 p = tile[warp][2 * m], q = tile[warp][2 * m + 1];
+      pairs64<GUARD>(x, y, z, p.x, p.y, q.x, q.y, eps2, ax, ay, az);
+    }
   }
-  if (i < nt) {
-    long o = (long)blockIdx.y * 3 * nt + i;
-    partial[o] = kBiotSavartTwice * (y * az - z * ay);
-    partial[nt + o] = kBiotSavartTwice * (z * ax - x * az);
-    partial[2 * nt + o] = kBiotSavartTwice * (x * ay - y * ax);
+#pragma unroll
+  for (int r = 0; r < TPT; r++) {
+    double* p = red + warp * 3 * TB + lane + 32 * r;
+    p[0] = ax[r];
+    p[TB] = ay[r];
+    p[2 * TB] = az[r];
   }
+  direct_reduce<PARTS, TB>(red, bsum, nt, tx, ty, tz, kBiotSavartTwice, ux, uy, uz);
 }
 
-// Mixed: each block measures both tiles relative to their first point (in
-// float64), so float32 carries only the small in-tile offsets.
-__global__ void __launch_bounds__(kDirectThreads)
+// Mixed: 128 targets per block, two per thread (the paired float32
+// instructions take one source against both), groups of 64 threads walking
+// the source groups; both tiles are measured relative to their first point
+// (in float64), so float32 carries only the small in-tile offsets.  A
+// target's sources are added in order, per tile of 128 in float32 and over
+// the tiles in float64.
+__global__ void __cluster_dims__(1, kDirectRanks, 1) __launch_bounds__(kDirectThreads)
     k_direct_bve32(long nt, const double* __restrict__ tx, const double* __restrict__ ty,
                    const double* __restrict__ tz, long ns, const double* __restrict__ sx,
                    const double* __restrict__ sy, const double* __restrict__ sz, const double* __restrict__ sw,
-                   double eps, double* __restrict__ partial) {
-  __shared__ float4 tile[kDirectThreads];
-  long i = blockIdx.x * (long)kDirectThreads + threadIdx.x;
-  long i0 = blockIdx.x * (long)kDirectThreads;
+                   int groups, double eps, double* __restrict__ ux, double* __restrict__ uy, double* __restrict__ uz) {
+  constexpr int TB = 128, NT = 64, PARTS = kDirectThreads / NT;
+  __shared__ float4 tile[PARTS][TB];
+  __shared__ double red[PARTS * 3 * TB], bsum[3 * TB];
+  const int part = threadIdx.x / NT, th = threadIdx.x % NT;
+  const long i0 = blockIdx.x * (long)TB;
   const double tcx = tx[i0], tcy = ty[i0], tcz = tz[i0];
-  double x = tcx, y = tcy, z = tcz;
-  if (i < nt) {
-    x = tx[i];
-    y = ty[i];
-    z = tz[i];
+  float dtx[2], dty[2], dtz[2];
+  double ax[2] = {0, 0}, ay[2] = {0, 0}, az[2] = {0, 0};
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    const long i = i0 + th + NT * r;
+    dtx[r] = i < nt ? (float)((tx[i] - tcx) * kPackScale) : 0.f;
+    dty[r] = i < nt ? (float)((ty[i] - tcy) * kPackScale) : 0.f;
+    dtz[r] = i < nt ? (float)((tz[i] - tcz) * kPackScale) : 0.f;
   }
-  const float dtx = (float)((x - tcx) * kPackScale), dty = (float)((y - tcy) * kPackScale),
-              dtz = (float)((z - tcz) * kPackScale);
-  long per = (ns + gridDim.y - 1) / gridDim.y;
-  long s0 = blockIdx.y * per, s1 = min(ns, s0 + per);
-  double ax = 0, ay = 0, az = 0;
   const float feps = (float)eps;
-  for (long b = s0; b < s1; b += kDirectThreads) {
-    const double scx = sx[b], scy = sy[b], scz = sz[b];
-    long k = b + threadIdx.x;
-    tile[threadIdx.x] = k < s1 ? make_float4((float)((sx[k] - scx) * kPackScale), (float)((sy[k] - scy) * kPackScale),
-                                             (float)((sz[k] - scz) * kPackScale), (float)sw[k])
-                               : make_float4(0, 0, 0, 0);
-    __syncthreads();
-    float bx = (float)((scx - tcx) * kPackScale) - dtx, by = (float)((scy - tcy) * kPackScale) - dty,
-          bz = (float)((scz - tcz) * kPackScale) - dtz;
-    float fx = 0, fy = 0, fz = 0;
-    int cnt = (int)min((long)kDirectThreads, s1 - b);
-    for (int m = 0; m < cnt; m++) pair32<true>(bx, by, bz, tile[m], feps, fx, fy, fz);
-    ax += fx;
-    ay += fy;
-    az += fz;
-    __syncthreads();
+  const float2 eps2 = make_float2(feps, feps);
+  const long per = (ns + groups - 1) / groups;
+  for (int grp = blockIdx.y * PARTS + part; grp < groups; grp += kDirectRanks * PARTS) {
+    const long s0 = grp * per, s1 = min(ns, s0 + per);
+    for (long b = s0; b < s1; b += TB) {
+      const double scx = sx[b], scy = sy[b], scz = sz[b];
+      const int cnt = (int)min((long)TB, s1 - b);
+      asm volatile("bar.sync %0, %1;" : : "r"(1 + part), "n"(NT) : "memory");
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        const int m = th + NT * r;
+        const long k = b + m;
+        if (m < cnt)
+          tile[part][m] = make_float4((float)((sx[k] - scx) * kPackScale), (float)((sy[k] - scy) * kPackScale),
+                                      (float)((sz[k] - scz) * kPackScale), (float)sw[k]);
+      }
+      asm volatile("bar.sync %0, %1;" : : "r"(1 + part), "n"(NT) : "memory");
+      const float cx = (float)((scx - tcx) * kPackScale), cy = (float)((scy - tcy) * kPackScale),
+                  cz = (float)((scz - tcz) * kPackScale);
+      const float2 bx = make_float2(cx - dtx[0], cx - dtx[1]), by = make_float2(cy - dty[0], cy - dty[1]),
+                   bz = make_float2(cz - dtz[0], cz - dtz[1]);
+      float2 fx = make_float2(0.f, 0.f), fy = fx, fz = fx;
+#pragma unroll 8
+      for (int m = 0; m < cnt; m++) {
+        const float4 v = tile[part][m];
+        pair32x2<true>(bx, by, bz, make_float2(v.x, v.x), make_float2(v.y, v.y), make_float2(v.z, v.z),
+                       make_float2(v.w, v.w), eps2, fx, fy, fz);
+      }
+      ax[0] += fx.x;
+      ay[0] += fy.x;
+      az[0] += fz.x;
+      ax[1] += fx.y;
+      ay[1] += fy.y;
+      az[1] += fz.y;
+    }
   }
-  if (i < nt) {
-    long o = (long)blockIdx.y * 3 * nt + i;
-    partial[o] = kBiotSavartPacked * (y * az - z * ay);
-    partial[nt + o] = kBiotSavartPacked * (z * ax - x * az);
-    partial[2 * nt + o] = kBiotSavartPacked * (x * ay - y * ax);
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    double* p = red + part * 3 * TB + th + NT * r;
+    p[0] = ax[r];
+    p[TB] = ay[r];
+    p[2 * TB] = az[r];
   }
+  direct_reduce<PARTS, TB>(red, bsum, nt, tx, ty, tz, kBiotSavartPacked, ux, uy, uz);
 }
 
 // inv_lap (src/direct_sum_impl.hpp:20-27): soln_i += sum_{j != i}
 // -1/(4 pi) log(1 - x_i.x_j) area_j pots_j.
-__global__ void __launch_bounds__(kDirectThreads)
+__global__ void __launch_bounds__(kInvLapThreads)
     k_inv_lap(long n, const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
               const double* __restrict__ area, const double* __restrict__ pots, double* __restrict__ soln) {
-  __shared__ double4 tile[kDirectThreads];
-  long i = blockIdx.x * (long)kDirectThreads + threadIdx.x;
+  __shared__ double4 tile[kInvLapThreads];
+  long i = blockIdx.x * (long)kInvLapThreads + threadIdx.x;
   double xi = 0, yi = 0, zi = 0;
   if (i < n) {
     xi = x[i];
@@ -1064,11 +1154,11 @@ __global__ void __launch_bounds__(kDirectThreads)
     zi = z[i];
   }
   double acc = 0;
-  for (long b = 0; b < n; b += kDirectThreads) {
+  for (long b = 0; b < n; b += kInvLapThreads) {
     long k = b + threadIdx.x;
     tile[threadIdx.x] = k < n ? make_double4(x[k], y[k], z[k], area[k] * pots[k]) : make_double4(0, 0, 0, 0);
     __syncthreads();
-    int cnt = (int)min((long)kDirectThreads, n - b);
+    int cnt = (int)min((long)kInvLapThreads, n - b);
     for (int m = 0; m < cnt; m++) {
       if (b + m == i) continue;
       double4 s = tile[m];
@@ -1387,27 +1477,35 @@ void launch_depart_remap_batch(const StepGeom& g, const BliTable* tab, int membe
 #undef SB_DRB
 }
 
+// Source groups of the mixed direct sum (a group's tiles start at its own
+// first source): enough groups for a few blocks per SM, none below 1,024
+// sources, 64 at most.
 int direct_groups(long nt, long ns) {
-  // enough blocks to fill 148 SMs a few times over, without tiny groups
-  long tblocks = (nt + kDirectThreads - 1) / kDirectThreads;
-  long want = (4L * 148 * 8 + tblocks - 1) / tblocks;
-  long maxg = (ns + 1023) / 1024;
-  long gsel = want < maxg ? want : maxg;
+  const long tblocks = (nt + 127) / 128;
+  const long want = (4L * 148 * 8 + tblocks - 1) / tblocks, maxg = (ns + 1023) / 1024;
+  const long gsel = want < maxg ? want : maxg;
   return (int)(gsel < 1 ? 1 : (gsel > 64 ? 64 : gsel));
 }
 
 void launch_direct_bve(long nt, const double* tx, const double* ty, const double* tz, long ns, const double* sx,
-                       const double* sy, const double* sz, const double* s, double eps, int precision, double* partial,
-                       int groups, double* ux, double* uy, double* uz, cudaStream_t st) {
-  dim3 grid(blocks_for(nt, kDirectThreads), groups);
-  if (precision == SBSLPM_MIXED)
-    SB_LAUNCH(k_direct_bve32, grid, kDirectThreads, 0, st, nt, tx, ty, tz, ns, sx, sy, sz, s, eps, partial);
+                       const double* sy, const double* sz, const double* s, double eps, int precision, int groups,
+                       double* ux, double* uy, double* uz, cudaStream_t st) {
+  if (precision == SBSLPM_MIXED) {
+    SB_LAUNCH(k_direct_bve32, dim3(blocks_for(nt, 128), kDirectRanks), kDirectThreads, 0, st, nt, tx, ty, tz, ns, sx,
+              sy, sz, s, groups, eps, ux, uy, uz);
+    return;
+  }
+  // a warp's share of the sources, at least one tile
+  const long parts = kDirectRanks * (kDirectThreads / 32), per = std::max(32L, (ns + parts - 1) / parts);
+  const dim3 grid(blocks_for(nt, 64), kDirectRanks);
+  // with eps > 0 a coincident pair adds g * 0; the guard is for eps = 0 and for
+  // eps so small that g would overflow
+  if (eps >= 1e-100)
+    SB_LAUNCH(k_direct_bve64<false>, grid, kDirectThreads, 0, st, nt, tx, ty, tz, ns, sx, sy, sz, s, per, eps, ux, uy,
+              uz);
   else
-    SB_LAUNCH(k_direct_bve64, grid, kDirectThreads, 0, st, nt, tx, ty, tz, ns, sx, sy, sz, s, eps, partial);
-  // reduce into the three output arrays (they need not be contiguous)
-  double* outs[3] = {ux, uy, uz};
-  for (int c = 0; c < 3; c++)
-    SB_LAUNCH(k_reduce_groups, blocks_for(nt, 256), 256, 0, st, partial + (long)c * nt, groups, nt, 3 * nt, outs[c]);
+    SB_LAUNCH(k_direct_bve64<true>, grid, kDirectThreads, 0, st, nt, tx, ty, tz, ns, sx, sy, sz, s, per, eps, ux, uy,
+              uz);
 }
 
 void launch_ssw_forcing(int leaves, int q, int type, double omega, const double* time, const double* x,
@@ -1421,7 +1519,7 @@ void launch_time_advance(double* time, double dt, cudaStream_t st) {
 
 void launch_inv_lap(long n, const double* x, const double* y, const double* z, const double* area,
                     const double* pots, double* soln, cudaStream_t st) {
-  SB_LAUNCH(k_inv_lap, blocks_for(n, kDirectThreads), kDirectThreads, 0, st, n, x, y, z, area, pots, soln);
+  SB_LAUNCH(k_inv_lap, blocks_for(n, kInvLapThreads), kInvLapThreads, 0, st, n, x, y, z, area, pots, soln);
 }
 
 }  // namespace sbslpm

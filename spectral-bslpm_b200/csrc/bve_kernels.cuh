@@ -105,8 +105,7 @@ void launch_copy_strength(const StepGeom& g, const double4* src, double* out, cu
 // Stand-alone direct sums (no tree).
 int direct_groups(long n_targets, long n_sources);
 void launch_direct_bve(long nt, const double* tx, const double* ty, const double* tz, long ns, const double* sx,
-                       const double* sy, const double* sz, const double* s, double eps, int precision, double* partial,
-                       int groups, double* ux, double* uy, double* uz, cudaStream_t st);
+                       const double* sy, const double* sz, const double* s, double eps, int precision, int groups, double* ux, double* uy, double* uz, cudaStream_t st);
 // bve_ssw_forcing / bve_ssw_forcing_2 (src/forcing_funcs.cpp:6-80) at the
 // device-held time: force[leaf][q]; then time += dt (launch_time_advance).
 void launch_ssw_forcing(int leaves, int q, int type, double omega, const double* time, const double* x,

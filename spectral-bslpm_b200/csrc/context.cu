@@ -1154,12 +1154,8 @@ sbslpm_status sbslpm_direct_sum_bve(long nt, const double* tx, const double* ty,
     SB_CUDA(cudaStreamSynchronize(st));
     return SBSLPM_OK;
   }
-  int groups = direct_groups(nt, ns);
-  double* partial = nullptr;
-  SB_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&partial), sizeof(double) * 3 * nt * groups, st));
-  launch_direct_bve(nt, tx, ty, tz, ns, sx, sy, sz, s, eps, precision, partial, groups, ux, uy, uz, st);
+  launch_direct_bve(nt, tx, ty, tz, ns, sx, sy, sz, s, eps, precision, direct_groups(nt, ns), ux, uy, uz, st);
   SB_CUDA(cudaGetLastError());
-  SB_CUDA(cudaFreeAsync(partial, st));
   SB_CUDA(cudaStreamSynchronize(st));
   return SBSLPM_OK;
 }
