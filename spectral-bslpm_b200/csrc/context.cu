@@ -848,7 +848,7 @@ sbslpm_status sbslpm_destroy(sbslpm_ctx* c) {
                   c->adj_w, c->adj_vel, c->adj_near_ts, c->adj_near_tt, c->adj_cc_ts, c->adj_cc_tt, c->adj_tbar,
                   c->adj_qbl, c->self, c->force, c->d_time, c->cc_partial, c->entry32, c->fentry32, c->fsrcp,
                   c->mutual_units, c->near_slot, c->fsrc2, c->psrc2, c->fsrcf2, c->psrcf2, c->adj_ynl,
-                  c->swe_cc_partial};
+                  c->swe_cc_partial, c->log_table};
   for (void* b : bufs)
     if (b) cudaFree(b);
   for (int k = 0; k < 4; k++) {

@@ -27,7 +27,15 @@ namespace dev {
 
 template <int Q, int FIELDS>
 struct ListShape {
-  static constexpr int TPT = Q <= 1 ? 1 : Q <= 4 ? 2 : Q <= 9 ? 3 : Q <= 16 ? 2 : 5;
+  static constexpr int TPT = Q <= 1    ? 1
+                             : Q <= 4   ? 2
+                             : Q <= 9   ? 3
+                             : Q <= 16  ? 2
+                             : Q <= 49  ? 5
+                             : Q <= 64  ? 4
+                             : Q <= 81  ? 3
+                             : Q <= 100 ? 7
+                                        : 4;
   static constexpr int LPT = (Q + TPT - 1) / TPT;
   static constexpr int S = 32 / LPT;
   static constexpr int STRIDE = 2 * Q + 1;              // double2 per split, buffer and field
@@ -52,6 +60,13 @@ inline int list_warps(int target_panels) {
 
 __device__ __forceinline__ void copy_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+               :
+               : "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+__device__ __forceinline__ void copy_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
                :
                : "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
                : "memory");
