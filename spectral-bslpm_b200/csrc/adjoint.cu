@@ -31,7 +31,7 @@ constexpr int kAdjThreads = 128;
 
 // ---------------------------------------------------------------------------
 // Biot-Savart sum: vector-Jacobian product with respect to the sources.
-// One thread per source; target tiles (x_i, c_i = ubar_i x x_i) staged in
+// Two sources per thread; target tiles (x_i, c_i = ubar_i x x_i) staged in
 // shared memory; gridDim.y groups of targets write partials [group][4][ns]
 // (qbar, ybar x, y, z) that k_sum_groups adds in group order.
 template <bool GUARD>
@@ -39,47 +39,59 @@ __global__ void __launch_bounds__(kAdjThreads)
     k_bs_vjp64(long nt, const double* __restrict__ tx, const double* __restrict__ ty, const double* __restrict__ tz,
                const double* __restrict__ ux, const double* __restrict__ uy, const double* __restrict__ uz, long ns,
                const double4* __restrict__ src, double eps, double* __restrict__ partial) {
-  __shared__ double sx[kAdjThreads], sy[kAdjThreads], sz[kAdjThreads], scx[kAdjThreads], scy[kAdjThreads],
-      scz[kAdjThreads];
-  const long j = blockIdx.x * (long)kAdjThreads + threadIdx.x;
+  constexpr int TPT = 2;  // sources per thread: a shared-memory read of a target feeds two pairs
+  __shared__ __align__(16) double2 tile[kAdjThreads][3];  // x, y | z, cx | cy, cz with c = ubar x x
   const long per = (nt + gridDim.y - 1) / gridDim.y;
   const long t0 = blockIdx.y * per, t1 = min(nt, t0 + per);
-  double4 s = j < ns ? src[j] : make_double4(0, 0, 0, 0);
-  double qb = 0, bx = 0, by = 0, bz = 0;
+  double sx[TPT], sy[TPT], sz[TPT], qb[TPT], bx[TPT], by[TPT], bz[TPT];
+#pragma unroll
+  for (int r = 0; r < TPT; r++) {
+    const long j = min(ns - 1, (blockIdx.x * (long)TPT + r) * kAdjThreads + threadIdx.x);
+    const double4 s = src[j];
+    sx[r] = s.x;
+    sy[r] = s.y;
+    sz[r] = s.z;
+    qb[r] = bx[r] = by[r] = bz[r] = 0;
+  }
   for (long base = t0; base < t1; base += kAdjThreads) {
     const long i = base + threadIdx.x;
     __syncthreads();
     if (i < t1) {
       const double x = tx[i], y = ty[i], z = tz[i], a = ux[i], b = uy[i], c = uz[i];
-      sx[threadIdx.x] = x;
-      sy[threadIdx.x] = y;
-      sz[threadIdx.x] = z;
-      scx[threadIdx.x] = b * z - c * y;  // ubar x x
-      scy[threadIdx.x] = c * x - a * z;
-      scz[threadIdx.x] = a * y - b * x;
+      tile[threadIdx.x][0] = make_double2(x, y);
+      tile[threadIdx.x][1] = make_double2(z, b * z - c * y);
+      tile[threadIdx.x][2] = make_double2(c * x - a * z, a * y - b * x);
     }
     __syncthreads();
     const int cnt = (int)min((long)kAdjThreads, t1 - base);
+#pragma unroll 4
     for (int k = 0; k < cnt; k++) {
-      const double dx = s.x - sx[k], dy = s.y - sy[k], dz = s.z - sz[k];
-      const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-      double g = recip_nr(fma(0.5, r2, eps));
-      if (GUARD) g = r2 > 0.0 ? g : 0.0;
-      const double cx = scx[k], cy = scy[k], cz = scz[k];
-      const double sd = fma(cx, dx, fma(cy, dy, cz * dz));
-      qb = fma(g, sd, qb);
-      const double t = g * g * sd;
-      bx = fma(g, cx, fma(-t, dx, bx));
-      by = fma(g, cy, fma(-t, dy, by));
-      bz = fma(g, cz, fma(-t, dz, bz));
+      const double2 A = tile[k][0], B = tile[k][1], C = tile[k][2];
+#pragma unroll
+      for (int r = 0; r < TPT; r++) {
+        const double dx = sx[r] - A.x, dy = sy[r] - A.y, dz = sz[r] - B.x;
+        const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+        double g = recip_nr(fma(0.5, r2, eps));
+        if (GUARD) g = r2 > 0.0 ? g : 0.0;
+        const double u = g * fma(B.y, dx, fma(C.x, dy, C.y * dz));
+        qb[r] += u;
+        const double t = g * u;
+        bx[r] = fma(g, B.y, fma(-t, dx, bx[r]));
+        by[r] = fma(g, C.x, fma(-t, dy, by[r]));
+        bz[r] = fma(g, C.y, fma(-t, dz, bz[r]));
+      }
     }
   }
-  if (j < ns) {
-    double* p = partial + (long)blockIdx.y * 4 * ns;
-    p[j] = kBiotSavart * qb;
-    p[ns + j] = kBiotSavart * s.w * bx;
-    p[2 * ns + j] = kBiotSavart * s.w * by;
-    p[3 * ns + j] = kBiotSavart * s.w * bz;
+  double* p = partial + (long)blockIdx.y * 4 * ns;
+#pragma unroll
+  for (int r = 0; r < TPT; r++) {
+    const long j = (blockIdx.x * (long)TPT + r) * kAdjThreads + threadIdx.x;
+    if (j >= ns) continue;
+    const double w = kBiotSavart * src[j].w;
+    p[j] = kBiotSavart * qb[r];
+    p[ns + j] = w * bx[r];
+    p[2 * ns + j] = w * by[r];
+    p[3 * ns + j] = w * bz[r];
   }
 }
 
@@ -412,9 +424,9 @@ __global__ void k_depart_remap_adjoint(StepGeom g, BliTable tab, const double* _
 }
 
 int vjp_groups(long nt, long ns) {
-  const long sblocks = (ns + kAdjThreads - 1) / kAdjThreads;
+  const long sblocks = (ns + 2 * kAdjThreads - 1) / (2 * kAdjThreads);
   long want = (4L * 148 * 8 + sblocks - 1) / sblocks;
-  const long maxg = (nt + 1023) / 1024;
+  const long maxg = (nt + 255) / 256;
   long gsel = want < maxg ? want : maxg;
   return (int)(gsel < 1 ? 1 : (gsel > 64 ? 64 : gsel));
 }
@@ -426,7 +438,7 @@ int adjoint_groups(long nt, long ns) { return vjp_groups(nt, ns); }
 void launch_bs_vjp(long nt, const double* tx, const double* ty, const double* tz, const double* ux,
                    const double* uy, const double* uz, long ns, const double4* src, double eps, double* partial,
                    int groups, double* qbar, double* ybar, cudaStream_t st) {
-  const dim3 grid(blocks_for(ns, kAdjThreads), (unsigned)groups);
+  const dim3 grid(blocks_for(ns, 2 * kAdjThreads), (unsigned)groups);
   if (eps > 0)
     SB_LAUNCH(k_bs_vjp64<false>, grid, kAdjThreads, 0, st, nt, tx, ty, tz, ux, uy, uz, ns, src, eps, partial);
   else

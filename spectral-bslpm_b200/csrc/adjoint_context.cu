@@ -28,7 +28,7 @@ sbslpm_status adjoint_setup(sbslpm_ctx* c) {
   SB_TRY(dalloc(&c->adj_vbar, 4 * 3 * ln));
   SB_TRY(dalloc(&c->adj_q, ln));
   SB_TRY(dalloc(&c->adj_y, 3 * ln));
-  SB_TRY(dalloc(&c->adj_part, (size_t)c->adj_groups * 4 * ln));
+  if (c->cfg.velocity == SBSLPM_VEL_DIRECT) SB_TRY(dalloc(&c->adj_part, (size_t)c->adj_groups * 4 * ln));
   SB_TRY(dalloc(&c->adj_w, ln));
   SB_TRY(dalloc(&c->adj_vel, 3 * ln));
   if (c->tree) {

@@ -23,6 +23,7 @@
 // gives position adjoints, and a non-leaf proxy's displacement is the BLI
 // interpolation of its containing leaf's (bve_disp_interp), whose transpose
 // scatters back onto the leaf velocities.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "adjoint_pair32.cuh"
@@ -36,82 +37,148 @@ using namespace dev;
 
 constexpr int kT = 128;
 
-// Tbar_leaf[c][k] = sum_i B_k(x_i) vbar_c,i over the leaf's particles.
-__global__ void k_tree_to_particles_T(TreeGeom tg, StepGeom fg, const double* __restrict__ vbar,
-                                      double* __restrict__ tbar) {
-  extern __shared__ double sv[];  // 3 x npl
-  const int f = blockIdx.x, npl = tg.npl, n1 = tg.n + 1, qx = n1 * n1;
-  const long N = tg.N, pn = (long)fg.panels * qx;
-  for (int i = threadIdx.x; i < npl; i += blockDim.x)
-    for (int c = 0; c < 3; c++) sv[c * npl + i] = vbar[c * N + (long)f * npl + i];
+constexpr int kLeafThreads = 256;
+
+// Blocks of a cluster that share a source panel or leaf: enough that the tree
+// gives each SM about eight blocks (the 96 leaves of a 24,576-particle tree
+// left a third of the SMs without one), at most the portable eight.
+unsigned split_ranks(int units) {
+  unsigned r = 1;
+  while (r < 8 && units * (int)r < 8 * 148) r *= 2;
+  return r;
+}
+
+// Tbar_leaf[c][k] = sum_i B_k(x_i) vbar_c,i over the leaf's particles, one
+// block per (leaf, component c): the leaf-box bases in shared memory, the
+// particles in G contiguous groups (a thread per group and proxy), the
+// groups' sums added in order.
+__global__ void __launch_bounds__(kLeafThreads) k_tree_to_particles_T(TreeGeom tg, StepGeom fg,
+                                                                     const double* __restrict__ vbar,
+                                                                     double* __restrict__ tbar) {
+  extern __shared__ double sh[];  // npl values, npl n1 of each basis, G qx partial sums
+  const int f = blockIdx.x, c = blockIdx.y, npl = tg.npl, n1 = tg.n + 1, qx = n1 * n1;
+  const long pn = (long)fg.panels * qx;
+  double* sv = sh;
+  double* lx = sv + npl;
+  double* ly = lx + npl * n1;
+  double* part = ly + npl * n1;
+  for (int i = threadIdx.x; i < npl; i += blockDim.x) sv[i] = vbar[c * tg.N + (long)f * npl + i];
+  for (int i = threadIdx.x; i < npl * n1; i += blockDim.x) {
+    lx[i] = tg.lx[i];
+    ly[i] = tg.ly[i];
+  }
   __syncthreads();
-  const long base = (long)(fg.offset + f) * qx;
-  for (int m = threadIdx.x; m < 3 * qx; m += blockDim.x) {
-    const int c = m / qx, k = m % qx, a = k / n1, b = k % n1;
+  const int G = blockDim.x / qx > 0 ? blockDim.x / qx : 1, per = (npl + G - 1) / G;
+  for (int t = threadIdx.x; t < G * qx; t += blockDim.x) {
+    const int gi = t / qx, k = t - gi * qx, a = k / n1, b = k - a * n1;
+    const int i1 = min(npl, (gi + 1) * per);
     double acc = 0;
-    for (int i = 0; i < npl; i++) acc = fma(__ldg(tg.lx + i * n1 + a) * __ldg(tg.ly + i * n1 + b), sv[c * npl + i], acc);
-    tbar[c * pn + base + k] = acc;
+    for (int i = gi * per; i < i1; i++) acc = fma(lx[i * n1 + a] * ly[i * n1 + b], sv[i], acc);
+    part[t] = acc;
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < qx; k += blockDim.x) {
+    double acc = part[k];
+    for (int gi = 1; gi < G; gi++) acc += part[gi * qx + k];
+    tbar[c * pn + (long)(fg.offset + f) * qx + k] = acc;
   }
 }
 
-// One level of the transpose of the downward pass: parents at `level` add
-// the anterpolation of their children's three fields (child_to_parent form).
-__global__ void k_tree_up3(StepGeom fg, int level, double* __restrict__ t) {
+// One level of the transpose of the downward pass: a parent at `level` adds
+// the anterpolation of its children's fields (child_to_parent form), one
+// direction at a time as in the forward pass, a block per (parent, field).
+__global__ void __launch_bounds__(kT) k_tree_up3(StepGeom fg, int level, double* __restrict__ t) {
+  extern __shared__ double sh[];  // 4 children, 4 half-contracted
   const int n1 = fg.degree + 1, q = fg.q;
   const long pn = (long)fg.panels * q;
-  const long np = 6L << (2 * level);
-  const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (idx >= np * q * 3) return;
-  const int c3 = (int)(idx / (np * q));
-  const long r = idx % (np * q);
-  const long p = level_start(level) + r / q;
-  const int k = (int)(r % q), a = k / n1, b = k % n1;
-  double acc = 0;
-  for (int c = 0; c < 4; c++) {
-    const long ch = level_start(level + 1) + 4 * (p - level_start(level)) + c;
-    const double* lx = fg.child_1d + ((c == 1 || c == 2) ? n1 * n1 : 0);
-    const double* ly = fg.child_1d + (c >= 2 ? n1 * n1 : 0);
-    const double* tc = t + c3 * pn + ch * q;
-    for (int i = 0; i < n1; i++) {
-      double s = 0;
-      for (int j = 0; j < n1; j++) s = fma(__ldg(ly + j * n1 + b), tc[i * n1 + j], s);
-      acc = fma(__ldg(lx + i * n1 + a), s, acc);
-    }
+  const int p = blockIdx.x;  // relative to the level
+  double* field = t + blockIdx.y * pn;
+  const double* ch = field + ((long)level_start(level + 1) + 4 * p) * q;
+  double* half = sh + 4 * q;
+  for (int k = threadIdx.x; k < 4 * q; k += blockDim.x) sh[k] = ch[k];
+  __syncthreads();
+  for (int k = threadIdx.x; k < 4 * q; k += blockDim.x) {  // half[c][i][b] = sum_j Ly_c[j][b] S_c[i][j]
+    const int c = k / q, i = (k - c * q) / n1, b = k % n1;
+    const double* ly = fg.child_1d + (c >= 2 ? n1 * n1 : 0) + b;
+    const double* sc = sh + c * q + i * n1;
+    double acc = 0;
+    for (int j = 0; j < n1; j++) acc = fma(__ldg(ly + j * n1), sc[j], acc);
+    half[k] = acc;
   }
-  t[c3 * pn + p * q + k] += acc;
+  __syncthreads();
+  for (int k = threadIdx.x; k < q; k += blockDim.x) {
+    const int a = k / n1, b = k - a * n1;
+    double acc = 0;
+    for (int c = 0; c < 4; c++) {
+      const double* lx = fg.child_1d + ((c == 1 || c == 2) ? n1 * n1 : 0) + a;
+      const double* hc = half + c * q + b;
+      for (int i = 0; i < n1; i++) acc = fma(__ldg(lx + i * n1), hc[i * n1], acc);
+    }
+    field[((long)level_start(level) + p) * q + k] += acc;
+  }
 }
 
-// One level of the transpose of the upward pass: children of `level` add the
-// interpolation of their parent's (final) adjoint strengths.
-__global__ void k_tree_down1(StepGeom fg, int level, double* __restrict__ qb) {
-  const int n1 = fg.degree + 1, q = fg.q;
-  const long nc = 6L << (2 * (level + 1));
-  const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (idx >= nc * q) return;
-  const long ch = level_start(level + 1) + idx / q;
-  const int k = (int)(idx % q), i = k / n1, j = k % n1;
-  const long rel = ch - level_start(level + 1);
-  const long p = level_start(level) + rel / 4;
-  const int c = (int)(rel % 4);
-  const double* lx = fg.child_1d + ((c == 1 || c == 2) ? n1 * n1 : 0) + i * n1;
-  const double* ly = fg.child_1d + (c >= 2 ? n1 * n1 : 0) + j * n1;
-  double acc = 0;
-  for (int a = 0; a < n1; a++) {
-    double s = 0;
-    for (int b = 0; b < n1; b++) s = fma(__ldg(ly + b), qb[p * q + a * n1 + b], s);
-    acc = fma(__ldg(lx + a), s, acc);
+// One level of the transpose of the upward pass: the children of `level` add
+// the interpolation of their parent's (final) adjoint strengths, a block per
+// parent.
+__global__ void __launch_bounds__(kT) k_tree_down1(StepGeom fg, int level, double* __restrict__ qb) {
+  extern __shared__ double sh[];  // the parent, 2 halves contracted in eta
+  const int n1 = fg.degree + 1, q = fg.q, p = blockIdx.x;
+  const double* parent = qb + ((long)level_start(level) + p) * q;
+  double* ch = qb + ((long)level_start(level + 1) + 4 * p) * q;
+  double* half = sh + q;
+  for (int k = threadIdx.x; k < q; k += blockDim.x) sh[k] = parent[k];
+  __syncthreads();
+  for (int k = threadIdx.x; k < 2 * q; k += blockDim.x) {  // half[e][a][j] = sum_b Ly_e[j][b] Q[a][b]
+    const int e = k / q, a = (k - e * q) / n1, j = k % n1;
+    const double* ly = fg.child_1d + e * n1 * n1 + j * n1;
+    double acc = 0;
+    for (int b = 0; b < n1; b++) acc = fma(__ldg(ly + b), sh[a * n1 + b], acc);
+    half[k] = acc;
   }
-  qb[ch * q + k] += acc;
+  __syncthreads();
+  for (int k = threadIdx.x; k < 4 * q; k += blockDim.x) {
+    const int c = k / q, i = (k - c * q) / n1, j = k % n1;
+    const double* lx = fg.child_1d + ((c == 1 || c == 2) ? n1 * n1 : 0) + i * n1;
+    const double* h = half + (c >= 2 ? q : 0) + j;
+    double acc = 0;
+    for (int a = 0; a < n1; a++) acc = fma(__ldg(lx + a), h[a * n1], acc);
+    ch[k] += acc;
+  }
+}
+
+// Adds the cluster's partial sums v (COUNT values of each of `n` items, this
+// block's at sum[COUNT][n] in shared memory) rank by rank and calls
+// done(item, totals) for this rank's share of the items.
+template <int COUNT, class Done>
+__device__ __forceinline__ void cluster_totals(double* sum, int n, const Done& done) {
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  cl.sync();
+  const int ranks = (int)cl.num_blocks(), share = (n + ranks - 1) / ranks, i0 = (int)cl.block_rank() * share;
+  for (int i = i0 + threadIdx.x; i < min(n, i0 + share); i += blockDim.x) {
+    double tot[COUNT];
+#pragma unroll
+    for (int c = 0; c < COUNT; c++) tot[c] = 0;
+    for (int r = 0; r < ranks; r++) {
+      const double* b = cl.map_shared_rank(sum, r);
+#pragma unroll
+      for (int c = 0; c < COUNT; c++) tot[c] += b[c * n + i];
+    }
+    done(i, tot);
+  }
+  cl.sync();  // the sums stay until every rank has read them
 }
 
 // Transposed well-separated interactions: source panel s (blockIdx.x) sums
 // over the target panels t whose list holds s: Qbar_s,k = K sum_t sum_i g c.d,
-// c = Tbar_t,i x x_i, d = y_k - x_i.
+// c = Tbar_t,i x x_i, d = y_k - x_i.  A thread per source proxy; the cluster's
+// blocks (split_ranks) take the list's entries in turn.
 template <bool GUARD>
 __global__ void __launch_bounds__(kT) k_tree_cc_T(StepGeom fg, const int* __restrict__ tstart,
                                                  const int* __restrict__ ttgt, const double* __restrict__ tbar,
                                                  double* __restrict__ qbar) {
-  __shared__ double sx[kT], sy[kT], sz[kT], cx[kT], cy[kT], cz[kT];
+  __shared__ __align__(16) double2 tile[kT][3];  // x, y | z, cx | cy, cz
+  __shared__ double sum[kT];
   const int s = blockIdx.x, q = fg.q;
   const long pn = (long)fg.panels * q;
   const int k = threadIdx.x;
@@ -122,88 +189,136 @@ __global__ void __launch_bounds__(kT) k_tree_cc_T(StepGeom fg, const int* __rest
     yz = fg.px[2 * pn + (long)s * q + k];
   }
   double acc = 0;
-  for (int e = tstart[s]; e < tstart[s + 1]; e++) {
+  for (int e = tstart[s] + blockIdx.y; e < tstart[s + 1]; e += gridDim.y) {
     const long tb = (long)ttgt[e] * q;
     __syncthreads();
     if (k < q) {
       const double x = fg.px[tb + k], y = fg.px[pn + tb + k], z = fg.px[2 * pn + tb + k];
       const double a = tbar[tb + k], b = tbar[pn + tb + k], c = tbar[2 * pn + tb + k];
-      sx[k] = x;
-      sy[k] = y;
-      sz[k] = z;
-      cx[k] = b * z - c * y;
-      cy[k] = c * x - a * z;
-      cz[k] = a * y - b * x;
+      tile[k][0] = make_double2(x, y);
+      tile[k][1] = make_double2(z, b * z - c * y);
+      tile[k][2] = make_double2(c * x - a * z, a * y - b * x);
     }
     __syncthreads();
-    if (k < q)
+    if (k < q) {
+#pragma unroll 4
       for (int i = 0; i < q; i++) {
-        const double dx = yx - sx[i], dy = yy - sy[i], dz = yz - sz[i];
+        const double2 A = tile[i][0], B = tile[i][1], C = tile[i][2];
+        const double dx = yx - A.x, dy = yy - A.y, dz = yz - B.x;
         const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
         double g = recip_nr(fma(0.5, r2, fg.eps));
         if (GUARD) g = r2 > 0.0 ? g : 0.0;
-        acc = fma(g, fma(cx[i], dx, fma(cy[i], dy, cz[i] * dz)), acc);
+        acc = fma(g, fma(B.y, dx, fma(C.x, dy, C.y * dz)), acc);
       }
+    }
   }
-  if (k < q) qbar[(long)s * q + k] = kBiotSavart * acc;
+  if (k < q) sum[k] = acc;
+  cluster_totals<1>(sum, q, [&](int i, const double* v) { qbar[(long)s * q + i] = kBiotSavart * v[0]; });
 }
 
-// Transposed near field: source leaf sl (blockIdx.x), one thread per source
-// particle, over the target leaves whose near list holds sl.  Writes qbar_j
-// and ybar_j (3 components) of the leaf's particles.
-template <bool GUARD>
-__global__ void __launch_bounds__(512) k_tree_near_T(TreeGeom tg, const int* __restrict__ tstart,
+// Transposed near field: blockIdx.x = (source leaf sl, chunk of 2 NT of its
+// particles), two source particles per thread, over the target leaves whose
+// near list holds sl, cut into tiles of 64 targets that the cluster's blocks
+// (split_ranks) share out.  Writes qbar_j
+// and ybar_j (3 components) of the leaf's particles.  One block of 256 threads
+// per leaf took 345 us at 24,576 particles (96 blocks), this 215 us: bound by
+// the FP64 pipe and its register reads (22 operations a pair, 9 of them with
+// three different registers).
+template <int NT, bool GUARD>
+__global__ void __launch_bounds__(NT) k_tree_near_T(TreeGeom tg, const int* __restrict__ tstart,
                                                    const int* __restrict__ ttgt, const double* __restrict__ x,
                                                    const double* __restrict__ y, const double* __restrict__ z,
                                                    const double* __restrict__ vbar, const double4* __restrict__ psrc,
                                                    double* __restrict__ qbar, double* __restrict__ ybar) {
-  extern __shared__ double tile[];  // 6 x npl: target positions, c = vbar x x
-  const int sl = blockIdx.x, npl = tg.npl;
-  const long N = tg.N;
-  double* tx = tile;
-  double* ty = tx + npl;
-  double* tz = ty + npl;
-  double* cx = tz + npl;
-  double* cy = cx + npl;
-  double* cz = cy + npl;
-  const int j = threadIdx.x;
-  const long oj = (long)sl * npl + j;
-  const double4 s = j < npl ? psrc[oj] : make_double4(0, 0, 0, 0);
-  double qb = 0, bx = 0, by = 0, bz = 0;
-  for (int e = tstart[sl]; e < tstart[sl + 1]; e++) {
-    const long tb = (long)ttgt[e] * npl;
+  constexpr int TPT = 2, TS = 64, NSRC = TPT * NT;
+  __shared__ __align__(16) double2 tile[TS][3];  // x, y | z, cx | cy, cz with c = vbar x x
+  __shared__ double sum[4 * NSRC];
+  const int npl = tg.npl, chunks = (npl + NSRC - 1) / NSRC, sl = blockIdx.x / chunks;
+  const int first = (blockIdx.x - sl * chunks) * NSRC, count = min(NSRC, npl - first);
+  const long N = tg.N, o0 = (long)sl * npl + first;
+  double sx[TPT], sy[TPT], sz[TPT], qb[TPT], bx[TPT], by[TPT], bz[TPT];
+#pragma unroll
+  for (int r = 0; r < TPT; r++) {
+    const int j = threadIdx.x + r * NT;
+    const double4 s = psrc[o0 + (j < count ? j : 0)];
+    sx[r] = s.x;
+    sy[r] = s.y;
+    sz[r] = s.z;
+    qb[r] = bx[r] = by[r] = bz[r] = 0;
+  }
+  const int e0 = tstart[sl], tiles = (npl + TS - 1) / TS;
+  const long total = (long)(tstart[sl + 1] - e0) * tiles;
+  const long t1 = total * (blockIdx.y + 1) / gridDim.y;
+  for (long tt = total * blockIdx.y / gridDim.y; tt < t1; tt++) {
+    const int i0 = (int)(tt % tiles) * TS, cnt = min(TS, npl - i0);
+    const long tb = (long)ttgt[e0 + tt / tiles] * npl + i0;
     __syncthreads();
-    for (int i = threadIdx.x; i < npl; i += blockDim.x) {
+    for (int i = threadIdx.x; i < cnt; i += NT) {
       const double a = vbar[tb + i], b = vbar[N + tb + i], c = vbar[2 * N + tb + i];
       const double px = x[tb + i], py = y[tb + i], pz = z[tb + i];
-      tx[i] = px;
-      ty[i] = py;
-      tz[i] = pz;
-      cx[i] = b * pz - c * py;
-      cy[i] = c * px - a * pz;
-      cz[i] = a * py - b * px;
+      tile[i][0] = make_double2(px, py);
+      tile[i][1] = make_double2(pz, b * pz - c * py);
+      tile[i][2] = make_double2(c * px - a * pz, a * py - b * px);
     }
     __syncthreads();
-    if (j < npl)
-      for (int i = 0; i < npl; i++) {
-        const double dx = s.x - tx[i], dy = s.y - ty[i], dz = s.z - tz[i];
-        const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-        double g = recip_nr(fma(0.5, r2, tg.eps));
-        if (GUARD) g = r2 > 0.0 ? g : 0.0;
-        const double sd = fma(cx[i], dx, fma(cy[i], dy, cz[i] * dz));
-        qb = fma(g, sd, qb);
-        const double t = g * g * sd;
-        bx = fma(g, cx[i], fma(-t, dx, bx));
-        by = fma(g, cy[i], fma(-t, dy, by));
-        bz = fma(g, cz[i], fma(-t, dz, bz));
+#pragma unroll 4
+    for (int i = 0; i < cnt; i++) {
+      const double2 A = tile[i][0], B = tile[i][1], C = tile[i][2];
+      // step by step for both sources: an operand held over from the
+      // instruction before saves a register read (pairs64)
+      double dx[TPT], dy[TPT], dz[TPT], g[TPT], u[TPT], t[TPT];
+#pragma unroll
+      for (int r = 0; r < TPT; r++) dx[r] = sx[r] - A.x;
+#pragma unroll
+      for (int r = 0; r < TPT; r++) dy[r] = sy[r] - A.y;
+#pragma unroll
+      for (int r = 0; r < TPT; r++) dz[r] = sz[r] - B.x;
+#pragma unroll
+      for (int r = 0; r < TPT; r++) {
+        const double r2 = fma(dx[r], dx[r], fma(dy[r], dy[r], dz[r] * dz[r]));
+        g[r] = recip_nr(fma(0.5, r2, tg.eps));
+        if (GUARD) g[r] = r2 > 0.0 ? g[r] : 0.0;
       }
+#pragma unroll
+      for (int r = 0; r < TPT; r++) u[r] = C.y * dz[r];
+#pragma unroll
+      for (int r = 0; r < TPT; r++) u[r] = fma(C.x, dy[r], u[r]);
+#pragma unroll
+      for (int r = 0; r < TPT; r++) u[r] = fma(B.y, dx[r], u[r]);
+#pragma unroll
+      for (int r = 0; r < TPT; r++) {
+        u[r] = g[r] * u[r];
+        qb[r] += u[r];
+        t[r] = -g[r] * u[r];
+      }
+#pragma unroll
+      for (int r = 0; r < TPT; r++) {
+        bx[r] = fma(t[r], dx[r], bx[r]);
+        by[r] = fma(t[r], dy[r], by[r]);
+        bz[r] = fma(t[r], dz[r], bz[r]);
+        bx[r] = fma(g[r], B.y, bx[r]);
+        by[r] = fma(g[r], C.x, by[r]);
+        bz[r] = fma(g[r], C.y, bz[r]);
+      }
+    }
   }
-  if (j < npl) {
-    qbar[oj] = kBiotSavart * qb;
-    ybar[oj] = kBiotSavart * s.w * bx;
-    ybar[N + oj] = kBiotSavart * s.w * by;
-    ybar[2 * N + oj] = kBiotSavart * s.w * bz;
+#pragma unroll
+  for (int r = 0; r < TPT; r++) {
+    const int j = threadIdx.x + r * NT;
+    sum[j] = qb[r];
+    sum[NSRC + j] = bx[r];
+    sum[2 * NSRC + j] = by[r];
+    sum[3 * NSRC + j] = bz[r];
   }
+  cluster_totals<4>(sum, NSRC, [&](int j, const double* v) {
+    if (j >= count) return;
+    const long o = o0 + j;
+    const double w = kBiotSavart * psrc[o].w;
+    qbar[o] = kBiotSavart * v[0];
+    ybar[o] = w * v[1];
+    ybar[N + o] = w * v[2];
+    ybar[2 * N + o] = w * v[3];
+  });
 }
 
 // Mixed-precision transposed near field: source leaf sl (blockIdx.x), one
@@ -308,35 +423,42 @@ __global__ void __launch_bounds__(kT) k_tree_cc_T32(StepGeom fg, const int* __re
 
 // 1-D barycentric basis on the leaf's Chebyshev proxies and its derivative,
 // without a range check (displaced particles may leave their leaf).
-__device__ __forceinline__ void bli_free_deriv(double t, double lo, double hi, int n, const BliTable& tab, double* f,
+template <int n>
+__device__ __forceinline__ void bli_free_deriv(double t, double lo, double hi, const BliTable& tab, double* f,
                                                double* df) {
   const double range = 0.5 * (hi - lo), offset = 0.5 * (hi + lo);
   int hit = -1;
+#pragma unroll
   for (int i = 0; i <= n; i++)
     if (hit < 0 && fabs(t - (tab.cosv[i] * range + offset)) < 1e-15) hit = i;
   if (hit >= 0) {
     const double th = tab.cosv[hit] * range + offset;
     double sum = 0;
+#pragma unroll
     for (int a = 0; a <= n; a++) {
       f[a] = a == hit ? 1.0 : 0.0;
       df[a] = a == hit ? 0.0 : (tab.w[a] / tab.w[hit]) / (th - (tab.cosv[a] * range + offset));
       sum += df[a];
     }
-    df[hit] = -sum;
+#pragma unroll
+    for (int a = 0; a <= n; a++) df[a] = a == hit ? -sum : df[a];
     return;
   }
   double S = 0, T = 0;
+#pragma unroll
   for (int k = 0; k <= n; k++) {
-    const double dk = t - (tab.cosv[k] * range + offset);
-    const double r = tab.w[k] / dk;
+    const double inv = 1.0 / (t - (tab.cosv[k] * range + offset));
+    const double r = tab.w[k] * inv;
     f[k] = r;
+    df[k] = inv;
     S += r;
-    T += r / dk;
+    T = fma(r, inv, T);
   }
   const double iS = 1.0 / S, TS = T * iS;
+#pragma unroll
   for (int a = 0; a <= n; a++) {
     f[a] *= iS;
-    df[a] = f[a] * (TS - 1.0 / (t - (tab.cosv[a] * range + offset)));
+    df[a] = f[a] * (TS - df[a]);
   }
 }
 
@@ -350,11 +472,13 @@ __device__ __forceinline__ void atan_grad2(double u, int iu, double su, double w
 // Anterpolation adjoint: particle j of tree leaf f (blockIdx.x) adds
 // sum_k B_k(y_j) Qbar_k to qbar_j and q_j sum_k grad B_k(y_j) Qbar_k to ybar_j,
 // B_k = Lx_a(xi(y)) Ly_b(eta(y)) on the leaf's face.
-__global__ void k_tree_sources_T(TreeGeom tg, StepGeom fg, BliTable tab, const double4* __restrict__ psrc,
+template <int PD>  // proxy degree (the bases stay in registers)
+__global__ void __launch_bounds__(kLeafThreads) k_tree_sources_T(TreeGeom tg, StepGeom fg, BliTable tab, const double4* __restrict__ psrc,
                                  const double* __restrict__ qbl, double* __restrict__ qbar,
                                  double* __restrict__ ybar) {
   extern __shared__ double sq[];  // the leaf's adjoint proxy strengths, qx
-  const int f = blockIdx.x, npl = tg.npl, n = tg.n, n1 = n + 1, qx = n1 * n1;
+  const int f = blockIdx.x, npl = tg.npl;
+  constexpr int n = PD, n1 = n + 1, qx = n1 * n1;
   const long N = tg.N;
   const int panel = fg.offset + f;
   for (int k = threadIdx.x; k < qx; k += blockDim.x) sq[k] = qbl[(long)panel * qx + k];
@@ -366,17 +490,23 @@ __global__ void k_tree_sources_T(TreeGeom tg, StepGeom fg, BliTable tab, const d
     const double4 s = psrc[o];
     double xi, eta;
     xieta_from_xyz_face(s.x, s.y, s.z, face, xi, eta);
-    double fx[kMaxDegree + 1], dfx[kMaxDegree + 1], fe[kMaxDegree + 1], dfe[kMaxDegree + 1];
-    bli_free_deriv(xi, bd[0], bd[1], n, tab, fx, dfx);
-    bli_free_deriv(eta, bd[2], bd[3], n, tab, fe, dfe);
+    double fx[n1], dfx[n1], fe[n1], dfe[n1];
+    bli_free_deriv<n>(xi, bd[0], bd[1], tab, fx, dfx);
+    bli_free_deriv<n>(eta, bd[2], bd[3], tab, fe, dfe);
     double val = 0, dxi = 0, deta = 0;
-    for (int a = 0; a <= n; a++)
+#pragma unroll
+    for (int a = 0; a <= n; a++) {
+      double row = 0, drow = 0;
+#pragma unroll
       for (int b = 0; b <= n; b++) {
         const double qk = sq[a * n1 + b];
-        val = fma(fx[a] * fe[b], qk, val);
-        dxi = fma(dfx[a] * fe[b], qk, dxi);
-        deta = fma(fx[a] * dfe[b], qk, deta);
+        row = fma(fe[b], qk, row);
+        drow = fma(dfe[b], qk, drow);
       }
+      val = fma(fx[a], row, val);
+      dxi = fma(dfx[a], row, dxi);
+      deta = fma(fx[a], drow, deta);
+    }
     double gxi[3], geta[3];
     const double X = s.x, Y = s.y, Z = s.z;
     switch (face) {
@@ -545,6 +675,43 @@ __global__ void k_nonleaf_positions_T(StepGeom g, double h, const double* __rest
   }
 }
 
+void launch_up3(const StepGeom& g, double* t, cudaStream_t st) {
+  for (int lev = g.levels - 2; lev >= 0; lev--)
+    SB_LAUNCH(k_tree_up3, dim3(6u << (2 * lev), 3), kT, sizeof(double) * 8 * g.q, st, g, lev, t);
+}
+
+void launch_down1(const StepGeom& g, double* qb, cudaStream_t st) {
+  for (int lev = 0; lev < g.levels - 1; lev++)
+    SB_LAUNCH(k_tree_down1, 6u << (2 * lev), kT, sizeof(double) * 3 * g.q, st, g, lev, qb);
+}
+
+template <int NT>
+void launch_near_T(const TreeGeom& tg, int leaves, const TreeAdjointLists& tl, const double* x, const double* y,
+                   const double* z, const double* vbar, const double4* psrc, double* qbar, double* ybar,
+                   cudaStream_t st) {
+  const int blocks = leaves * ((tg.npl + 2 * NT - 1) / (2 * NT));
+  const unsigned ranks = split_ranks(blocks);
+  if (tg.eps > 0)
+    launch_cluster(k_tree_near_T<NT, false>, blocks, ranks, NT, 0, st, tg, tl.near_tstart, tl.near_ttgt, x, y, z, vbar,
+                   psrc, qbar, ybar);
+  else
+    launch_cluster(k_tree_near_T<NT, true>, blocks, ranks, NT, 0, st, tg, tl.near_tstart, tl.near_ttgt, x, y, z, vbar,
+                   psrc, qbar, ybar);
+}
+
+void launch_sources_T(const TreeGeom& tg, const StepGeom& fg, const BliTable& ftab, const double4* psrc,
+                      const double* qbl, double* qbar, double* ybar, cudaStream_t st) {
+#define SB_ST(N)                                                                                             \
+  case N:                                                                                                    \
+    SB_LAUNCH(k_tree_sources_T<N>, (unsigned)fg.leaves, kLeafThreads, sizeof(double) * fg.q, st, tg, fg, ftab, \
+              psrc, qbl, qbar, ybar);                                                                        \
+    break;
+  switch (tg.n) {
+    SB_ST(1) SB_ST(2) SB_ST(3) SB_ST(4) SB_ST(5) SB_ST(6) SB_ST(7) SB_ST(8) SB_ST(9) SB_ST(10)
+  }
+#undef SB_ST
+}
+
 }  // namespace
 
 void launch_spectral_velocity_adjoint(const StepGeom& g, const int* tstart, const int* ttgt, const double* vbar,
@@ -557,19 +724,13 @@ void launch_spectral_velocity_adjoint(const StepGeom& g, const int* tstart, cons
   cudaMemsetAsync(tbar, 0, sizeof(double) * 3 * pn, st);
   for (int c = 0; c < 3; c++)
     cudaMemcpyAsync(tbar + c * pn + off, vbar + c * ln, sizeof(double) * ln, cudaMemcpyDeviceToDevice, st);
-  for (int lev = g.levels - 2; lev >= 0; lev--) {
-    const long work = (6L << (2 * lev)) * q * 3;
-    SB_LAUNCH(k_tree_up3, blocks_for(work, 256), 256, 0, st, g, lev, tbar);
-  }
+  launch_up3(g, tbar, st);
   if (q <= 4) launch_spec_interact_T_g<4>(g, mixed, tstart, ttgt, tbar, src, qbar, ybar_leaf, ybar_nl, st);
   else if (q <= 16) launch_spec_interact_T_g<16>(g, mixed, tstart, ttgt, tbar, src, qbar, ybar_leaf, ybar_nl, st);
   else if (q <= 32) launch_spec_interact_T_g<32>(g, mixed, tstart, ttgt, tbar, src, qbar, ybar_leaf, ybar_nl, st);
   else launch_spec_interact_T_g<kT>(g, mixed, tstart, ttgt, tbar, src, qbar, ybar_leaf, ybar_nl, st);
   // the strengths' upward pass transposed: interpolate their adjoints down
-  for (int lev = 0; lev < g.levels - 1; lev++) {
-    const long work = (6L << (2 * (lev + 1))) * q;
-    SB_LAUNCH(k_tree_down1, blocks_for(work, 256), 256, 0, st, g, lev, qbar);
-  }
+  launch_down1(g, qbar, st);
 }
 
 void launch_nonleaf_positions_adjoint(const StepGeom& g, double h, const double* vprev, const double* ybar_nl,
@@ -586,30 +747,24 @@ void launch_tree_velocity_adjoint(const TreeGeom& tg, const StepGeom& fg, const 
   const long pn = (long)Pf * qx;
   // leaf interpolation, transposed; non-leaf rows start at zero
   cudaMemsetAsync(tbar, 0, sizeof(double) * 3 * pn, st);
-  SB_LAUNCH(k_tree_to_particles_T, (unsigned)fg.leaves, kT, sizeof(double) * 3 * tg.npl, st, tg, fg, vbar, tbar);
-  // downward pass, transposed: accumulate up the tree
-  for (int lev = fg.levels - 2; lev >= 0; lev--) {
-    const long work = (6L << (2 * lev)) * qx * 3;
-    SB_LAUNCH(k_tree_up3, blocks_for(work, 256), 256, 0, st, fg, lev, tbar);
-  }
+  const int n1 = tg.n + 1, groups = kLeafThreads / qx > 0 ? kLeafThreads / qx : 1;
+  static std::atomic<unsigned long long> attr_t{0};
+  raise_smem_once(attr_t, 128 * 1024, k_tree_to_particles_T);
+  SB_LAUNCH(k_tree_to_particles_T, dim3((unsigned)fg.leaves, 3), kLeafThreads,
+            sizeof(double) * (tg.npl + 2 * tg.npl * n1 + groups * qx), st, tg, fg, vbar, tbar);
+  launch_up3(fg, tbar, st);
   // well-separated interactions, transposed
   if (mixed) {
     if (fg.eps > 0) SB_LAUNCH(k_tree_cc_T32<false>, (unsigned)Pf, kT, 0, st, fg, tl.cc_tstart, tl.cc_ttgt, tbar, qbl);
     else SB_LAUNCH(k_tree_cc_T32<true>, (unsigned)Pf, kT, 0, st, fg, tl.cc_tstart, tl.cc_ttgt, tbar, qbl);
   } else if (fg.eps > 0) {
-    SB_LAUNCH(k_tree_cc_T<false>, (unsigned)Pf, kT, 0, st, fg, tl.cc_tstart, tl.cc_ttgt, tbar, qbl);
+    launch_cluster(k_tree_cc_T<false>, Pf, split_ranks(Pf), kT, 0, st, fg, tl.cc_tstart, tl.cc_ttgt, tbar, qbl);
   } else {
-    SB_LAUNCH(k_tree_cc_T<true>, (unsigned)Pf, kT, 0, st, fg, tl.cc_tstart, tl.cc_ttgt, tbar, qbl);
+    launch_cluster(k_tree_cc_T<true>, Pf, split_ranks(Pf), kT, 0, st, fg, tl.cc_tstart, tl.cc_ttgt, tbar, qbl);
   }
   // upward pass, transposed: interpolate down the tree
-  for (int lev = 0; lev < fg.levels - 1; lev++) {
-    const long work = (6L << (2 * (lev + 1))) * qx;
-    SB_LAUNCH(k_tree_down1, blocks_for(work, 256), 256, 0, st, fg, lev, qbl);
-  }
+  launch_down1(fg, qbl, st);
   // near field, transposed (writes qbar, ybar), then the anterpolation adjoint (adds)
-  const size_t sm = sizeof(double) * 6 * tg.npl;
-  static std::atomic<unsigned long long> attr{0};
-  raise_smem_once(attr, 64 * 1024, k_tree_near_T<false>, k_tree_near_T<true>);
   const int nth = tg.npl <= 256 ? 256 : 512;
   if (mixed) {
     const size_t sm32 = sizeof(float4) * 3 * ((tg.npl + 1) / 2);
@@ -619,13 +774,12 @@ void launch_tree_velocity_adjoint(const TreeGeom& tg, const StepGeom& fg, const 
     else
       SB_LAUNCH(k_tree_near_T32<true>, (unsigned)fg.leaves, nth, sm32, st, tg, fg, tl.near_tstart, tl.near_ttgt, x, y,
                 z, vbar, psrc, qbar, ybar);
-  } else if (tg.eps > 0)
-    SB_LAUNCH(k_tree_near_T<false>, (unsigned)fg.leaves, nth, sm, st, tg, tl.near_tstart, tl.near_ttgt, x, y, z, vbar,
-              psrc, qbar, ybar);
-  else
-    SB_LAUNCH(k_tree_near_T<true>, (unsigned)fg.leaves, nth, sm, st, tg, tl.near_tstart, tl.near_ttgt, x, y, z, vbar,
-              psrc, qbar, ybar);
-  SB_LAUNCH(k_tree_sources_T, (unsigned)fg.leaves, kT, sizeof(double) * qx, st, tg, fg, ftab, psrc, qbl, qbar, ybar);
+  } else if (tg.npl <= 128) {
+    launch_near_T<64>(tg, fg.leaves, tl, x, y, z, vbar, psrc, qbar, ybar, st);
+  } else {
+    launch_near_T<128>(tg, fg.leaves, tl, x, y, z, vbar, psrc, qbar, ybar, st);
+  }
+  launch_sources_T(tg, fg, ftab, psrc, qbl, qbar, ybar, st);
 }
 
 }  // namespace sbslpm

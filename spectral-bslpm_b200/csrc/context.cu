@@ -4,6 +4,7 @@
 // piecewise entry points that mirror the reference's FMM functions.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -223,7 +224,10 @@ sbslpm_status precompute_tree(sbslpm_ctx* c) {
   SB_CUDA(cudaMemcpy(c->fsrc, init.data(), sizeof(double4) * pn, cudaMemcpyHostToDevice));
   SB_TRY(dalloc(&c->ftgt, 3 * pn));
   SB_TRY(dalloc(&c->psrc, N));
-  SB_TRY(dalloc(&c->near, (size_t)4 * 3 * N));
+  // up to four near-field splits; on trees of few leaves as many as give the
+  // GPU 16 blocks per SM (24,576 particles: 96 leaves), at most 16
+  c->near_max_splits = std::min(16, std::max(4, 148 * 16 / t.Af));
+  SB_TRY(dalloc(&c->near, (size_t)c->near_max_splits * 3 * N));
   if (c->cfg.precision == SBSLPM_MIXED) {
     SB_TRY(dalloc(&c->fsrcf, pn));
     SB_TRY(dalloc(&c->psrcf, N));
@@ -568,7 +572,7 @@ sbslpm_status cc_autotune(sbslpm_ctx* c) {
 }
 
 // Times every near-field launch shape (threads x targets per thread covering a
-// treecode leaf, 1..4 source-list splits) on the stage-0 sources and keeps the
+// treecode leaf, 1..4 source-list splits, on small trees up to 16) on the stage-0 sources and keeps the
 // fastest.  Runs once per context, before the first step, outside any capture.
 sbslpm_status near_autotune(sbslpm_ctx* c, const double* x, const double* y, const double* z, const double* area,
                             const double* vors) {
@@ -592,7 +596,7 @@ sbslpm_status near_autotune(sbslpm_ctx* c, const double* x, const double* y, con
   int cand = 0;
   for (const auto& sh : shapes) {
     if (sh[0] * sh[1] < c->npl || sh[0] * sh[1] >= 4 * c->npl) continue;
-    for (int sp = 1; sp <= 4; sp++) {
+    for (int sp = c->near_max_splits > 4 ? 2 : 1; sp <= c->near_max_splits; sp += sp < 4 ? 1 : 4) {
       auto run = [&] {
         launch_bltc_near_batch(c->self, 1, owned_leaves(c), c->npl, c->cfg.kernel_eps, prec, x, y, z, c->psrc,
                                c->psrcf, c->near, sp, sh[0], sh[1], c->near_expanded, st);

@@ -67,7 +67,8 @@ struct sbslpm_ctx {
   double4 *fsrc2 = nullptr, *psrc2 = nullptr;
   float4 *fsrcf2 = nullptr, *psrcf2 = nullptr;
   double* gx = nullptr;  // [3][particles]: the particle grid, for timing the near kernel alone
-  double* near = nullptr;  // [4][3][particles] near-field partial sums (near_splits in use)
+  int near_max_splits = 4;
+  double* near = nullptr;  // [near_max_splits][3][particles] near-field partial sums (near_splits in use)
   int near_splits = 2, near_nt = 128, near_tpt = 2;  // near-field launch shape (autotuned on the first step)
   // the mixed near field's pair form: expanded (near_expanded_ok at set-up,
   // or sbslpm_set_near_form) or difference

@@ -366,6 +366,26 @@ inline void raise_smem_once(std::atomic<unsigned long long>& done, int bytes, K.
   if (bit) done.fetch_or(bit, std::memory_order_acq_rel);
 }
 
+// A launch whose blocks (x, 0 .. ranks-1) form one cluster for every x.
+template <typename... P, typename... A>
+inline void launch_cluster(void (*kernel)(P...), unsigned blocks, unsigned ranks, unsigned threads, size_t smem,
+                           cudaStream_t st, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = 1;
+  at.val.clusterDim.y = ranks;
+  at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks, ranks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  launch_counter()++;
+}
+
 }  // namespace sbslpm
 
 #define SB_LAUNCH(kernel, grid, block, shmem, st, ...)      \
