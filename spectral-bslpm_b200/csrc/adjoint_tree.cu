@@ -644,7 +644,7 @@ void launch_spec_interact_T_g(const StepGeom& g, bool mixed, const int* tstart, 
 }
 
 // Non-leaf proxy positions, reversed: y_i = proj(p_i + h sum_m B_mi v[row_i + m])
-// (k_nonleaf_positions); vbar[c][row_i + m] += h B_mi J(p)^T ybar_i with
+// (nonleaf_position); vbar[c][row_i + m] += h B_mi J(p)^T ybar_i with
 // J(p)^T ybar = (ybar - yhat (yhat.ybar)) / |p|.  Proxies of one leaf row add
 // into the same velocity entries: double atomics.
 __global__ void k_nonleaf_positions_T(StepGeom g, double h, const double* __restrict__ vprev,

@@ -45,10 +45,12 @@ constexpr int kWarpsPerBlock = 4;
 __global__ void k_leaf_sources(StepGeom g, int stage, double dt_s, const double* __restrict__ vprev,
                                const double* __restrict__ x, const double* __restrict__ y,
                                const double* __restrict__ z, const double* __restrict__ vors,
-                               const double* __restrict__ area, double4* __restrict__ src) {
+                               const double* __restrict__ area, double4* __restrict__ src,
+                               double* __restrict__ keep) {
   long n = (long)g.leaves * g.q;
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
+  if (keep) keep[i] = vors[i];
   long pn = (long)g.panels * g.q;
   long o = (long)g.offset * g.q + i;
   double px = g.px[o], py = g.px[pn + o], pz = g.px[2 * pn + o];
@@ -103,29 +105,62 @@ __global__ void k_copy_strength(StepGeom g, const double4* __restrict__ src, dou
 // One CTA owns the subtree of depth D below one panel of level r and keeps
 // the strengths (upward) or target values (downward) of all its levels in
 // shared memory, so a pass over the whole tree takes ceil((L-1)/3) launches.
+// The passes are bound by latency (a chain of short phases between barriers):
+// the node count n1 is a template argument (index arithmetic without
+// divisions, contractions unrolled) and a CTA has a thread per point of its
+// widest level where it can.
 //
 // Upward, mode 0 (the step): when the subtree reaches the leaves, the leaf
 // sources are computed here (bve_disp_update, src/bve_time_step.cpp:69-105,
-// with the forcing copy and base_pots folded in); the non-leaf proxies of the
-// subtree get their displaced positions (bve_disp_interp,
+// with the forcing copy and base_pots folded in) and, at stage 0, the
+// vorticity is copied to `keep` for the remap; strengths are anterpolated
+// level by level; in mixed precision the packed float4 sources are written.
+// The displaced positions of the non-leaf proxies (bve_disp_interp,
 // src/bve_time_step.cpp:107-160, leaf row and BLI basis precomputed on the
-// host); strengths are anterpolated level by level; in mixed precision the
-// packed float4 sources are written for every panel the CTA owns.
+// host) come from the blocks past `roots` of the first launch, a thread per
+// point, beside the subtrees: they write the positions only, the subtrees the
+// strengths only.  Levels 5, degree 3, us per stage: positions 7.0, passes up
+// 13.1 and down 11.7 before; 7.9 and 8.3 now.
 // Mode 1 (sbslpm_upward_pass): leaf strengths area * pots, positions untouched.
 // Mode 2 (treecode): leaf strengths already anterpolated into src, fixed
 // proxy positions untouched, mixed packing as in mode 0.
 
+__device__ __forceinline__ float4 packed_source(const StepGeom& g, long panel, double x, double y, double z,
+                                                double w) {
+  const double* c = g.pd_centre + 4 * panel;
+  return make_float4((float)((x - c[0]) * kPackScale), (float)((y - c[1]) * kPackScale),
+                     (float)((z - c[2]) * kPackScale), (float)w);
+}
+
+template <int N1>
+__device__ __forceinline__ void nonleaf_source(const StepGeom& g, long i, int stage, double dt_s,
+                                               const double* __restrict__ vprev, double4* __restrict__ src,
+                                               int mixed) {
+  const int q = N1 > 0 ? N1 * N1 : g.q;
+  double px, py, pz;
+  nonleaf_position<N1 * N1>(g, i, stage, dt_s, vprev, px, py, pz);
+  src[i].x = px;
+  src[i].y = py;
+  src[i].z = pz;
+  if (mixed) {
+    const float4 f = packed_source(g, i / q, px, py, pz, 0.0);
+    g.srcf[i].x = f.x;
+    g.srcf[i].y = f.y;
+    g.srcf[i].z = f.z;
+  }
+}
+
+template <int N1>
 __device__ __forceinline__ void upward_subtree_body(const StepGeom& g, int root_rel, int r, int D, int mode,
-                                                    int positions, int stage, double dt_s,
-                                                    const double* __restrict__ vprev,
+                                                    int stage, double dt_s, const double* __restrict__ vprev,
                                                     const double* __restrict__ x, const double* __restrict__ y,
                                                     const double* __restrict__ z, const double* __restrict__ vors,
                                                     const double* __restrict__ area, double4* __restrict__ src,
-                                                    int mixed) {
+                                                    int mixed, double* __restrict__ keep) {
   extern __shared__ double sh[];  // strengths of levels r..r+D (level k at q*(4^k-1)/3), then scratch
-  const int q = g.q, n1 = g.degree + 1;
+  const int n1 = N1 > 0 ? N1 : g.degree + 1, q = N1 > 0 ? N1 * N1 : g.q;
   const bool leaves_here = (r + D == g.levels - 1);
-  const long ln = (long)g.leaves * g.q, pn = (long)g.panels * g.q;
+  const long ln = (long)g.leaves * q, pn = (long)g.panels * q;
   auto lvl = [&](int k) { return sh + q * (((1 << (2 * k)) - 1) / 3); };
 
   // bottom level of the subtree: leaf sources, or strengths computed by the previous launch
@@ -142,13 +177,15 @@ __device__ __forceinline__ void upward_subtree_body(const StepGeom& g, int root_
           src[o].w = w;
         } else {
           double px = g.px[o], py = g.px[pn + o], pz = g.px[2 * pn + o];
+          const double vor = vors[i];
+          if (keep) keep[i] = vor;
           if (stage == 0) {
-            w = area[i] * (g.force ? vors[i] + g.force[i] : vors[i]);
+            w = area[i] * (g.force ? vor + g.force[i] : vor);
           } else {
             double vx = vprev[i], vy = vprev[ln + i], vz = vprev[2 * ln + i];
             double xx = x[i] + vx * dt_s, yy = y[i] + vy * dt_s, zz = z[i] + vz * dt_s;
             project_to_sphere(xx, yy, zz);
-            double dvor = vors[i] + 2 * g.omega * z[i] - 2 * g.omega * zz;
+            double dvor = vor + 2 * g.omega * z[i] - 2 * g.omega * zz;
             w = area[i] * (g.force ? dvor + g.force[i] : dvor);
             px += dt_s * vx;
             py += dt_s * vy;
@@ -156,23 +193,13 @@ __device__ __forceinline__ void upward_subtree_body(const StepGeom& g, int root_
           }
           project_to_sphere(px, py, pz);
           src[o] = make_double4(px, py, pz, w);
+          if (mixed) g.srcf[o] = packed_source(g, o / q, px, py, pz, w);
         }
         bot[t] = w;
       } else {
-        bot[t] = src[o].w;
-      }
-    }
-  }
-  // displaced positions of the subtree's non-leaf proxies (levels r..r+D-1),
-  // unless k_nonleaf_positions wrote them before the pass
-  if (mode == 0 && positions) {
-    for (int k = 0; k < D; k++) {
-      const int first = subtree_first(r, root_rel, k), npts = (1 << (2 * k)) * q;
-      for (int t = threadIdx.x; t < npts; t += blockDim.x) {
-        const long i = (long)first * q + t;
-        double px, py, pz;
-        nonleaf_position(g, i, stage, dt_s, vprev, px, py, pz);
-        src[i] = make_double4(px, py, pz, 0.0);
+        const double4 v = src[o];
+        bot[t] = v.w;
+        if (mixed && leaves_here) g.srcf[o] = packed_source(g, o / q, v.x, v.y, v.z, v.w);
       }
     }
   }
@@ -188,95 +215,68 @@ __device__ __forceinline__ void upward_subtree_body(const StepGeom& g, int root_
       const double* ly = g.child_1d + ((cc & 3) >= 2 ? n1 * n1 : 0);
       const double* sc = ch + cc * q + i * n1;
       double acc = 0;
-      for (int j = 0; j < n1; j++) acc = fma(__ldg(ly + j * n1 + b), sc[j], acc);
+#pragma unroll
+      for (int j = 0; j < (N1 > 0 ? N1 : n1); j++) acc = fma(__ldg(ly + j * n1 + b), sc[j], acc);
       scratch[t] = acc;
     }
     __syncthreads();
     for (int t = threadIdx.x; t < np * q; t += blockDim.x) {  // S[p][a][b]
       const int p = t / q, rem = t % q, a = rem / n1, b = rem % n1;
       double acc = 0;
+#pragma unroll
       for (int c = 0; c < 4; c++) {
         const double* lx = g.child_1d + ((c == 1 || c == 2) ? n1 * n1 : 0);
         const double* tc = scratch + (4 * p + c) * q + b;
-        for (int i = 0; i < n1; i++) acc = fma(__ldg(lx + i * n1 + a), tc[i * n1], acc);
+#pragma unroll
+        for (int i = 0; i < (N1 > 0 ? N1 : n1); i++) acc = fma(__ldg(lx + i * n1 + a), tc[i * n1], acc);
       }
       pa[t] = acc;
-      src[(long)first * q + t].w = acc;
+      const long o = (long)first * q + t;
+      if (mixed && mode == 2) {
+        const double4 v = src[o];
+        g.srcf[o] = packed_source(g, o / q, v.x, v.y, v.z, acc);
+      } else if (mixed && mode == 0) {
+        g.srcf[o].w = (float)acc;
+      }
+      src[o].w = acc;
     }
     __syncthreads();
   }
-  // mixed precision: float4 sources relative to the panel centre, for every panel this CTA owns
-  if (mixed && mode != 1) {
-    const int kmax = leaves_here ? D : D - 1;
-    for (int k = 0; k <= kmax; k++) {
-      const int first = subtree_first(r, root_rel, k), npts = (1 << (2 * k)) * q;
-      for (int t = threadIdx.x; t < npts; t += blockDim.x) {
-        const long i = (long)first * q + t;
-        const double* cc = g.pd_centre + 4 * (i / q);
-        double4 sv = src[i];
-        g.srcf[i] = make_float4((float)((sv.x - cc[0]) * kPackScale), (float)((sv.y - cc[1]) * kPackScale),
-                                (float)((sv.z - cc[2]) * kPackScale), (float)sv.w);
-      }
-    }
-  }
 }
 
-__global__ void k_upward_subtree(StepGeom g, int r, int D, int mode, int positions, int stage, double dt_s,
-                                 const double* __restrict__ vprev, const double* __restrict__ x,
-                                 const double* __restrict__ y, const double* __restrict__ z,
-                                 const double* __restrict__ vors, const double* __restrict__ area,
-                                 double4* __restrict__ src, int mixed) {
-  upward_subtree_body(g, blockIdx.x, r, D, mode, positions, stage, dt_s, vprev, x, y, z, vors, area, src, mixed);
-}
+constexpr int kTreeThreads = 1024;
 
-// The displaced positions of every non-leaf proxy (bve_disp_interp,
-// src/bve_time_step.cpp:107-160) in one flat launch, a thread per point, ahead
-// of the subtree passes of mode 0: the same arithmetic as nonleaf_position,
-// with the q-term interpolation unrolled for q = 16, so that the passes
-// themselves no longer wait on these gathers level by level.
-template <int Q>
-__global__ void k_nonleaf_positions(StepGeom g, int stage, double dt_s, const double* __restrict__ vprev,
-                                    double4* __restrict__ src) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const int q = Q > 0 ? Q : g.q;
-  if (i >= (long)g.offset * q) return;
-  const long pn = (long)g.panels * q, ln = (long)g.leaves * q;
-  double px = g.px[i], py = g.px[pn + i], pz = g.px[2 * pn + i];
-  if (stage > 0) {
-    const long np = (long)g.offset * q;
-    const long row = (long)g.il_row[i] * q;
-    double ax = 0, ay = 0, az = 0;
-#pragma unroll
-    for (int m = 0; m < (Q > 0 ? Q : q); m++) {
-      const double bm = g.il_basis[m * np + i];
-      ax += (dt_s * vprev[row + m]) * bm;
-      ay += (dt_s * vprev[ln + row + m]) * bm;
-      az += (dt_s * vprev[2 * ln + row + m]) * bm;
-    }
-    px += ax;
-    py += ay;
-    pz += az;
+template <int N1>
+__global__ void __launch_bounds__(kTreeThreads)
+    k_upward_subtree(StepGeom g, int roots, int chunk, int r, int D, int mode, int stage, double dt_s,
+                     const double* __restrict__ vprev, const double* __restrict__ x, const double* __restrict__ y,
+                     const double* __restrict__ z, const double* __restrict__ vors, const double* __restrict__ area,
+                     double4* __restrict__ src, int mixed, double* __restrict__ keep) {
+  if ((int)blockIdx.x >= roots) {
+    const long i = ((long)blockIdx.x - roots) * chunk + threadIdx.x;
+    if ((int)threadIdx.x < chunk && i < (long)g.offset * (N1 > 0 ? N1 * N1 : g.q)) nonleaf_source<N1>(g, i, stage, dt_s, vprev, src, mixed);
+    return;
   }
-  project_to_sphere(px, py, pz);
-  src[i] = make_double4(px, py, pz, 0.0);
+  upward_subtree_body<N1>(g, blockIdx.x, r, D, mode, stage, dt_s, vprev, x, y, z, vors, area, src, mixed, keep);
 }
 
 // Batched treecode members (mode 2): member blockIdx.z.
 __global__ void k_upward_subtree_batch(const BatchMember* __restrict__ mem, int r, int D, int mixed) {
   const StepGeom g = mem[blockIdx.z].fg;
-  upward_subtree_body(g, blockIdx.x, r, D, 2, 0, 0, 0.0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                      mem[blockIdx.z].fsrc, mixed);
+  upward_subtree_body<0>(g, blockIdx.x, r, D, 2, 0, 0.0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+                         mem[blockIdx.z].fsrc, mixed, nullptr);
 }
 
 // Downward: the root's targets are final; children of levels r+1..r+D get
 // own + interpolated parent values.  Leaves go to leaf_out when given (the
 // stage velocity), intermediate levels stay in shared memory, and the
 // deepest non-leaf level is written back for the next launch.
+template <int N1>
 __device__ __forceinline__ void downward_subtree_body(const StepGeom& g, int root_rel, int r, int D,
                                                       double* __restrict__ tgt, double* __restrict__ leaf_out) {
   extern __shared__ double sh[];  // 3 fields x levels r..r+D, then 3 x 4^D q scratch
-  const int q = g.q, n1 = g.degree + 1;
-  const long pn = (long)g.panels * g.q, ln = (long)g.leaves * g.q;
+  const int n1 = N1 > 0 ? N1 : g.degree + 1, q = N1 > 0 ? N1 * N1 : g.q;
+  const long pn = (long)g.panels * q, ln = (long)g.leaves * q;
   const int per_field = q * (((1 << (2 * (D + 1))) - 1) / 3);
   auto lvl = [&](int f, int k) { return sh + f * per_field + q * (((1 << (2 * k)) - 1) / 3); };
   double* scratch = sh + 3 * per_field;
@@ -297,7 +297,8 @@ __device__ __forceinline__ void downward_subtree_body(const StepGeom& g, int roo
       const double *p0 = lvl(0, k - 1) + pp * q + a * n1, *p1 = lvl(1, k - 1) + pp * q + a * n1,
                    *p2 = lvl(2, k - 1) + pp * q + a * n1;
       double u0 = 0, u1 = 0, u2 = 0;
-      for (int b = 0; b < n1; b++) {
+#pragma unroll
+      for (int b = 0; b < (N1 > 0 ? N1 : n1); b++) {
         const double l = __ldg(ly + b);
         u0 = fma(l, p0[b], u0);
         u1 = fma(l, p1[b], u1);
@@ -313,7 +314,8 @@ __device__ __forceinline__ void downward_subtree_body(const StepGeom& g, int roo
       const double* lx = g.child_1d + ((c == 1 || c == 2) ? n1 * n1 : 0) + i * n1;
       const double* u = scratch + cc * q + j;
       double a0 = 0, a1 = 0, a2 = 0;
-      for (int a = 0; a < n1; a++) {
+#pragma unroll
+      for (int a = 0; a < (N1 > 0 ? N1 : n1); a++) {
         const double l = __ldg(lx + a);
         a0 = fma(l, u[a * n1], a0);
         a1 = fma(l, u[sstride + a * n1], a1);
@@ -341,14 +343,15 @@ __device__ __forceinline__ void downward_subtree_body(const StepGeom& g, int roo
   }
 }
 
-__global__ void k_downward_subtree(StepGeom g, int r, int D, double* __restrict__ tgt,
-                                   double* __restrict__ leaf_out) {
-  downward_subtree_body(g, blockIdx.x, r, D, tgt, leaf_out);
+template <int N1>
+__global__ void __launch_bounds__(kTreeThreads)
+    k_downward_subtree(StepGeom g, int r, int D, double* __restrict__ tgt, double* __restrict__ leaf_out) {
+  downward_subtree_body<N1>(g, blockIdx.x, r, D, tgt, leaf_out);
 }
 
 __global__ void k_downward_subtree_batch(const BatchMember* __restrict__ mem, int r, int D) {
   const StepGeom g = mem[blockIdx.z].fg;
-  downward_subtree_body(g, blockIdx.x, r, D, mem[blockIdx.z].ftgt, nullptr);
+  downward_subtree_body<0>(g, blockIdx.x, r, D, mem[blockIdx.z].ftgt, nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -936,16 +939,23 @@ __device__ __forceinline__ void depart_remap_body(const StepGeom& g, const BliTa
 // the chain of four locate -> gather rounds per particle is latency-bound,
 // and the extra resident warps measured 9 us per launch faster at 393,216
 // particles (78 vs 87 us) than the 76-register build.
-template <int D>
+template <int D, int MODE>
 __global__ void __launch_bounds__(128, 8) k_depart_remap(StepGeom g, BliTable tab, const double* __restrict__ x, const double* __restrict__ y,
                                const double* __restrict__ z, const double* __restrict__ v0,
                                const double* __restrict__ v1, const double* __restrict__ v2,
                                const double* __restrict__ v3, double dt, double* __restrict__ dep,
                                const double* __restrict__ vors, const double* __restrict__ tracers, int T,
-                               double* __restrict__ new_vors, double* __restrict__ new_tracers, int mode) {
+                               double* __restrict__ new_vors, double* __restrict__ new_tracers,
+                               VelocityOut out) {
   const long o = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (o >= (long)g.leaves * g.q) return;
-  depart_remap_body<D>(g, tab, o, x, y, z, v0, v1, v2, v3, dt, dep, vors, tracers, T, new_vors, new_tracers, mode);
+  const long n = (long)g.leaves * g.q;
+  if (o >= n) return;
+  if (out.x) {
+    out.x[o] = v0[o];
+    out.y[o] = v0[n + o];
+    out.z[o] = v0[2 * n + o];
+  }
+  depart_remap_body<D>(g, tab, o, x, y, z, v0, v1, v2, v3, dt, dep, vors, tracers, T, new_vors, new_tracers, MODE);
 }
 
 // Batched members on one particle grid (member blockIdx.y): departure and
@@ -1214,9 +1224,9 @@ using dev::blocks_for;
 
 void launch_leaf_sources(const StepGeom& g, int stage, double dt_s, const double* vprev, const double* x,
                          const double* y, const double* z, const double* vors, const double* area, double4* src,
-                         cudaStream_t st) {
+                         cudaStream_t st, double* keep) {
   long n = (long)g.leaves * g.q;
-  SB_LAUNCH(k_leaf_sources, blocks_for(n, 256), 256, 0, st, g, stage, dt_s, vprev, x, y, z, vors, area, src);
+  SB_LAUNCH(k_leaf_sources, blocks_for(n, 256), 256, 0, st, g, stage, dt_s, vprev, x, y, z, vors, area, src, keep);
 }
 
 void launch_sources_from_disp(const StepGeom& g, const double* dx, const double* dy, const double* dz,
@@ -1239,28 +1249,51 @@ static size_t subtree_smem(int q, int fields, int D) {
   return (size_t)q * fields * 8 * ((((1L << (2 * (D + 1))) - 1) / 3) + (1L << (2 * D)));
 }
 
+// A thread per point of a subtree's bottom level, up to kTreeThreads.
+static unsigned subtree_threads(int q, int D) {
+  return std::min((unsigned)kTreeThreads, (unsigned)(((q << (2 * D)) + 31) / 32 * 32));
+}
+
+// f(std::integral_constant<int, N1>) for the node count per direction, 0 where
+// no kernel is built for it.
+template <class F>
+static void with_n1(int degree, F f) {
+  switch (degree + 1) {
+    case 3: f(std::integral_constant<int, 3>()); break;
+    case 4: f(std::integral_constant<int, 4>()); break;
+    case 5: f(std::integral_constant<int, 5>()); break;
+    case 6: f(std::integral_constant<int, 6>()); break;
+    case 7: f(std::integral_constant<int, 7>()); break;
+    case 8: f(std::integral_constant<int, 8>()); break;
+    case 9: f(std::integral_constant<int, 9>()); break;
+    case 10: f(std::integral_constant<int, 10>()); break;
+    case 11: f(std::integral_constant<int, 11>()); break;
+    default: f(std::integral_constant<int, 0>()); break;
+  }
+}
+
 void launch_upward_fused(const StepGeom& g, int mode, int stage, double dt_s, const double* vprev, const double* x,
                          const double* y, const double* z, const double* vors, const double* area, double4* src,
-                         bool mixed, cudaStream_t st) {
-  static std::atomic<unsigned long long> attr{0};
-  raise_smem_once(attr, 164 * 1024, k_upward_subtree);
-  const int Dmax = subtree_depth(g.q);
-  int r = g.levels - 1;  // the bottom of the next subtree
-  const long nl = (long)g.offset * g.q;  // non-leaf proxy points
-  const bool flat = mode == 0 && nl > 0;
-  if (flat) {
-    if (g.q == 16) SB_LAUNCH(k_nonleaf_positions<16>, blocks_for(nl, 256), 256, 0, st, g, stage, dt_s, vprev, src);
-    else SB_LAUNCH(k_nonleaf_positions<0>, blocks_for(nl, 256), 256, 0, st, g, stage, dt_s, vprev, src);
-  }
-  bool first = true;
-  while (first || r > 0) {
-    int D = first ? (r < Dmax ? r : Dmax) : (r < Dmax ? r : Dmax);
-    int root = r - D;
-    SB_LAUNCH(k_upward_subtree, (unsigned)(6 << (2 * root)), 256, subtree_smem(g.q, 1, D), st, g, root, D, mode,
-              flat ? 0 : 1, stage, dt_s, vprev, x, y, z, vors, area, src, mixed ? 1 : 0);
-    r = root;
-    first = false;
-  }
+                         bool mixed, cudaStream_t st, double* keep) {
+  with_n1(g.degree, [&](auto n1) {
+    static std::atomic<unsigned long long> attr{0};
+    raise_smem_once(attr, 164 * 1024, k_upward_subtree<n1.value>);
+    const int Dmax = subtree_depth(g.q);
+    int r = g.levels - 1;  // the bottom of the next subtree
+    bool first = true;
+    while (first || r > 0) {
+      const int D = r < Dmax ? r : Dmax, root = r - D, roots = 6 << (2 * root);
+      const unsigned threads = subtree_threads(g.q, D);
+      // the non-leaf proxies' positions beside the first launch's subtrees
+      const long points = first && mode == 0 ? (long)g.offset * g.q : 0;
+      const int chunk = nonleaf_chunk(points, threads);
+      const unsigned extra = blocks_for(points, chunk);
+      SB_LAUNCH(k_upward_subtree<n1.value>, roots + extra, threads, subtree_smem(g.q, 1, D), st, g, roots, chunk, root, D,
+                mode, stage, dt_s, vprev, x, y, z, vors, area, src, mixed ? 1 : 0, keep);
+      r = root;
+      first = false;
+    }
+  });
 }
 
 void launch_upward_batch(const BatchMember* mem, int members, int levels, int qmax, bool mixed, cudaStream_t st) {
@@ -1312,16 +1345,18 @@ void launch_cc_batch(const BatchMember* mem, const int* idx, int count, int q, i
 }
 
 void launch_downward_fused(const StepGeom& g, double* tgt, double* leaf_out, cudaStream_t st) {
-  static std::atomic<unsigned long long> attr{0};
-  raise_smem_once(attr, 164 * 1024, k_downward_subtree);
-  const int Dmax = subtree_depth(g.q);
-  int r = 0;
-  while (r < g.levels - 1) {
-    int D = (g.levels - 1 - r) < Dmax ? (g.levels - 1 - r) : Dmax;
-    SB_LAUNCH(k_downward_subtree, (unsigned)(6 << (2 * r)), 256, subtree_smem(g.q, 3, D), st, g, r, D, tgt,
-              leaf_out);
-    r += D;
-  }
+  with_n1(g.degree, [&](auto n1) {
+    static std::atomic<unsigned long long> attr{0};
+    raise_smem_once(attr, 164 * 1024, k_downward_subtree<n1.value>);
+    const int Dmax = subtree_depth(g.q);
+    int r = 0;
+    while (r < g.levels - 1) {
+      const int D = (g.levels - 1 - r) < Dmax ? (g.levels - 1 - r) : Dmax;
+      SB_LAUNCH(k_downward_subtree<n1.value>, (unsigned)(6 << (2 * r)), subtree_threads(g.q, D),
+                subtree_smem(g.q, 3, D), st, g, r, D, tgt, leaf_out);
+      r += D;
+    }
+  });
 }
 
 namespace {
@@ -1447,18 +1482,23 @@ void launch_direct_leaves(const StepGeom& g, int precision, const double4* src, 
 void launch_depart_remap(const StepGeom& g, const BliTable* tab, const double* x, const double* y, const double* z,
                          const double* v0, const double* v1, const double* v2, const double* v3, double dt,
                          double* dep, const double* vors, const double* tracers, int T, double* new_vors,
-                         double* new_tracers, int mode, cudaStream_t st) {
+                         double* new_tracers, int mode, cudaStream_t st, VelocityOut vel) {
   long n = (long)g.leaves * g.q;
   unsigned grid = blocks_for(n, 128);
-#define SB_DR(D)                                                                                                   \
-  case D:                                                                                                          \
-    SB_LAUNCH(k_depart_remap<D>, grid, 128, 0, st, g, *tab, x, y, z, v0, v1, v2, v3, dt, dep, vors, tracers, T,   \
-              new_vors, new_tracers, mode);                                                                        \
+#define SB_DRM(D, MODE)                                                                                            \
+  SB_LAUNCH((k_depart_remap<D, MODE>), grid, 128, 0, st, g, *tab, x, y, z, v0, v1, v2, v3, dt, dep, vors, tracers, \
+            T, new_vors, new_tracers, vel)
+#define SB_DR(D)                     \
+  case D:                            \
+    if (mode == 1) SB_DRM(D, 1);     \
+    else if (mode == 2) SB_DRM(D, 2); \
+    else SB_DRM(D, 3);               \
     break;
   switch (g.degree) {
     SB_DR(0) SB_DR(1) SB_DR(2) SB_DR(3) SB_DR(4) SB_DR(5) SB_DR(6) SB_DR(7) SB_DR(8) SB_DR(9) SB_DR(10)
   }
 #undef SB_DR
+#undef SB_DRM
 }
 
 void launch_depart_remap_batch(const StepGeom& g, const BliTable* tab, int members, const double* x,

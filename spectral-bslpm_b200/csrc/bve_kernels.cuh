@@ -76,17 +76,25 @@ struct BatchMember {
   double* ftgt;   // [3][tree panels * q] proxy targets
 };
 
-// Launch wrappers (stream-ordered).
+// Where the step's first-stage velocity goes (null: nowhere).
+struct VelocityOut {
+  double* x = nullptr;
+  double* y = nullptr;
+  double* z = nullptr;
+};
+
+// Launch wrappers (stream-ordered).  keep, where given, receives a copy of
+// vors (the remap then gathers from it and writes vors in place).
 void launch_leaf_sources(const StepGeom& g, int stage, double dt_s, const double* vprev, const double* x,
                          const double* y, const double* z, const double* vors, const double* area, double4* src,
-                         cudaStream_t st);
+                         cudaStream_t st, double* keep = nullptr);
 // Fused passes: whole tree in ceil((levels-1)/3) launches.  mode 0 = the
 // step's sources (leaf sources, non-leaf positions, strengths, mixed
 // packing); mode 1 = strengths area*pots only; mode 2 = leaf strengths
 // already in src (treecode proxies), mixed packing.
 void launch_upward_fused(const StepGeom& g, int mode, int stage, double dt_s, const double* vprev, const double* x,
                          const double* y, const double* z, const double* vors, const double* area, double4* src,
-                         bool mixed, cudaStream_t st);
+                         bool mixed, cudaStream_t st, double* keep = nullptr);
 // leaf_out == nullptr: leaf values stay in tgt.
 void launch_downward_fused(const StepGeom& g, double* tgt, double* leaf_out, cudaStream_t st);
 void launch_interactions(const StepGeom& g, int precision, const double4* src, double* tgt, bool accumulate,
@@ -96,7 +104,7 @@ void launch_direct_leaves(const StepGeom& g, int precision, const double4* src, 
 void launch_depart_remap(const StepGeom& g, const BliTable* tab, const double* x, const double* y, const double* z,
                          const double* v0, const double* v1, const double* v2, const double* v3, double dt,
                          double* dep, const double* vors, const double* tracers, int tracer_count, double* new_vors,
-                         double* new_tracers, int mode, cudaStream_t st);
+                         double* new_tracers, int mode, cudaStream_t st, VelocityOut vel = {});
 // Raw-array helpers for the piecewise API.
 void launch_sources_from_disp(const StepGeom& g, const double* dx, const double* dy, const double* dz,
                               const double* source, double4* src, cudaStream_t st);

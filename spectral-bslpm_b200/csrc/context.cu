@@ -362,13 +362,14 @@ void launch_tree_cc(sbslpm_ctx* c, cudaStream_t st) {
   }
 }
 
-// One velocity evaluation (one RK4 stage) into v (contiguous [3][leaves*q]).
+// One velocity evaluation (one RK4 stage) into v (contiguous [3][leaves*q]);
+// keep, where given, receives a copy of vors.
 void velocity_eval(sbslpm_ctx* c, int stage, double dt_s, const double* vprev, const double* x, const double* y,
-                   const double* z, const double* area, const double* vors, double* v) {
+                   const double* z, const double* area, const double* vors, double* v, double* keep) {
   cudaStream_t st = c->stream();
   const StepGeom& g = c->geom;
   if (c->cfg.velocity == SBSLPM_VEL_DIRECT) {
-    launch_leaf_sources(g, stage, dt_s, vprev, x, y, z, vors, area, c->src, st);
+    launch_leaf_sources(g, stage, dt_s, vprev, x, y, z, vors, area, c->src, st, keep);
     launch_direct_leaves(g, c->cfg.precision, c->src, v, c->partial, c->groups, st);
     return;
   }
@@ -377,6 +378,7 @@ void velocity_eval(sbslpm_ctx* c, int stage, double dt_s, const double* vprev, c
     const StepGeom& fg = c->fgeom;
     launch_bltc_sources(c->tgeom, fg, c->ftab, stage, dt_s, vprev, x, y, z, vors, area, c->psrc, c->psrcf, c->fsrc,
                         mixed, st);
+    if (keep) cudaMemcpyAsync(keep, vors, sizeof(double) * c->tgeom.N, cudaMemcpyDeviceToDevice, st);
     // the tree passes (proxy sources up, well-separated pairs, proxy targets
     // down) depend only on the leaf proxies, the near field only on the
     // particle sources: the tree runs on the auxiliary stream beside it
@@ -402,7 +404,7 @@ void velocity_eval(sbslpm_ctx* c, int stage, double dt_s, const double* vprev, c
     launch_bltc_to_particles(c->tgeom, fg, c->ftgt, c->near, splits, v, st);
     return;
   }
-  launch_upward_fused(g, 0, stage, dt_s, vprev, x, y, z, vors, area, c->src, mixed, st);
+  launch_upward_fused(g, 0, stage, dt_s, vprev, x, y, z, vors, area, c->src, mixed, st, keep);
   launch_interactions_only(g, c->cfg.precision, c->src, c->tgt, st);
   if (c->L == 1) {
     cudaMemcpyAsync(v, c->tgt, sizeof(double) * 3 * c->P * c->q, cudaMemcpyDeviceToDevice, st);
@@ -430,7 +432,8 @@ void enqueue_step(sbslpm_ctx* c, const double* x, const double* y, const double*
   for (int s = 0; s < 4; s++) {
     {
       NvtxRange r(stage_name[s]);
-      velocity_eval(c, s, stage_dt[s], s ? v[s - 1] : nullptr, x, y, z, area, vors, v[s]);
+      // the first stage's sources leave a copy of the vorticity, which the remap reads
+      velocity_eval(c, s, stage_dt[s], s ? v[s - 1] : nullptr, x, y, z, area, vors, v[s], s ? nullptr : c->newvor);
     }
     if (c->nccl_comm) {
       NvtxRange r("sbslpm stage velocity all-gather");
@@ -441,15 +444,9 @@ void enqueue_step(sbslpm_ctx* c, const double* x, const double* y, const double*
   if (c->force) launch_time_advance(c->d_time, dt, st);
   const int T = c->cfg.tracer_count;
   NvtxRange remap_range("sbslpm departure + remap");
-  launch_depart_remap(c->geom, &c->tab, x, y, z, v[0], v[1], v[2], v[3], dt, c->dep, vors, tracers, T, c->newvor,
-                      c->newtr, 3, st);
-  cudaMemcpyAsync(vors, c->newvor, sizeof(double) * ln, cudaMemcpyDeviceToDevice, st);
+  launch_depart_remap(c->geom, &c->tab, x, y, z, v[0], v[1], v[2], v[3], dt, c->dep, c->newvor, tracers, T, vors,
+                      c->newtr, 3, st, VelocityOut{vel_x, vel_y, vel_z});
   if (T > 0) cudaMemcpyAsync(tracers, c->newtr, sizeof(double) * ln * T, cudaMemcpyDeviceToDevice, st);
-  if (vel_x) {
-    cudaMemcpyAsync(vel_x, v[0], sizeof(double) * ln, cudaMemcpyDeviceToDevice, st);
-    cudaMemcpyAsync(vel_y, v[0] + ln, sizeof(double) * ln, cudaMemcpyDeviceToDevice, st);
-    cudaMemcpyAsync(vel_z, v[0] + 2 * ln, sizeof(double) * ln, cudaMemcpyDeviceToDevice, st);
-  }
 }
 
 // Waits for the stream, then turns launch errors and the device error word

@@ -190,7 +190,7 @@ void enqueue_step(sbslpm_ctx* c, const double* x, const double* y, const double*
                   double* vel_x, double* vel_y, double* vel_z, double* tracers,
                   cudaEvent_t stage0 = nullptr);
 void velocity_eval(sbslpm_ctx* c, int stage, double dt_s, const double* vprev, const double* x, const double* y,
-                   const double* z, const double* area, const double* vors, double* v);
+                   const double* z, const double* area, const double* vors, double* v, double* keep = nullptr);
 void launch_add3(const double* t, long n, double* a, double* b, double* cc, cudaStream_t st);
 sbslpm_status install_cc_lists(sbslpm_ctx* c, const std::vector<int>& cs, const std::vector<int>& csrc);
 // shard.cpp: all-gathers a stage velocity [3][particles] over the context's

@@ -168,19 +168,24 @@ __device__ __forceinline__ int subtree_first(int level, int root_rel, int k) {
   return level_start(level + k) + (root_rel << (2 * k));
 }
 
+// Displaced, re-projected position of non-leaf proxy i: its containing leaf's
+// BLI interpolation of dt_s * vprev, unrolled where Q (= q) is given.
+template <int Q>
 __device__ __forceinline__ void nonleaf_position(const StepGeom& g, long i, int stage, double dt_s,
                                                  const double* __restrict__ vprev, double& px, double& py,
                                                  double& pz) {
-  const long pn = (long)g.panels * g.q, ln = (long)g.leaves * g.q;
+  const int q = Q > 0 ? Q : g.q;
+  const long pn = (long)g.panels * q, ln = (long)g.leaves * q;
   px = g.px[i];
   py = g.px[pn + i];
   pz = g.px[2 * pn + i];
   if (stage > 0) {
-    const long np = (long)g.offset * g.q;
-    const long row = (long)g.il_row[i] * g.q;
+    const long np = (long)g.offset * q;
+    const long row = (long)g.il_row[i] * q;
     double ax = 0, ay = 0, az = 0;
-    for (int m = 0; m < g.q; m++) {
-      double bm = g.il_basis[m * np + i];
+#pragma unroll
+    for (int m = 0; m < (Q > 0 ? Q : q); m++) {
+      const double bm = g.il_basis[m * np + i];
       ax += (dt_s * vprev[row + m]) * bm;
       ay += (dt_s * vprev[ln + row + m]) * bm;
       az += (dt_s * vprev[2 * ln + row + m]) * bm;
@@ -191,7 +196,6 @@ __device__ __forceinline__ void nonleaf_position(const StepGeom& g, long i, int 
   }
   project_to_sphere(px, py, pz);
 }
-
 
 // Point location + tensor-product BLI basis at a point (point_locate_panel
 // and interp_vals_bli, src/interp_funcs_impl.hpp:11-142), and gathers of a
@@ -258,7 +262,8 @@ __device__ __forceinline__ void bli_1d_common(double t, double lo, double hi, co
 }
 
 __device__ __forceinline__ void project_to_sphere_rcp(double& x, double& y, double& z) {
-  const double inv = 1.0 / sqrt(x * x + y * y + z * z);
+  // written out: the single and the batched step's kernels must contract alike
+  const double inv = 1.0 / sqrt(fma(z, z, fma(y, y, x * x)));
   x *= inv;
   y *= inv;
   z *= inv;
@@ -343,6 +348,13 @@ __device__ __forceinline__ void gather3(const Basis<D>& b, const double* __restr
       c += v[n + b.row + m] * bm;
       e += v[2 * n + b.row + m] * bm;
     }
+}
+
+// Non-leaf points per block of an upward pass's first launch: few enough that
+// the points reach every SM (all threads of the block where there are many).
+inline int nonleaf_chunk(long points, unsigned threads) {
+  const long per = (points / 148 + 31) / 32 * 32;
+  return (int)(per < 128 ? (threads < 128 ? threads : 128) : per < threads ? per : threads);
 }
 
 inline unsigned blocks_for(long n, int t) { return (unsigned)((n + t - 1) / t); }

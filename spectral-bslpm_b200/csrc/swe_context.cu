@@ -205,13 +205,9 @@ void swe_enqueue_step(sbslpm_ctx* c, const double* x, const double* y, const dou
   StepGeom g0 = g;
   g0.omega = 0.0;
   const int nt = c->cfg.tracer_count;
-  launch_depart_remap(g0, &c->tab, x, y, z, v[0], v[1], v[2], v[3], dt, c->dep, c->avor, tracers, nt, c->newvor,
-                      c->newtr, 3, st);
-  cudaMemcpyAsync(vors, c->newvor, sizeof(double) * ln, cudaMemcpyDeviceToDevice, st);
+  launch_depart_remap(g0, &c->tab, x, y, z, v[0], v[1], v[2], v[3], dt, c->dep, c->avor, tracers, nt, vors,
+                      c->newtr, 3, st, VelocityOut{vel_x, vel_y, vel_z});
   if (nt > 0) cudaMemcpyAsync(tracers, c->newtr, sizeof(double) * ln * nt, cudaMemcpyDeviceToDevice, st);
-  cudaMemcpyAsync(vel_x, v[0], sizeof(double) * ln, cudaMemcpyDeviceToDevice, st);
-  cudaMemcpyAsync(vel_y, v[0] + ln, sizeof(double) * ln, cudaMemcpyDeviceToDevice, st);
-  cudaMemcpyAsync(vel_z, v[0] + 2 * ln, sizeof(double) * ln, cudaMemcpyDeviceToDevice, st);
 }
 
 bool bad(const void* p) { return p == nullptr; }

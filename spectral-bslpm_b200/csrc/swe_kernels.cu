@@ -14,6 +14,7 @@
 // Every kernel is owner-computes (no atomics) and deterministic.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "../../include/sbslpm.h"
@@ -55,22 +56,61 @@ __device__ __forceinline__ float4 pack(const double* c, double x, double y, doub
                      (float)((z - c[2]) * kPackScale), (float)w);
 }
 
+// Positions of the non-leaf proxies of both fields (swe_disp_interp_2,
+// src/swe_time_step_2.cpp:436-476, identical to the BVE form): the vorticity
+// sources displaced by the interpolated leaf velocity, the divergence sources
+// at the fixed proxies.  Positions only; the subtrees write the strengths.
+template <int N1>
+__device__ __forceinline__ void swe_nonleaf_source(const StepGeom& g, const SweGeom& sw, long i, int stage, double dtd,
+                                                   const double* __restrict__ vprev, double4* __restrict__ src,
+                                                   double4* __restrict__ src2, int mixed) {
+  const int q = N1 > 0 ? N1 * N1 : g.q;
+  const long pn = (long)g.panels * q;
+  const double x0 = g.px[i], y0 = g.px[pn + i], z0 = g.px[2 * pn + i];
+  double px, py, pz;
+  nonleaf_position<N1 * N1>(g, i, stage, dtd, vprev, px, py, pz);
+  src[i].x = px;
+  src[i].y = py;
+  src[i].z = pz;
+  src2[i].x = x0;
+  src2[i].y = y0;
+  src2[i].z = z0;
+  if (mixed) {
+    const double* c = g.pd_centre + 4 * (i / q);
+    const float4 a = pack(c, px, py, pz, 0.0), b = pack(c, x0, y0, z0, 0.0);
+    g.srcf[i].x = a.x;
+    g.srcf[i].y = a.y;
+    g.srcf[i].z = a.z;
+    sw.srcf2[i].x = b.x;
+    sw.srcf2[i].y = b.y;
+    sw.srcf2[i].z = b.z;
+  }
+}
+
 // Fused upward pass over one subtree (the SWE form of k_upward_subtree): leaf
-// sources of both fields when the subtree reaches the leaves, displaced
-// positions of its non-leaf proxies (swe_disp_interp_2,
-// src/swe_time_step_2.cpp:436-476, identical to the BVE form), both strengths
+// sources of both fields when the subtree reaches the leaves, both strengths
 // anterpolated level by level (upward_pass, src/fmm_funcs.cpp:341-355), and
-// the packed float sources in mixed precision.
-__global__ void k_swe_upward_subtree(StepGeom g, SweGeom sw, int r, int D, int positions, int stage, double dtd,
-                                     double dts,
-                                     const double* __restrict__ vprev, const double* __restrict__ tprev,
-                                     const double* __restrict__ vors, const double* __restrict__ divs,
-                                     const double* __restrict__ area, double4* __restrict__ src,
-                                     double4* __restrict__ src2, int mixed) {
+// the packed float sources in mixed precision; the blocks past `roots` of the
+// first launch place the non-leaf proxies.
+constexpr int kTreeThreads = 1024;
+
+template <int N1>
+__global__ void __launch_bounds__(kTreeThreads)
+    k_swe_upward_subtree(StepGeom g, SweGeom sw, int roots, int chunk, int r, int D, int stage, double dtd, double dts,
+                         const double* __restrict__ vprev, const double* __restrict__ tprev,
+                         const double* __restrict__ vors, const double* __restrict__ divs,
+                         const double* __restrict__ area, double4* __restrict__ src, double4* __restrict__ src2,
+                         int mixed) {
+  const int n1 = N1 > 0 ? N1 : g.degree + 1, q = N1 > 0 ? N1 * N1 : g.q;
+  if ((int)blockIdx.x >= roots) {
+    const long i = ((long)blockIdx.x - roots) * chunk + threadIdx.x;
+    if ((int)threadIdx.x < chunk && i < (long)g.offset * q) swe_nonleaf_source<N1>(g, sw, i, stage, dtd, vprev, src, src2, mixed);
+    return;
+  }
   extern __shared__ double sh[];  // 2 fields x levels r..r+D, then 2 x 4^D q scratch
-  const int q = g.q, root_rel = blockIdx.x, n1 = g.degree + 1;
+  const int root_rel = blockIdx.x;
   const bool leaves_here = (r + D == g.levels - 1);
-  const long ln = (long)g.leaves * g.q, pn = (long)g.panels * g.q;
+  const long ln = (long)g.leaves * q, pn = (long)g.panels * q;
   const int per_field = q * (((1 << (2 * (D + 1))) - 1) / 3);
   auto lvl = [&](int f, int k) { return sh + f * per_field + q * (((1 << (2 * k)) - 1) / 3); };
   double* scratch = sh + 2 * per_field;
@@ -84,8 +124,9 @@ __global__ void k_swe_upward_subtree(StepGeom g, SweGeom sw, int r, int D, int p
       if (leaves_here) {
         const long i = o - (long)g.offset * q;
         leaf_strengths(i, ln, stage, dts, tprev, vors, divs, area, wv, wd);
-        double px = g.px[o], py = g.px[pn + o], pz = g.px[2 * pn + o];
-        src2[o] = make_double4(px, py, pz, wd);
+        const double x0 = g.px[o], y0 = g.px[pn + o], z0 = g.px[2 * pn + o];
+        double px = x0, py = y0, pz = z0;
+        src2[o] = make_double4(x0, y0, z0, wd);
         if (stage > 0) {
           px += dtd * vprev[i];
           py += dtd * vprev[ln + i];
@@ -93,6 +134,11 @@ __global__ void k_swe_upward_subtree(StepGeom g, SweGeom sw, int r, int D, int p
         }
         project_to_sphere(px, py, pz);
         src[o] = make_double4(px, py, pz, wv);
+        if (mixed) {
+          const double* c = g.pd_centre + 4 * (o / q);
+          g.srcf[o] = pack(c, px, py, pz, wv);
+          sw.srcf2[o] = pack(c, x0, y0, z0, wd);
+        }
       } else {
         wv = src[o].w;
         wd = src2[o].w;
@@ -101,90 +147,42 @@ __global__ void k_swe_upward_subtree(StepGeom g, SweGeom sw, int r, int D, int p
       lvl(1, D)[t] = wd;
     }
   }
-  for (int k = 0; positions && k < D; k++) {  // else k_swe_nonleaf_positions wrote them
-    const int first = subtree_first(r, root_rel, k), npts = (1 << (2 * k)) * q;
-    for (int t = threadIdx.x; t < npts; t += blockDim.x) {
-      const long i = (long)first * q + t;
-      double px, py, pz;
-      nonleaf_position(g, i, stage, dtd, vprev, px, py, pz);
-      src[i] = make_double4(px, py, pz, 0.0);
-      src2[i] = make_double4(g.px[i], g.px[pn + i], g.px[2 * pn + i], 0.0);
-    }
-  }
   __syncthreads();
   for (int k = D - 1; k >= 0; k--) {
     const int np = 1 << (2 * k), first = subtree_first(r, root_rel, k);
     for (int t = threadIdx.x; t < 2 * 4 * np * q; t += blockDim.x) {  // T[f][cc][i][b]
-      const int f = t / (4 * np * q), tt = t % (4 * np * q);
+      const int f = t >= 4 * np * q, tt = t - f * 4 * np * q;
       const int cc = tt / q, rem = tt % q, i = rem / n1, b = rem % n1;
       const double* ly = g.child_1d + ((cc & 3) >= 2 ? n1 * n1 : 0);
       const double* sc = lvl(f, k + 1) + cc * q + i * n1;
       double acc = 0;
-      for (int j = 0; j < n1; j++) acc = fma(__ldg(ly + j * n1 + b), sc[j], acc);
+#pragma unroll
+      for (int j = 0; j < (N1 > 0 ? N1 : n1); j++) acc = fma(__ldg(ly + j * n1 + b), sc[j], acc);
       scratch[f * sstride + tt] = acc;
     }
     __syncthreads();
     for (int t = threadIdx.x; t < 2 * np * q; t += blockDim.x) {  // S[f][p][a][b]
-      const int f = t / (np * q), tt = t % (np * q);
+      const int f = t >= np * q, tt = t - f * np * q;
       const int p = tt / q, rem = tt % q, a = rem / n1, b = rem % n1;
       double acc = 0;
+#pragma unroll
       for (int c = 0; c < 4; c++) {
         const double* lx = g.child_1d + ((c == 1 || c == 2) ? n1 * n1 : 0);
         const double* tc = scratch + f * sstride + (4 * p + c) * q + b;
-        for (int i = 0; i < n1; i++) acc = fma(__ldg(lx + i * n1 + a), tc[i * n1], acc);
+#pragma unroll
+        for (int i = 0; i < (N1 > 0 ? N1 : n1); i++) acc = fma(__ldg(lx + i * n1 + a), tc[i * n1], acc);
       }
       lvl(f, k)[tt] = acc;
-      if (f == 0) src[(long)first * q + tt].w = acc;
-      else src2[(long)first * q + tt].w = acc;
+      const long o = (long)first * q + tt;
+      if (f == 0) src[o].w = acc;
+      else src2[o].w = acc;
+      if (mixed) {
+        if (f == 0) g.srcf[o].w = (float)acc;
+        else sw.srcf2[o].w = (float)acc;
+      }
     }
     __syncthreads();
   }
-  if (mixed) {
-    const int kmax = leaves_here ? D : D - 1;
-    for (int k = 0; k <= kmax; k++) {
-      const int first = subtree_first(r, root_rel, k), npts = (1 << (2 * k)) * q;
-      for (int t = threadIdx.x; t < npts; t += blockDim.x) {
-        const long i = (long)first * q + t;
-        const double* cc = g.pd_centre + 4 * (i / q);
-        const double4 a = src[i], b = src2[i];
-        g.srcf[i] = pack(cc, a.x, a.y, a.z, a.w);
-        sw.srcf2[i] = pack(cc, b.x, b.y, b.z, b.w);
-      }
-    }
-  }
-}
-
-// Positions of every non-leaf proxy of both fields in one flat launch ahead
-// of the subtree passes, a thread per point: the vorticity sources displaced
-// by the interpolated leaf velocity (nonleaf_position's arithmetic, q = 16
-// unrolled), the divergence sources at the fixed proxies.
-template <int Q>
-__global__ void k_swe_nonleaf_positions(StepGeom g, int stage, double dtd, const double* __restrict__ vprev,
-                                        double4* __restrict__ src, double4* __restrict__ src2) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  const int q = Q > 0 ? Q : g.q;
-  if (i >= (long)g.offset * q) return;
-  const long pn = (long)g.panels * q, ln = (long)g.leaves * q;
-  const double x0 = g.px[i], y0 = g.px[pn + i], z0 = g.px[2 * pn + i];
-  double px = x0, py = y0, pz = z0;
-  if (stage > 0) {
-    const long np = (long)g.offset * q;
-    const long row = (long)g.il_row[i] * q;
-    double ax = 0, ay = 0, az = 0;
-#pragma unroll
-    for (int m = 0; m < (Q > 0 ? Q : q); m++) {
-      const double bm = g.il_basis[m * np + i];
-      ax += (dtd * vprev[row + m]) * bm;
-      ay += (dtd * vprev[ln + row + m]) * bm;
-      az += (dtd * vprev[2 * ln + row + m]) * bm;
-    }
-    px += ax;
-    py += ay;
-    pz += az;
-  }
-  project_to_sphere(px, py, pz);
-  src[i] = make_double4(px, py, pz, 0.0);
-  src2[i] = make_double4(x0, y0, z0, 0.0);
 }
 
 // Direct velocity: leaf sources of both fields (no tree).
@@ -670,30 +668,40 @@ size_t swe_subtree_smem(int q, int D) {
   return (size_t)q * 2 * 8 * ((((1L << (2 * (D + 1))) - 1) / 3) + (1L << (2 * D)));
 }
 
+template <int N1>
+void swe_upward(const StepGeom& g, const SweGeom& s, int stage, double dtd, double dts, const double* vprev,
+                const double* tprev, const double* vors, const double* divs, const double* area, double4* src,
+                double4* src2, bool mixed, cudaStream_t st) {
+  static std::atomic<unsigned long long> attr{0};
+  raise_smem_once(attr, 200 * 1024, k_swe_upward_subtree<N1>);
+  const int Dmax = g.q <= 25 ? 3 : 1;
+  int r = g.levels - 1;
+  bool first = true;
+  do {
+    const int D = r < Dmax ? r : Dmax, root = r - D, roots = 6 << (2 * root);
+    const unsigned threads = std::min((unsigned)kTreeThreads, (unsigned)(((g.q << (2 * D)) + 31) / 32 * 32));
+    const long points = first ? (long)g.offset * g.q : 0;
+    const int chunk = nonleaf_chunk(points, threads);
+    const unsigned extra = blocks_for(points, chunk);
+    SB_LAUNCH(k_swe_upward_subtree<N1>, roots + extra, threads, swe_subtree_smem(g.q, D), st, g, s, roots, chunk, root, D,
+              stage, dtd, dts, vprev, tprev, vors, divs, area, src, src2, mixed ? 1 : 0);
+    r = root;
+    first = false;
+  } while (r > 0);
+}
+
 }  // namespace
 
 void launch_swe_upward(const StepGeom& g, const SweGeom& s, int stage, double dtd, double dts, const double* vprev,
                        const double* tprev, const double*, const double*, const double*, const double* vors,
                        const double* divs, const double* area, double4* src, double4* src2, bool mixed,
                        cudaStream_t st) {
-  static std::atomic<unsigned long long> attr{0};
-  raise_smem_once(attr, 200 * 1024, k_swe_upward_subtree);
-  const int Dmax = g.q <= 25 ? 3 : 1;
-  int r = g.levels - 1;
-  const long nl = (long)g.offset * g.q;  // non-leaf proxy points
-  if (nl > 0) {
-    if (g.q == 16)
-      SB_LAUNCH(k_swe_nonleaf_positions<16>, blocks_for(nl, 256), 256, 0, st, g, stage, dtd, vprev, src, src2);
-    else
-      SB_LAUNCH(k_swe_nonleaf_positions<0>, blocks_for(nl, 256), 256, 0, st, g, stage, dtd, vprev, src, src2);
+  switch (g.degree) {
+    case 2: swe_upward<3>(g, s, stage, dtd, dts, vprev, tprev, vors, divs, area, src, src2, mixed, st); break;
+    case 3: swe_upward<4>(g, s, stage, dtd, dts, vprev, tprev, vors, divs, area, src, src2, mixed, st); break;
+    case 4: swe_upward<5>(g, s, stage, dtd, dts, vprev, tprev, vors, divs, area, src, src2, mixed, st); break;
+    default: swe_upward<0>(g, s, stage, dtd, dts, vprev, tprev, vors, divs, area, src, src2, mixed, st); break;
   }
-  do {
-    const int D = r < Dmax ? r : Dmax;
-    const int root = r - D;
-    SB_LAUNCH(k_swe_upward_subtree, (unsigned)(6 << (2 * root)), 256, swe_subtree_smem(g.q, D), st, g, s, root, D,
-              nl > 0 ? 0 : 1, stage, dtd, dts, vprev, tprev, vors, divs, area, src, src2, mixed ? 1 : 0);
-    r = root;
-  } while (r > 0);
 }
 
 void launch_swe_leaf_sources(const StepGeom& g, const SweGeom& s, int stage, double dtd, double dts,
