@@ -19,6 +19,7 @@
 #include "../../include/sbslpm.h"
 #include "bve_kernels.cuh"
 #include "device_common.cuh"
+#include "list32.cuh"
 #include "list64.cuh"
 
 namespace sbslpm {
@@ -32,7 +33,6 @@ namespace {
 
 using namespace dev;
 
-constexpr int kWarpsPerBlock = 4;
 
 // ---------------------------------------------------------------------------
 // Source preparation.
@@ -125,13 +125,6 @@ __global__ void k_copy_strength(StepGeom g, const double4* __restrict__ src, dou
 // Mode 2 (treecode): leaf strengths already anterpolated into src, fixed
 // proxy positions untouched, mixed packing as in mode 0.
 
-__device__ __forceinline__ float4 packed_source(const StepGeom& g, long panel, double x, double y, double z,
-                                                double w) {
-  const double* c = g.pd_centre + 4 * panel;
-  return make_float4((float)((x - c[0]) * kPackScale), (float)((y - c[1]) * kPackScale),
-                     (float)((z - c[2]) * kPackScale), (float)w);
-}
-
 template <int N1>
 __device__ __forceinline__ void nonleaf_source(const StepGeom& g, long i, int stage, double dt_s,
                                                const double* __restrict__ vprev, double4* __restrict__ src,
@@ -143,10 +136,9 @@ __device__ __forceinline__ void nonleaf_source(const StepGeom& g, long i, int st
   src[i].y = py;
   src[i].z = pz;
   if (mixed) {
-    const float4 f = packed_source(g, i / q, px, py, pz, 0.0);
-    g.srcf[i].x = f.x;
-    g.srcf[i].y = f.y;
-    g.srcf[i].z = f.z;
+    const double* c = g.pd_centre + 4 * (i / q);
+    store_packed_xyz(g.srcf, q, i / q, (int)(i % q), (float)((px - c[0]) * kPackScale),
+                     (float)((py - c[1]) * kPackScale), (float)((pz - c[2]) * kPackScale));
   }
 }
 
@@ -193,13 +185,14 @@ __device__ __forceinline__ void upward_subtree_body(const StepGeom& g, int root_
           }
           project_to_sphere(px, py, pz);
           src[o] = make_double4(px, py, pz, w);
-          if (mixed) g.srcf[o] = packed_source(g, o / q, px, py, pz, w);
+          if (mixed) store_packed(g.srcf, q, o / q, t % q, g.pd_centre + 4 * (o / q), px, py, pz, w);
         }
         bot[t] = w;
       } else {
         const double4 v = src[o];
         bot[t] = v.w;
-        if (mixed && leaves_here) g.srcf[o] = packed_source(g, o / q, v.x, v.y, v.z, v.w);
+        if (mixed && leaves_here)
+          store_packed(g.srcf, q, o / q, t % q, g.pd_centre + 4 * (o / q), v.x, v.y, v.z, v.w);
       }
     }
   }
@@ -234,9 +227,9 @@ __device__ __forceinline__ void upward_subtree_body(const StepGeom& g, int root_
       const long o = (long)first * q + t;
       if (mixed && mode == 2) {
         const double4 v = src[o];
-        g.srcf[o] = packed_source(g, o / q, v.x, v.y, v.z, acc);
+        store_packed(g.srcf, q, o / q, rem, g.pd_centre + 4 * (o / q), v.x, v.y, v.z, acc);
       } else if (mixed && mode == 0) {
-        g.srcf[o].w = (float)acc;
+        store_packed_w(g.srcf, q, o / q, rem, (float)acc);
       }
       src[o].w = acc;
     }
@@ -368,13 +361,6 @@ __global__ void k_downward_subtree_batch(const BatchMember* __restrict__ mem, in
 // Direct mode (ALL_LEAVES) splits the source leaves into gridDim.y groups
 // and writes per-group partials that k_reduce_groups sums in order.
 
-template <int Q>
-struct WarpShape {
-  static constexpr int S = Q <= 16 ? 32 / Q : 1;          // source splits per warp
-  static constexpr int Q2 = (Q + 1) / 2;                    // source pairs per panel
-  static constexpr int STAGE2 = (S > 1 ? S : 1) * 2 * Q2;   // float4 slots per warp, paired layout
-};
-
 // Float64, q <= 25 (list64.cuh).
 template <int Q, int WPT, bool ALL_LEAVES, bool GUARD>
 __global__ void __launch_bounds__(32 * ListShape<Q, 1>::NW)
@@ -404,309 +390,27 @@ __global__ void k_pack_mixed(StepGeom g, const double4* __restrict__ src, float4
   long pn = (long)g.panels * g.q;
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= pn) return;
-  const double* c = g.pd_centre + 4 * (i / g.q);
-  double4 s = src[i];
-  srcf[i] = make_float4((float)((s.x - c[0]) * kPackScale), (float)((s.y - c[1]) * kPackScale),
-                        (float)((s.z - c[2]) * kPackScale), (float)s.w);
+  const double4 s = src[i];
+  store_packed(srcf, g.q, i / g.q, (int)(i % g.q), g.pd_centre + 4 * (i / g.q), s.x, s.y, s.z, s.w);
 }
 
-template <int Q, bool ALL_LEAVES, bool GUARD>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock) k_interact32(StepGeom g, const float4* __restrict__ srcf,
-                                                                    double* __restrict__ out, long out_stride) {
-  using W = WarpShape<Q>;
-  __shared__ float4 stage[kWarpsPerBlock][W::STAGE2];
-  __shared__ double red[kWarpsPerBlock][3][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tp_first = ALL_LEAVES ? g.offset : 0;
-  const int tp_count = ALL_LEAVES ? g.leaves : g.panels;
-  const int tix = blockIdx.x * kWarpsPerBlock + warp;
-  if (tix >= tp_count) return;
-  const int t = tp_first + tix;
-  const long pn = (long)g.panels * g.q;
-  int e0, e1;
-  if (ALL_LEAVES) {
-    int per = (g.leaves + gridDim.y - 1) / gridDim.y;
-    e0 = blockIdx.y * per;
-    e1 = min(g.leaves, e0 + per);
-  } else {
-    e0 = g.tgt_start[t];
-    e1 = g.tgt_start[t + 1];
-  }
-  const double* ct = g.pd_centre + 4 * (long)t;
-  const double ctx = ct[0], cty = ct[1], ctz = ct[2];
-  const float eps = (float)g.eps;
-  if constexpr (Q <= 32) {
-    const int h = lane / Q, j = lane % Q;
-    const bool active = h < W::S;
-    double tx = 0, ty = 0, tz = 0;
-    float dtx = 0, dty = 0, dtz = 0;
-    if (active) {
-      long o = (long)t * Q + j;
-      tx = g.px[o];
-      ty = g.px[pn + o];
-      tz = g.px[2 * pn + o];
-      dtx = (float)((tx - ctx) * kPackScale);
-      dty = (float)((ty - cty) * kPackScale);
-      dtz = (float)((tz - ctz) * kPackScale);
-    }
-    double ax = 0, ay = 0, az = 0;
-    const float2 eps2 = make_float2(eps, eps);
-    // each split's panel staged two sources per pair slot, transposed as
-    // (x0,x1,y0,y1),(z0,z1,w0,w1); a missing partner (odd q) has zero strength
-    float* sl = reinterpret_cast<float*>(&stage[warp][0]) + h * 8 * W::Q2;
-    if constexpr (ALL_LEAVES) {
-      for (int e = e0; e < e1; e += W::S) {
-        int sp = 0;
-        if (active && e + h < e1) {
-          sp = g.offset + e + h;
-          const float4 sv = srcf[(long)sp * Q + j];
-          const int k2 = j >> 1, o = j & 1;
-          sl[8 * k2 + o] = sv.x;
-          sl[8 * k2 + 2 + o] = sv.y;
-          sl[8 * k2 + 4 + o] = sv.z;
-          sl[8 * k2 + 6 + o] = sv.w;
-          if ((Q & 1) && j == Q - 1) {
-            sl[8 * k2 + 1] = 0.f;
-            sl[8 * k2 + 3] = 0.f;
-            sl[8 * k2 + 5] = 0.f;
-            sl[8 * k2 + 7] = 0.f;
-          }
-        }
-        __syncwarp();
-        if (active && e + h < e1) {
-          const double* cs = g.pd_centre + 4 * (long)sp;
-          const float b0 = (float)((cs[0] - ctx) * kPackScale) - dtx, b1 = (float)((cs[1] - cty) * kPackScale) - dty,
-                      b2 = (float)((cs[2] - ctz) * kPackScale) - dtz;
-          const float2 bx = make_float2(b0, b0), by = make_float2(b1, b1), bz = make_float2(b2, b2);
-          float2 fx = make_float2(0.f, 0.f), fy = fx, fz = fx;
-          const float4* sb = reinterpret_cast<const float4*>(sl);
-#pragma unroll
-          for (int k2 = 0; k2 < W::Q2; k2++) {
-            const float4 A = sb[2 * k2], B = sb[2 * k2 + 1];
-            pair32x2<GUARD>(bx, by, bz, make_float2(A.x, A.y), make_float2(A.z, A.w), make_float2(B.x, B.y),
-                            make_float2(B.z, B.w), eps2, fx, fy, fz);
-          }
-          ax += (double)(fx.x + fx.y);
-          ay += (double)(fy.x + fy.y);
-          az += (double)(fz.x + fz.y);
-        }
-        __syncwarp();
-      }
-    } else {
-      // The list in batches of 32 entries (g.entry: source panel and its
-      // centre's offset from the target's, one entry per lane), handed to the
-      // splits by shuffles; the next entry's sources are loaded while the
-      // current ones are evaluated.  A source pair is staged by one store per
-      // lane: the even node of a pair writes (x0,x1,y0,y1), the odd one
-      // (z0,z1,w0,w1), each taking its partner's half by a shuffle.
-      const unsigned full = 0xffffffffu;
-      float4* st4 = reinterpret_cast<float4*>(sl);
-      const bool odd = j & 1, last_odd = (Q & 1) && j == Q - 1;
-      const int partner = (odd ? lane - 1 : lane + 1) & 31;
-      for (int eb = e0; eb < e1; eb += 32) {
-        const int nb = min(32, e1 - eb);
-        int4 en = make_int4(0, 0, 0, 0);
-        if (lane < nb) en = __ldg(g.entry + eb + lane);
-        const int iters = (nb + W::S - 1) / W::S;
-        float cbx = __int_as_float(__shfl_sync(full, en.y, h & 31));
-        float cby = __int_as_float(__shfl_sync(full, en.z, h & 31));
-        float cbz = __int_as_float(__shfl_sync(full, en.w, h & 31));
-        float4 sv = make_float4(0.f, 0.f, 0.f, 0.f);
-        {
-          const int sp = __shfl_sync(full, en.x, h & 31);
-          if (active && h < nb) sv = srcf[(long)sp * Q + j];
-        }
-        for (int it = 0; it < iters; it++) {
-          const bool on = active && it * W::S + h < nb;
-          const int ns = (it + 1) * W::S + h;
-          const int sp_n = __shfl_sync(full, en.x, ns & 31);
-          const float nbx = __int_as_float(__shfl_sync(full, en.y, ns & 31));
-          const float nby = __int_as_float(__shfl_sync(full, en.z, ns & 31));
-          const float nbz = __int_as_float(__shfl_sync(full, en.w, ns & 31));
-          float4 sv_n = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (active && ns < nb) sv_n = srcf[(long)sp_n * Q + j];
-          const float r0 = __shfl_sync(full, odd ? sv.x : sv.z, partner);
-          const float r1 = __shfl_sync(full, odd ? sv.y : sv.w, partner);
-          if (on) {
-            const int k2 = j >> 1;
-            if (last_odd) {
-              st4[2 * k2] = make_float4(sv.x, 0.f, sv.y, 0.f);
-              st4[2 * k2 + 1] = make_float4(sv.z, 0.f, sv.w, 0.f);
-            } else if (!odd) {
-              st4[2 * k2] = make_float4(sv.x, r0, sv.y, r1);
-            } else {
-              st4[2 * k2 + 1] = make_float4(r0, sv.z, r1, sv.w);
-            }
-          }
-          __syncwarp();
-          if (on) {
-            const float b0 = cbx - dtx, b1 = cby - dty, b2 = cbz - dtz;
-            const float2 bx = make_float2(b0, b0), by = make_float2(b1, b1), bz = make_float2(b2, b2);
-            float2 fx = make_float2(0.f, 0.f), fy = fx, fz = fx;
-#pragma unroll
-            for (int k2 = 0; k2 < W::Q2; k2++) {
-              const float4 A = st4[2 * k2], B = st4[2 * k2 + 1];
-              pair32x2<GUARD>(bx, by, bz, make_float2(A.x, A.y), make_float2(A.z, A.w), make_float2(B.x, B.y),
-                              make_float2(B.z, B.w), eps2, fx, fy, fz);
-            }
-            ax += (double)(fx.x + fx.y);
-            ay += (double)(fy.x + fy.y);
-            az += (double)(fz.x + fz.y);
-          }
-          __syncwarp();
-          sv = sv_n;
-          cbx = nbx;
-          cby = nby;
-          cbz = nbz;
-        }
-      }
-    }
-    if (W::S > 1) {
-      red[warp][0][lane] = ax;
-      red[warp][1][lane] = ay;
-      red[warp][2][lane] = az;
-      __syncwarp();
-      if (h == 0)
-        for (int hh = 1; hh < W::S; hh++) {
-          ax += red[warp][0][hh * Q + j];
-          ay += red[warp][1][hh * Q + j];
-          az += red[warp][2][hh * Q + j];
-        }
-    }
-    if (h == 0) {
-      long o = ALL_LEAVES ? (long)blockIdx.y * 3 * out_stride + (long)tix * Q + j : (long)t * Q + j;
-      long s = ALL_LEAVES ? out_stride : pn;
-      out[o] = kBiotSavartPacked * (ty * az - tz * ay);
-      out[s + o] = kBiotSavartPacked * (tz * ax - tx * az);
-      out[2 * s + o] = kBiotSavartPacked * (tx * ay - ty * ax);
-    }
-  }
-}
-
-// The list kernel of the reference's default degree 3 (q = 16) in mixed
-// precision, two targets per lane: a warp holds one target panel as 4
-// source splits x 8 lanes, lane jj of a split owns target nodes jj and
-// jj + 8, stages the source pair (2 jj, 2 jj + 1) of its split's panel
-// ((x0,x1,y0,y1),(z0,z1,w0,w1), one pair slot per lane) and evaluates the
-// split's 16 sources against both targets, so every shared-memory read feeds
-// two targets' pairs.  Entries come in batches of 32 (g.entry) handed out by
-// shuffles, the next entry's sources are loaded while the current ones are
-// evaluated, and the four splits' float64 sums are added in split order.
-template <bool GUARD>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock) k_interact32_q16(StepGeom g, const float4* __restrict__ srcf,
-                                                                        double* __restrict__ out) {
-  constexpr int Q = 16, S = 4;
-  __shared__ float4 stage[kWarpsPerBlock][S][Q];
-  __shared__ double red[kWarpsPerBlock][6][32];
-  const unsigned full = 0xffffffffu;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x * kWarpsPerBlock + warp;
-  if (t >= g.panels) return;
+// Mixed precision, q <= 25 (list32.cuh).
+template <int Q, int WPT, bool ALL_LEAVES, bool GUARD>
+__global__ void __launch_bounds__(32 * ListShape32<Q, 1>::NW)
+    k_interact32(StepGeom g, const float4* __restrict__ srcf, double* __restrict__ out, long out_stride) {
+  using W = ListShape32<Q, 1>;
+  __shared__ __align__(16) double shared[W::NW * ((W::WARP + 1) & ~1)];
   const long pn = (long)g.panels * Q;
-  const int e0 = g.tgt_start[t], e1 = g.tgt_start[t + 1];
-  const int h = lane >> 3, jj = lane & 7;
-  const double* ct = g.pd_centre + 4 * (long)t;
-  float dtx[2], dty[2], dtz[2];
-#pragma unroll
-  for (int r = 0; r < 2; r++) {
-    const long o = (long)t * Q + jj + 8 * r;
-    dtx[r] = (float)((g.px[o] - ct[0]) * kPackScale);
-    dty[r] = (float)((g.px[pn + o] - ct[1]) * kPackScale);
-    dtz[r] = (float)((g.px[2 * pn + o] - ct[2]) * kPackScale);
-  }
-  double ax[2] = {0, 0}, ay[2] = {0, 0}, az[2] = {0, 0};
-  const float feps = (float)g.eps;
-  const float2 eps2 = make_float2(feps, feps);
-  float4* tile = stage[warp][h];
-  for (int eb = e0; eb < e1; eb += 32) {
-    const int nb = min(32, e1 - eb);
-    int4 en = make_int4(0, 0, 0, 0);
-    if (lane < nb) en = __ldg(g.entry + eb + lane);
-    const int iters = (nb + S - 1) / S;
-    float cbx = __int_as_float(__shfl_sync(full, en.y, h));
-    float cby = __int_as_float(__shfl_sync(full, en.z, h));
-    float cbz = __int_as_float(__shfl_sync(full, en.w, h));
-    float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
-    {
-      const int sp = __shfl_sync(full, en.x, h);
-      if (h < nb) {
-        s0 = srcf[(long)sp * Q + 2 * jj];
-        s1 = srcf[(long)sp * Q + 2 * jj + 1];
-      }
-    }
-    for (int it = 0; it < iters; it++) {
-      const bool on = it * S + h < nb;
-      const int ns = (it + 1) * S + h;
-      const int sp_n = __shfl_sync(full, en.x, ns & 31);
-      const float nbx = __int_as_float(__shfl_sync(full, en.y, ns & 31));
-      const float nby = __int_as_float(__shfl_sync(full, en.z, ns & 31));
-      const float nbz = __int_as_float(__shfl_sync(full, en.w, ns & 31));
-      float4 n0 = make_float4(0.f, 0.f, 0.f, 0.f), n1 = n0;
-      if (ns < nb) {
-        n0 = srcf[(long)sp_n * Q + 2 * jj];
-        n1 = srcf[(long)sp_n * Q + 2 * jj + 1];
-      }
-      if (on) {
-        tile[2 * jj] = make_float4(s0.x, s1.x, s0.y, s1.y);
-        tile[2 * jj + 1] = make_float4(s0.z, s1.z, s0.w, s1.w);
-      }
-      __syncwarp();
-      if (on) {
-        float2 bx[2], by[2], bz[2], fx[2], fy[2], fz[2];
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-          const float b0 = cbx - dtx[r], b1 = cby - dty[r], b2 = cbz - dtz[r];
-          bx[r] = make_float2(b0, b0);
-          by[r] = make_float2(b1, b1);
-          bz[r] = make_float2(b2, b2);
-          fx[r] = fy[r] = fz[r] = make_float2(0.f, 0.f);
-        }
-#pragma unroll
-        for (int k2 = 0; k2 < Q / 2; k2++) {
-          const float4 A = tile[2 * k2], B = tile[2 * k2 + 1];
-          const float2 sx = make_float2(A.x, A.y), sy = make_float2(A.z, A.w), sz = make_float2(B.x, B.y),
-                       sw = make_float2(B.z, B.w);
-#pragma unroll
-          for (int r = 0; r < 2; r++) pair32x2<GUARD>(bx[r], by[r], bz[r], sx, sy, sz, sw, eps2, fx[r], fy[r], fz[r]);
-        }
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-          ax[r] += (double)(fx[r].x + fx[r].y);
-          ay[r] += (double)(fy[r].x + fy[r].y);
-          az[r] += (double)(fz[r].x + fz[r].y);
-        }
-      }
-      __syncwarp();
-      s0 = n0;
-      s1 = n1;
-      cbx = nbx;
-      cby = nby;
-      cbz = nbz;
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < 2; r++) {
-    red[warp][3 * r][lane] = ax[r];
-    red[warp][3 * r + 1][lane] = ay[r];
-    red[warp][3 * r + 2][lane] = az[r];
-  }
-  __syncwarp();
-  if (h == 0) {
-#pragma unroll
-    for (int r = 0; r < 2; r++) {
-      double sx = ax[r], sy = ay[r], sz = az[r];
-      for (int hh = 1; hh < S; hh++) {
-        sx += red[warp][3 * r][hh * 8 + jj];
-        sy += red[warp][3 * r + 1][hh * 8 + jj];
-        sz += red[warp][3 * r + 2][hh * 8 + jj];
-      }
-      const long o = (long)t * Q + jj + 8 * r;
-      const double tx = g.px[o], ty = g.px[pn + o], tz = g.px[2 * pn + o];
-      out[o] = kBiotSavartPacked * (ty * sz - tz * sy);
-      out[pn + o] = kBiotSavartPacked * (tz * sx - tx * sz);
-      out[2 * pn + o] = kBiotSavartPacked * (tx * sy - ty * sx);
-    }
-  }
+  list32_sweep<Q, 1, WPT, ALL_LEAVES, GUARD>(
+      g, srcf, nullptr, shared, [&](int t, int tix, int j, const double* a) {
+        const long i = (long)t * Q + j;
+        const double x = g.px[i], y = g.px[pn + i], z = g.px[2 * pn + i];
+        const long o = ALL_LEAVES ? (long)blockIdx.y * 3 * out_stride + (long)tix * Q + j : i;
+        const long s = ALL_LEAVES ? out_stride : pn;
+        out[o] = kBiotSavartPacked * (y * a[2] - z * a[1]);
+        out[s + o] = kBiotSavartPacked * (z * a[0] - x * a[2]);
+        out[2 * s + o] = kBiotSavartPacked * (x * a[1] - y * a[0]);
+      });
 }
 
 // Wide panels (q > 32, e.g. 81 treecode proxies): one CTA of four warps per
@@ -1379,16 +1083,19 @@ void interact_qg(const StepGeom& g, int precision, const double4* src, double* o
       else SB_LAUNCH((k_interact_wide<Q, false, GUARD, false>), wgrid, 128, 0, st, g, src, g.srcf, out, out_stride);
     }
   } else {
-    const int threads = 32 * kWarpsPerBlock;
     if (precision == SBSLPM_MIXED) {
-      const dim3 grid(blocks_for(tp, kWarpsPerBlock), all_leaves ? groups : 1);
+      constexpr int NW = dev::ListShape32<Q, 1>::NW, threads = 32 * NW;
+      const int wpt = dev::list_warps<Q, 1>(tp);
       if (pack) SB_LAUNCH(k_pack_mixed, blocks_for((long)g.panels * g.q, 256), 256, 0, st, g, src, g.srcf);
       if (all_leaves)
-        SB_LAUNCH((k_interact32<Q, true, GUARD>), grid, threads, 0, st, g, g.srcf, out, out_stride);
-      else if constexpr (Q == 16)
-        SB_LAUNCH((k_interact32_q16<GUARD>), grid, threads, 0, st, g, g.srcf, out);
+        SB_LAUNCH((k_interact32<Q, 1, true, GUARD>), dim3(blocks_for(tp, NW), groups), threads, 0, st, g, g.srcf, out,
+                  out_stride);
+      else if (wpt == NW)
+        SB_LAUNCH((k_interact32<Q, NW, false, GUARD>), tp, threads, 0, st, g, g.srcf, out, out_stride);
+      else if (wpt == 2)
+        SB_LAUNCH((k_interact32<Q, 2, false, GUARD>), blocks_for(tp, NW / 2), threads, 0, st, g, g.srcf, out, out_stride);
       else
-        SB_LAUNCH((k_interact32<Q, false, GUARD>), grid, threads, 0, st, g, g.srcf, out, out_stride);
+        SB_LAUNCH((k_interact32<Q, 1, false, GUARD>), blocks_for(tp, NW), threads, 0, st, g, g.srcf, out, out_stride);
     } else {
       constexpr int NW = dev::ListShape<Q, 1>::NW, threads64 = 32 * NW;
       const int wpt = dev::list_warps<Q, 1>(tp);

@@ -18,6 +18,11 @@ namespace sbslpm {
 constexpr double kPackScale = 0.70710678118654752440;
 constexpr double kBiotSavartPacked = kBiotSavart * 1.41421356237309504880;
 
+// Packed float32 sources: panels of at most kPairedQ sources hold them in
+// pairs (store_packed_xyz), so an odd count takes one more; float4 per panel.
+constexpr int kPairedQ = 25;
+SB_HD constexpr int packed_stride(int q) { return q <= kPairedQ ? (q + 1) / 2 * 2 : q; }
+
 // Static per-problem constants used by the BLI code on the device.
 struct BliTable {
   double cosv[kMaxDegree + 1];  // cos(pi*i/d), computed on the host with libm
@@ -35,7 +40,7 @@ struct StepGeom {
   const double* il_basis;     // [q][(panels-leaves)*q] BLI basis at that leaf, term-major (coalesced per point)
   const double* child_1d;     // [2][d+1][d+1]: 1-D basis of parent node a at the node i of a child in the upper (0) / lower (1) half
   const double* pd_centre;    // mixed: panel centres [panels][4] (double)
-  float4* srcf;               // mixed: packed sources [panels*q] (workspace)
+  float4* srcf;               // mixed: packed sources [panels][packed_stride(q)] (workspace)
   // mixed, q <= 32: per list entry (CSR order) the source panel and the offset
   // of its centre from the target panel's, (float)((c_S - c_T) kPackScale) as
   // float bits

@@ -229,7 +229,7 @@ sbslpm_status precompute_tree(sbslpm_ctx* c) {
   c->near_max_splits = std::min(16, std::max(4, 148 * 16 / t.Af));
   SB_TRY(dalloc(&c->near, (size_t)c->near_max_splits * 3 * N));
   if (c->cfg.precision == SBSLPM_MIXED) {
-    SB_TRY(dalloc(&c->fsrcf, pn));
+    SB_TRY(alloc_packed(&c->fsrcf, t.Pf, t.qx));
     SB_TRY(dalloc(&c->psrcf, N));
     if (c->cc_partial) SB_TRY(dalloc(&c->fsrcp, (size_t)t.Pf * 2 * ((t.qx + 1) / 2)));
   }
@@ -240,7 +240,7 @@ sbslpm_status allocate_workspace(sbslpm_ctx* c) {
   const size_t pn = (size_t)c->P * c->q, ln = (size_t)c->A * c->q;
   if (!c->tree) {
     SB_TRY(dalloc(&c->src, pn));
-    if (c->cfg.precision == SBSLPM_MIXED) SB_TRY(dalloc(&c->srcf, pn));
+    if (c->cfg.precision == SBSLPM_MIXED) SB_TRY(alloc_packed(&c->srcf, c->P, c->q));
     SB_TRY(dalloc(&c->tgt, 3 * pn));
   }
   SB_TRY(dalloc(&c->vbuf, 4 * 3 * ln));

@@ -170,6 +170,17 @@ sbslpm_status dalloc(T** p, size_t count) {
   return SBSLPM_OK;
 }
 
+// Packed float32 sources of a tree (StepGeom::srcf), zeroed: the places that
+// close odd counts stay zero.
+inline sbslpm_status alloc_packed(float4** p, int panels, int q) {
+  const size_t n = (size_t)panels * packed_stride(q);
+  const sbslpm_status s = dalloc(p, n);
+  if (s != SBSLPM_OK) return s;
+  SB_CUDA(cudaMemset(*p, 0, sizeof(float4) * n));
+  SB_CUDA(cudaStreamSynchronize(nullptr));  // the context's streams do not wait for the legacy one
+  return SBSLPM_OK;
+}
+
 template <class T>
 sbslpm_status upload(T** p, const std::vector<T>& h) {
   sbslpm_status s = dalloc(p, h.size());

@@ -163,6 +163,37 @@ __device__ __forceinline__ void stage_expanded(const float4* __restrict__ src, i
   out[3] = make_float4(s0.w * s0.z, s1.w * s1.z, s0.w, s1.w);
 }
 
+// Where the packed float32 source j (of q) of a panel lies.  Panels of up to
+// kPairedQ sources (list32.cuh) hold them two by two, transposed, as the
+// paired FP32 instructions take them: (x0,x1,y0,y1) (z0,z1,w0,w1), an odd
+// count closing on a source that stays zero; larger panels hold one float4
+// per source.
+__device__ __forceinline__ void store_packed_xyz(float4* srcf, int q, long panel, int j, float x, float y, float z) {
+  if (q <= kPairedQ) {
+    float* p = reinterpret_cast<float*>(srcf + panel * packed_stride(q)) + 8 * (j >> 1) + (j & 1);
+    p[0] = x;
+    p[2] = y;
+    p[4] = z;
+  } else {
+    float4& f = srcf[panel * q + j];
+    f.x = x;
+    f.y = y;
+    f.z = z;
+  }
+}
+
+__device__ __forceinline__ void store_packed_w(float4* srcf, int q, long panel, int j, float w) {
+  if (q <= kPairedQ) (reinterpret_cast<float*>(srcf + panel * packed_stride(q)) + 8 * (j >> 1) + (j & 1))[6] = w;
+  else srcf[panel * q + j].w = w;
+}
+
+__device__ __forceinline__ void store_packed(float4* srcf, int q, long panel, int j, const double* c, double x,
+                                             double y, double z, double w) {
+  store_packed_xyz(srcf, q, panel, j, (float)((x - c[0]) * kPackScale), (float)((y - c[1]) * kPackScale),
+                   (float)((z - c[2]) * kPackScale));
+  store_packed_w(srcf, q, panel, j, (float)w);
+}
+
 // First panel id of the k-th level below the subtree root (level, root_rel).
 __device__ __forceinline__ int subtree_first(int level, int root_rel, int k) {
   return level_start(level + k) + (root_rel << (2 * k));

@@ -64,7 +64,7 @@ sbslpm_status swe_setup(sbslpm_ctx* c) {
     SB_CUDA(cudaMemcpy(c->fsrc2, init.data(), sizeof(double4) * fpn, cudaMemcpyHostToDevice));
     if (c->cfg.precision == SBSLPM_MIXED) {
       SB_TRY(dalloc(&c->psrcf2, (size_t)ln));
-      SB_TRY(dalloc(&c->fsrcf2, fpn));
+      SB_TRY(alloc_packed(&c->fsrcf2, c->Pf, c->qx));
       if (c->n_cc > 0 && c->cc_chunks[kSweCcLen - 1] && swe_tree_cc_supported(c->qx))
         SB_TRY(dalloc(&c->swe_cc_partial, (size_t)c->n_cc * 6 * c->qx));
     }
@@ -73,8 +73,8 @@ sbslpm_status swe_setup(sbslpm_ctx* c) {
     if (!c->src) SB_TRY(dalloc(&c->src, pn));
     SB_TRY(dalloc(&c->src2, pn));
     if (c->cfg.precision == SBSLPM_MIXED) {
-      if (!c->srcf) SB_TRY(dalloc(&c->srcf, pn));
-      SB_TRY(dalloc(&c->srcf2, pn));
+      if (!c->srcf) SB_TRY(alloc_packed(&c->srcf, c->P, c->q));
+      SB_TRY(alloc_packed(&c->srcf2, c->P, c->q));
     }
     if (!c->tgt) SB_TRY(dalloc(&c->tgt, 3 * pn));
   }

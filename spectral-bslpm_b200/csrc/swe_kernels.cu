@@ -19,6 +19,7 @@
 
 #include "../../include/sbslpm.h"
 #include "device_common.cuh"
+#include "list32.cuh"
 #include "list64.cuh"
 #include "swe_kernels.cuh"
 
@@ -51,11 +52,6 @@ __device__ __forceinline__ void leaf_strengths(long i, long ln, int stage, doubl
   }
 }
 
-__device__ __forceinline__ float4 pack(const double* c, double x, double y, double z, double w) {
-  return make_float4((float)((x - c[0]) * kPackScale), (float)((y - c[1]) * kPackScale),
-                     (float)((z - c[2]) * kPackScale), (float)w);
-}
-
 // Positions of the non-leaf proxies of both fields (swe_disp_interp_2,
 // src/swe_time_step_2.cpp:436-476, identical to the BVE form): the vorticity
 // sources displaced by the interpolated leaf velocity, the divergence sources
@@ -77,13 +73,10 @@ __device__ __forceinline__ void swe_nonleaf_source(const StepGeom& g, const SweG
   src2[i].z = z0;
   if (mixed) {
     const double* c = g.pd_centre + 4 * (i / q);
-    const float4 a = pack(c, px, py, pz, 0.0), b = pack(c, x0, y0, z0, 0.0);
-    g.srcf[i].x = a.x;
-    g.srcf[i].y = a.y;
-    g.srcf[i].z = a.z;
-    sw.srcf2[i].x = b.x;
-    sw.srcf2[i].y = b.y;
-    sw.srcf2[i].z = b.z;
+    store_packed_xyz(g.srcf, q, i / q, (int)(i % q), (float)((px - c[0]) * kPackScale),
+                     (float)((py - c[1]) * kPackScale), (float)((pz - c[2]) * kPackScale));
+    store_packed_xyz(sw.srcf2, q, i / q, (int)(i % q), (float)((x0 - c[0]) * kPackScale),
+                     (float)((y0 - c[1]) * kPackScale), (float)((z0 - c[2]) * kPackScale));
   }
 }
 
@@ -136,8 +129,8 @@ __global__ void __launch_bounds__(kTreeThreads)
         src[o] = make_double4(px, py, pz, wv);
         if (mixed) {
           const double* c = g.pd_centre + 4 * (o / q);
-          g.srcf[o] = pack(c, px, py, pz, wv);
-          sw.srcf2[o] = pack(c, x0, y0, z0, wd);
+          store_packed(g.srcf, q, o / q, t % q, c, px, py, pz, wv);
+          store_packed(sw.srcf2, q, o / q, t % q, c, x0, y0, z0, wd);
         }
       } else {
         wv = src[o].w;
@@ -177,8 +170,7 @@ __global__ void __launch_bounds__(kTreeThreads)
       if (f == 0) src[o].w = acc;
       else src2[o].w = acc;
       if (mixed) {
-        if (f == 0) g.srcf[o].w = (float)acc;
-        else sw.srcf2[o].w = (float)acc;
+        store_packed_w(f == 0 ? g.srcf : sw.srcf2, q, o / q, rem, (float)acc);
       }
     }
     __syncthreads();
@@ -199,7 +191,9 @@ __global__ void k_swe_leaf_sources(StepGeom g, SweGeom sw, int stage, double dtd
   leaf_strengths(i, ln, stage, dts, tprev, vors, divs, area, wv, wd);
   double px = g.px[o], py = g.px[pn + o], pz = g.px[2 * pn + o];
   src2[o] = make_double4(px, py, pz, wd);
-  if (mixed) sw.srcf2[o] = pack(g.pd_centre + 4 * (o / g.q), px, py, pz, wd);
+  const double* c = g.pd_centre + 4 * (o / g.q);
+  const int j = (int)(o % g.q);
+  if (mixed) store_packed(sw.srcf2, g.q, o / g.q, j, c, px, py, pz, wd);
   if (stage > 0) {
     px += dtd * vprev[i];
     py += dtd * vprev[ln + i];
@@ -207,7 +201,7 @@ __global__ void k_swe_leaf_sources(StepGeom g, SweGeom sw, int stage, double dtd
   }
   project_to_sphere(px, py, pz);
   src[o] = make_double4(px, py, pz, wv);
-  if (mixed) g.srcf[o] = pack(g.pd_centre + 4 * (o / g.q), px, py, pz, wv);
+  if (mixed) store_packed(g.srcf, g.q, o / g.q, j, c, px, py, pz, wv);
 }
 
 // Piecewise API: sources from explicit displacements (swe_vel_panel_interaction_2
@@ -226,27 +220,20 @@ __global__ void k_swe_sources_from_disp(StepGeom g, SweGeom sw, const double* __
   src2[i] = make_double4(x0, y0, z0, sd[i]);
   if (mixed) {
     const double* c = g.pd_centre + 4 * (i / g.q);
-    g.srcf[i] = pack(c, px, py, pz, sv[i]);
-    sw.srcf2[i] = pack(c, x0, y0, z0, sd[i]);
+    const int j = (int)(i % g.q);
+    store_packed(g.srcf, g.q, i / g.q, j, c, px, py, pz, sv[i]);
+    store_packed(sw.srcf2, g.q, i / g.q, j, c, x0, y0, z0, sd[i]);
   }
 }
 
 // ---------------------------------------------------------------------------
-// Interactions.  One warp per target panel; for q <= 16 the warp's lanes are
-// (32/q source splits) x (q target nodes), for larger q each lane owns
-// ceil(q/32) target nodes.  A source panel's q proxies of both fields are
-// staged in shared memory and every lane sweeps them (mixed: two proxies per
-// paired float32 instruction, each panel's two interleaved float32 halves
-// added before the float64 conversion).  ALL_LEAVES: every
-// leaf against every leaf, source leaves split into gridDim.y groups whose
-// partials are reduced in order afterwards.
-
-template <int Q>
-struct Shape {
-  static constexpr int S = Q <= 16 ? 32 / Q : 1;
-  static constexpr int TPL = Q <= 32 ? 1 : (Q + 31) / 32;
-  static constexpr int STAGE = S * Q > Q ? S * Q : Q;
-};
+// Interactions: q <= 25 by list64.cuh and list32.cuh below; larger q by one
+// warp per target panel, each lane owning ceil(q/32) target nodes.  A source
+// panel's q proxies of both fields are staged in shared memory and every lane
+// sweeps them (mixed: two proxies per paired float32 instruction, each panel's
+// two interleaved float32 halves added before the float64 conversion).
+// ALL_LEAVES: every leaf against every leaf, source leaves split into
+// gridDim.y groups whose partials are reduced in order afterwards.
 
 // u = K x cross A - K (B - x (x.B)); K = -1/(4 pi), or scaled by sqrt(2)
 // for the packed float sums.
@@ -263,14 +250,13 @@ template <int Q, bool ALL_LEAVES, bool GUARD, bool MIXED>
 __global__ void __launch_bounds__(32 * kWarps)
     k_swe_interact(StepGeom g, SweGeom sw, const double4* __restrict__ src, const double4* __restrict__ src2,
                    double* __restrict__ out, long out_stride) {
-  using W = Shape<Q>;
+  constexpr int TPL = (Q + 31) / 32;
   using Src = typename std::conditional<MIXED, float4, double4>::type;
-  // mixed: a split's Q proxies as ceil(Q/2) source pairs of two float4
+  // mixed: the Q proxies as ceil(Q/2) source pairs of two float4
   // (x0,x1,y0,y1),(z0,z1,w0,w1), an odd Q closing on a zero-strength source
   // at the panel's centre (which adds exactly zero)
-  constexpr int HQ = (Q + 1) / 2, SPLIT = MIXED ? 2 * HQ : Q, STG = MIXED ? W::S * 2 * HQ : W::STAGE;
-  __shared__ Src stage[kWarps][2][STG];
-  __shared__ double red[kWarps][6][32];
+  constexpr int HQ = (Q + 1) / 2;
+  __shared__ Src stage[kWarps][2][MIXED ? 2 * HQ : Q];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tp_first = ALL_LEAVES ? g.offset : 0;
   const int tp_count = ALL_LEAVES ? g.leaves : g.panels;
@@ -301,15 +287,12 @@ __global__ void __launch_bounds__(32 * kWarps)
   const float eps32 = (float)g.eps;
   const double deps2 = twice_eps(g.eps);
   constexpr double K = MIXED ? kBiotSavartPacked : kBiotSavartTwice;
-  constexpr int TPL = W::TPL;
-  const int h = Q <= 32 ? lane / Q : 0;
-  const bool active = Q <= 32 ? h < W::S : true;
 
   double tx[TPL], ty[TPL], tz[TPL], ax[TPL], ay[TPL], az[TPL], bx[TPL], by[TPL], bz[TPL];
   float dtx[TPL], dty[TPL], dtz[TPL];
 #pragma unroll
   for (int r = 0; r < TPL; r++) {
-    const int j = Q <= 32 ? lane % Q : lane + 32 * r;
+    const int j = lane + 32 * r;
     const long o = (long)t * Q + (j < Q ? j : 0);
     tx[r] = g.px[o];
     ty[r] = g.px[pn + o];
@@ -321,40 +304,28 @@ __global__ void __launch_bounds__(32 * kWarps)
     }
     ax[r] = ay[r] = az[r] = bx[r] = by[r] = bz[r] = 0;
   }
-  constexpr int STEP = Q <= 32 ? W::S : 1;
-  // a lane's share of the staging: a proxy (float64) or a source pair (mixed)
-  auto stage_one = [&](int sp, int k, int slot) {
-    if constexpr (MIXED) {
-      const long b = (long)sp * Q + 2 * k;
-      const bool two = 2 * k + 1 < Q;
-      const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
-      const float4 a0 = s1[b], a1 = two ? s1[b + 1] : none, c0 = s2[b], c1 = two ? s2[b + 1] : none;
-      stage[warp][0][slot + 2 * k] = make_float4(a0.x, a1.x, a0.y, a1.y);
-      stage[warp][0][slot + 2 * k + 1] = make_float4(a0.z, a1.z, a0.w, a1.w);
-      stage[warp][1][slot + 2 * k] = make_float4(c0.x, c1.x, c0.y, c1.y);
-      stage[warp][1][slot + 2 * k + 1] = make_float4(c0.z, c1.z, c0.w, c1.w);
-    } else {
-      stage[warp][0][slot + k] = s1[(long)sp * Q + k];
-      stage[warp][1][slot + k] = s2[(long)sp * Q + k];
-    }
-  };
-  constexpr int PER = MIXED ? HQ : Q;  // staging items per source panel
-  for (int e = e0; e < e1; e += STEP) {
-    int sp = 0;
-    if (Q <= 32) {
-      if (active && e + h < e1) {
-        sp = source_of(e + h);
-        const int j = lane % Q;
-        if (j < PER) stage_one(sp, j, h * SPLIT);
+  constexpr int PER = MIXED ? HQ : Q;  // staging items per source panel: proxies (float64) or source pairs (mixed)
+  for (int e = e0; e < e1; e++) {
+    const int sp = source_of(e);
+    for (int k = lane; k < PER; k += 32) {
+      if constexpr (MIXED) {
+        const long b = (long)sp * Q + 2 * k;
+        const bool two = 2 * k + 1 < Q;
+        const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 a0 = s1[b], a1 = two ? s1[b + 1] : none, c0 = s2[b], c1 = two ? s2[b + 1] : none;
+        stage[warp][0][2 * k] = make_float4(a0.x, a1.x, a0.y, a1.y);
+        stage[warp][0][2 * k + 1] = make_float4(a0.z, a1.z, a0.w, a1.w);
+        stage[warp][1][2 * k] = make_float4(c0.x, c1.x, c0.y, c1.y);
+        stage[warp][1][2 * k + 1] = make_float4(c0.z, c1.z, c0.w, c1.w);
+      } else {
+        stage[warp][0][k] = s1[(long)sp * Q + k];
+        stage[warp][1][k] = s2[(long)sp * Q + k];
       }
-    } else {
-      sp = source_of(e);
-      for (int k = lane; k < PER; k += 32) stage_one(sp, k, 0);
     }
     __syncwarp();
-    if (active && e + h < e1) {
-      const Src* st1 = &stage[warp][0][h * SPLIT];
-      const Src* st2 = &stage[warp][1][h * SPLIT];
+    {
+      const Src* st1 = stage[warp][0];
+      const Src* st2 = stage[warp][1];
       if constexpr (MIXED) {
         const double* cs = g.pd_centre + 4 * (long)sp;
         const float c0 = (float)((cs[0] - ct[0]) * kPackScale), c1 = (float)((cs[1] - ct[1]) * kPackScale),
@@ -399,29 +370,9 @@ __global__ void __launch_bounds__(32 * kWarps)
     }
     __syncwarp();
   }
-  if (Q <= 32 && W::S > 1) {
-    red[warp][0][lane] = ax[0];
-    red[warp][1][lane] = ay[0];
-    red[warp][2][lane] = az[0];
-    red[warp][3][lane] = bx[0];
-    red[warp][4][lane] = by[0];
-    red[warp][5][lane] = bz[0];
-    __syncwarp();
-    if (h == 0)
-      for (int hh = 1; hh < W::S; hh++) {
-        const int l = hh * Q + lane % Q;
-        ax[0] += red[warp][0][l];
-        ay[0] += red[warp][1][l];
-        az[0] += red[warp][2][l];
-        bx[0] += red[warp][3][l];
-        by[0] += red[warp][4][l];
-        bz[0] += red[warp][5][l];
-      }
-  }
-  if (h != 0) return;
 #pragma unroll
   for (int r = 0; r < TPL; r++) {
-    const int j = Q <= 32 ? lane % Q : lane + 32 * r;
+    const int j = lane + 32 * r;
     if (j >= Q) continue;
     double ux, uy, uz;
     const long ot = (long)t * Q + j;  // the target's position again: not held in registers across the sweep
@@ -457,150 +408,25 @@ __global__ void __launch_bounds__(32 * ListShape<Q, 2>::NW)
       });
 }
 
-// Mixed precision, q <= 32, list mode: the BVE list kernel's organisation
-// (k_interact32) with both source fields.  List entries come 32 at a time
-// from the static entry table (source panel, centre offset as float) and are
-// handed to the splits by shuffles; the next entry's sources of both fields
-// are loaded while the current ones are evaluated; each field's source pair
-// is staged (x0,x1,y0,y1),(z0,z1,w0,w1) by one store per lane, and both
-// fields' pairs run on the paired float32 instructions (pair32x2), two
-// sources per instruction.  A panel's float32 halves are added before the
-// float64 conversion.
-template <int Q, bool GUARD>
-__global__ void __launch_bounds__(32 * kWarps) k_swe_interact32_list(StepGeom g, SweGeom sw,
-                                                                     double* __restrict__ out) {
-  using W = Shape<Q>;
-  constexpr int Q2 = (Q + 1) / 2;
-  __shared__ float4 stage[kWarps][2][W::S * 2 * Q2];
-  __shared__ double red[kWarps][6][32];
-  const unsigned full = 0xffffffffu;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x * kWarps + warp;
-  if (t >= g.panels) return;
+// Mixed precision, q <= 25: both fields by list32.cuh.
+template <int Q, int WPT, bool ALL_LEAVES, bool GUARD>
+__global__ void __launch_bounds__(32 * ListShape32<Q, 2>::NW)
+    k_swe_interact32(StepGeom g, SweGeom sw, double* __restrict__ out, long out_stride) {
+  using W = ListShape32<Q, 2>;
+  __shared__ __align__(16) double shared[W::NW * ((W::WARP + 1) & ~1)];
   const long pn = (long)g.panels * Q;
-  const int e0 = g.tgt_start[t], e1 = g.tgt_start[t + 1];
-  const int h = lane / Q, j = lane % Q;
-  const bool active = h < W::S;
-  const double* ct = g.pd_centre + 4 * (long)t;
-  double tx = 0, ty = 0, tz = 0;
-  float dtx = 0, dty = 0, dtz = 0;
-  if (active) {
-    const long o = (long)t * Q + j;
-    tx = g.px[o];
-    ty = g.px[pn + o];
-    tz = g.px[2 * pn + o];
-    dtx = (float)((tx - ct[0]) * kPackScale);
-    dty = (float)((ty - ct[1]) * kPackScale);
-    dtz = (float)((tz - ct[2]) * kPackScale);
-  }
-  double ax = 0, ay = 0, az = 0, bx = 0, by = 0, bz = 0;
-  const float feps = (float)g.eps;
-  const float2 eps2 = make_float2(feps, feps);
-  float4* t1 = &stage[warp][0][(active ? h : 0) * 2 * Q2];
-  float4* t2 = &stage[warp][1][(active ? h : 0) * 2 * Q2];
-  const bool odd = j & 1, last_odd = (Q & 1) && j == Q - 1;
-  const int partner = (odd ? lane - 1 : lane + 1) & 31;
-  auto put = [&](float4* tl, const float4& v, float r0, float r1) {
-    const int k2 = j >> 1;
-    if (last_odd) {
-      tl[2 * k2] = make_float4(v.x, 0.f, v.y, 0.f);
-      tl[2 * k2 + 1] = make_float4(v.z, 0.f, v.w, 0.f);
-    } else if (!odd) {
-      tl[2 * k2] = make_float4(v.x, r0, v.y, r1);
-    } else {
-      tl[2 * k2 + 1] = make_float4(r0, v.z, r1, v.w);
-    }
-  };
-  for (int eb = e0; eb < e1; eb += 32) {
-    const int nb = min(32, e1 - eb);
-    int4 en = make_int4(0, 0, 0, 0);
-    if (lane < nb) en = __ldg(g.entry + eb + lane);
-    const int iters = (nb + W::S - 1) / W::S;
-    float cbx = __int_as_float(__shfl_sync(full, en.y, h & 31));
-    float cby = __int_as_float(__shfl_sync(full, en.z, h & 31));
-    float cbz = __int_as_float(__shfl_sync(full, en.w, h & 31));
-    float4 v1 = make_float4(0.f, 0.f, 0.f, 0.f), v2 = v1;
-    {
-      const int sp = __shfl_sync(full, en.x, h & 31);
-      if (active && h < nb) {
-        v1 = g.srcf[(long)sp * Q + j];
-        v2 = sw.srcf2[(long)sp * Q + j];
-      }
-    }
-    for (int it = 0; it < iters; it++) {
-      const bool on = active && it * W::S + h < nb;
-      const int ns = (it + 1) * W::S + h;
-      const int sp_n = __shfl_sync(full, en.x, ns & 31);
-      const float nbx = __int_as_float(__shfl_sync(full, en.y, ns & 31));
-      const float nby = __int_as_float(__shfl_sync(full, en.z, ns & 31));
-      const float nbz = __int_as_float(__shfl_sync(full, en.w, ns & 31));
-      float4 n1 = make_float4(0.f, 0.f, 0.f, 0.f), n2 = n1;
-      if (active && ns < nb) {
-        n1 = g.srcf[(long)sp_n * Q + j];
-        n2 = sw.srcf2[(long)sp_n * Q + j];
-      }
-      const float p0 = __shfl_sync(full, odd ? v1.x : v1.z, partner);
-      const float p1 = __shfl_sync(full, odd ? v1.y : v1.w, partner);
-      const float q0 = __shfl_sync(full, odd ? v2.x : v2.z, partner);
-      const float q1 = __shfl_sync(full, odd ? v2.y : v2.w, partner);
-      if (on) {
-        put(t1, v1, p0, p1);
-        put(t2, v2, q0, q1);
-      }
-      __syncwarp();
-      if (on) {
-        const float b0 = cbx - dtx, b1 = cby - dty, b2 = cbz - dtz;
-        const float2 px2 = make_float2(b0, b0), py2 = make_float2(b1, b1), pz2 = make_float2(b2, b2);
-        float2 fax = make_float2(0.f, 0.f), fay = fax, faz = fax, fbx = fax, fby = fax, fbz = fax;
-#pragma unroll
-        for (int k2 = 0; k2 < Q2; k2++) {
-          const float4 A = t1[2 * k2], B = t1[2 * k2 + 1], C = t2[2 * k2], D = t2[2 * k2 + 1];
-          pair32x2<GUARD>(px2, py2, pz2, make_float2(A.x, A.y), make_float2(A.z, A.w), make_float2(B.x, B.y),
-                          make_float2(B.z, B.w), eps2, fax, fay, faz);
-          pair32x2<GUARD>(px2, py2, pz2, make_float2(C.x, C.y), make_float2(C.z, C.w), make_float2(D.x, D.y),
-                          make_float2(D.z, D.w), eps2, fbx, fby, fbz);
-        }
-        ax += (double)(fax.x + fax.y);
-        ay += (double)(fay.x + fay.y);
-        az += (double)(faz.x + faz.y);
-        bx += (double)(fbx.x + fbx.y);
-        by += (double)(fby.x + fby.y);
-        bz += (double)(fbz.x + fbz.y);
-      }
-      __syncwarp();
-      v1 = n1;
-      v2 = n2;
-      cbx = nbx;
-      cby = nby;
-      cbz = nbz;
-    }
-  }
-  if (W::S > 1) {
-    red[warp][0][lane] = ax;
-    red[warp][1][lane] = ay;
-    red[warp][2][lane] = az;
-    red[warp][3][lane] = bx;
-    red[warp][4][lane] = by;
-    red[warp][5][lane] = bz;
-    __syncwarp();
-    if (h == 0)
-      for (int hh = 1; hh < W::S; hh++) {
-        const int l = hh * Q + j;
-        ax += red[warp][0][l];
-        ay += red[warp][1][l];
-        az += red[warp][2][l];
-        bx += red[warp][3][l];
-        by += red[warp][4][l];
-        bz += red[warp][5][l];
-      }
-  }
-  if (h != 0) return;
-  double ux, uy, uz;
-  swe_epilogue(kBiotSavartPacked, tx, ty, tz, ax, ay, az, bx, by, bz, ux, uy, uz);
-  const long o = (long)t * Q + j;
-  out[o] = ux;
-  out[pn + o] = uy;
-  out[2 * pn + o] = uz;
+  list32_sweep<Q, 2, WPT, ALL_LEAVES, GUARD>(
+      g, g.srcf, sw.srcf2, shared, [&](int t, int tix, int j, const double* a) {
+        const long i = (long)t * Q + j;
+        double ux, uy, uz;
+        swe_epilogue(kBiotSavartPacked, g.px[i], g.px[pn + i], g.px[2 * pn + i], a[0], a[1], a[2], a[3], a[4], a[5],
+                     ux, uy, uz);
+        const long o = ALL_LEAVES ? (long)blockIdx.y * 3 * out_stride + (long)tix * Q + j : i;
+        const long s = ALL_LEAVES ? out_stride : pn;
+        out[o] = ux;
+        out[s + o] = uy;
+        out[2 * s + o] = uz;
+      });
 }
 
 __global__ void k_swe_reduce(const double* __restrict__ partial, int groups, long n, long gstride,
@@ -620,16 +446,21 @@ void swe_interact_qg(const StepGeom& g, const SweGeom& s, int precision, const d
   const bool mixed = precision == SBSLPM_MIXED;
 #define SB_SWE_K(AL, MX) \
   SB_LAUNCH((k_swe_interact<Q, AL, GUARD, MX>), grid, 32 * kWarps, 0, st, g, s, src, src2, out, out_stride)
-  if (mixed) {
-    if constexpr (Q <= 32) {
-      if (!all_leaves && g.entry) {
-        SB_LAUNCH((k_swe_interact32_list<Q, GUARD>), grid, 32 * kWarps, 0, st, g, s, out);
-        return;
-      }
+  if constexpr (Q <= 32) {
+    if (mixed) {
+      constexpr int NW = ListShape32<Q, 2>::NW, threads = 32 * NW;
+      const int wpt = dev::list_warps<Q, 2>(tp);
+      if (all_leaves)
+        SB_LAUNCH((k_swe_interact32<Q, 1, true, GUARD>), dim3(blocks_for(tp, NW), groups), threads, 0, st, g, s, out,
+                  out_stride);
+      else if (tp <= 148 * 16)
+        SB_LAUNCH((k_swe_interact32<Q, NW, false, GUARD>), tp, threads, 0, st, g, s, out, out_stride);
+      else if (wpt == 2)
+        SB_LAUNCH((k_swe_interact32<Q, 2, false, GUARD>), blocks_for(tp, NW / 2), threads, 0, st, g, s, out, out_stride);
+      else
+        SB_LAUNCH((k_swe_interact32<Q, 1, false, GUARD>), blocks_for(tp, NW), threads, 0, st, g, s, out, out_stride);
+      return;
     }
-    if (all_leaves) SB_SWE_K(true, true);
-    else SB_SWE_K(false, true);
-  } else if constexpr (Q <= 32) {
     constexpr int NW = ListShape<Q, 2>::NW, threads = 32 * NW;
     const int wpt = dev::list_warps<Q, 2>(tp);
     if (all_leaves)
@@ -644,7 +475,9 @@ void swe_interact_qg(const StepGeom& g, const SweGeom& s, int precision, const d
       SB_LAUNCH((k_swe_interact64<Q, 1, false, GUARD>), blocks_for(tp, NW), threads, 0, st, g, src, src2, out,
                 out_stride);
   } else {
-    if (all_leaves) SB_SWE_K(true, false);
+    if (all_leaves && mixed) SB_SWE_K(true, true);
+    else if (all_leaves) SB_SWE_K(true, false);
+    else if (mixed) SB_SWE_K(false, true);
     else SB_SWE_K(false, false);
   }
 #undef SB_SWE_K

@@ -23,7 +23,7 @@ struct SweGeom {
   const int* pface;       // [leaves*q]: cube face of each grid point
   const int* ustart;      // [unique+1]: CSR of the grid points sharing one position, in [leaf][q] order
   const int* umem;        // [leaves*q]
-  float4* srcf2;          // mixed: packed divergence sources [panels*q] (workspace)
+  float4* srcf2;          // mixed: packed divergence sources, as StepGeom::srcf (workspace)
 };
 
 // Sources of one velocity evaluation and the upward pass, both source fields
