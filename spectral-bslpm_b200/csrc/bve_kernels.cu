@@ -13,7 +13,9 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdint>
 #include <cstdio>
+#include <initializer_list>
 #include <type_traits>
 
 #include "../../include/sbslpm.h"
@@ -577,7 +579,21 @@ __global__ void k_reduce_groups(const double* __restrict__ partial, int groups, 
 // kernel is bound by float64 division and atan latency, not by its 136 bytes
 // of traffic per particle.
 
-template <int D>
+// VEC: the gathered fields are read two values at a time (q even, rows on
+// 16-byte boundaries).
+template <int D, bool VEC>
+__device__ __forceinline__ void gather_velocity(const Basis<D>& b, const double* __restrict__ v, long n, double& x,
+                                                double& y, double& z) {
+  if constexpr (VEC) {
+    x = gather_vec<D>(b, v);
+    y = gather_vec<D>(b, v + n);
+    z = gather_vec<D>(b, v + 2 * n);
+  } else {
+    gather3<D>(b, v, n, x, y, z);
+  }
+}
+
+template <int D, bool VEC>
 __device__ __forceinline__ void depart_remap_body(const StepGeom& g, const BliTable& tab, long o,
                                                   const double* __restrict__ x, const double* __restrict__ y,
                                                   const double* __restrict__ z, const double* __restrict__ v0,
@@ -597,17 +613,17 @@ __device__ __forceinline__ void depart_remap_body(const StepGeom& g, const BliTa
     project_to_sphere_rcp(xx, yy, zz);
     locate_basis_rcp<D>(g, tab, xx, yy, zz, b, err);
     double k2x, k2y, k2z;
-    gather3<D>(b, v2, n, k2x, k2y, k2z);
+    gather_velocity<D, VEC>(b, v2, n, k2x, k2y, k2z);
     xx = x0 - 0.5 * dt * k2x, yy = y0 - 0.5 * dt * k2y, zz = z0 - 0.5 * dt * k2z;
     project_to_sphere_rcp(xx, yy, zz);
     locate_basis_rcp<D>(g, tab, xx, yy, zz, b, err);
     double k3x, k3y, k3z;
-    gather3<D>(b, v1, n, k3x, k3y, k3z);
+    gather_velocity<D, VEC>(b, v1, n, k3x, k3y, k3z);
     xx = x0 - dt * k3x, yy = y0 - dt * k3y, zz = z0 - dt * k3z;
     project_to_sphere_rcp(xx, yy, zz);
     locate_basis_rcp<D>(g, tab, xx, yy, zz, b, err);
     double k4x, k4y, k4z;
-    gather3<D>(b, v0, n, k4x, k4y, k4z);
+    gather_velocity<D, VEC>(b, v0, n, k4x, k4y, k4z);
     xx = x0 - 1.0 / 6.0 * dt * k1x, yy = y0 - 1.0 / 6.0 * dt * k1y, zz = z0 - 1.0 / 6.0 * dt * k1z;
     project_to_sphere_rcp(xx, yy, zz);
     xx -= -1.0 / 3.0 * dt * k2x, yy -= -1.0 / 3.0 * dt * k2y, zz -= -1.0 / 3.0 * dt * k2z;
@@ -631,7 +647,9 @@ __device__ __forceinline__ void depart_remap_body(const StepGeom& g, const BliTa
   }
   if (mode & 2) {
     locate_basis_rcp<D>(g, tab, dx, dy, dz, b, err);
-    double vor = gather<D>(b, vors);
+    double vor;
+    if constexpr (VEC) vor = gather_vec<D>(b, vors);
+    else vor = gather<D>(b, vors);
     for (int k = 0; k < T; k++) new_tracers[o * T + k] = gather<D>(b, tracers, T, k);
     vor += 2 * g.omega * dz;
     new_vors[o] = vor - 2 * g.omega * z[o];
@@ -639,12 +657,15 @@ __device__ __forceinline__ void depart_remap_body(const StepGeom& g, const BliTa
   flag(g.err, err);
 }
 
-// 128 threads held to 64 registers (eight blocks per SM; a few bytes spill):
-// the chain of four locate -> gather rounds per particle is latency-bound,
-// and the extra resident warps measured 9 us per launch faster at 393,216
-// particles (78 vs 87 us) than the 76-register build.
-template <int D, int MODE>
-__global__ void __launch_bounds__(128, 8) k_depart_remap(StepGeom g, BliTable tab, const double* __restrict__ x, const double* __restrict__ y,
+// 128 threads; held to 64 registers (BLOCKS = 8 per SM) where the grid fills
+// the SMs that often: the chain of four locate -> gather rounds per particle
+// is latency-bound, and the extra resident warps measured 9 us per launch
+// faster at 393,216 particles than a 76-register build.  A grid of at most
+// four blocks per SM has the registers to keep a round's loads in flight.
+// 393,216 particles: 74 us with a descent per location and one value per
+// load, 65 us now.
+template <int D, int MODE, bool VEC, int BLOCKS>
+__global__ void __launch_bounds__(128, BLOCKS) k_depart_remap(StepGeom g, BliTable tab, const double* __restrict__ x, const double* __restrict__ y,
                                const double* __restrict__ z, const double* __restrict__ v0,
                                const double* __restrict__ v1, const double* __restrict__ v2,
                                const double* __restrict__ v3, double dt, double* __restrict__ dep,
@@ -659,13 +680,13 @@ __global__ void __launch_bounds__(128, 8) k_depart_remap(StepGeom g, BliTable ta
     out.y[o] = v0[n + o];
     out.z[o] = v0[2 * n + o];
   }
-  depart_remap_body<D>(g, tab, o, x, y, z, v0, v1, v2, v3, dt, dep, vors, tracers, T, new_vors, new_tracers, MODE);
+  depart_remap_body<D, VEC>(g, tab, o, x, y, z, v0, v1, v2, v3, dt, dep, vors, tracers, T, new_vors, new_tracers, MODE);
 }
 
 // Batched members on one particle grid (member blockIdx.y): departure and
 // remap in one pass (mode 3), stage velocities v_k + m * 3n, vorticity + m * n.
-template <int D>
-__global__ void k_depart_remap_batch(StepGeom g, BliTable tab, const double* __restrict__ x,
+template <int D, bool VEC>
+__global__ void __launch_bounds__(128, 8) k_depart_remap_batch(StepGeom g, BliTable tab, const double* __restrict__ x,
                                      const double* __restrict__ y, const double* __restrict__ z,
                                      const double* __restrict__ v0, const double* __restrict__ v1,
                                      const double* __restrict__ v2, const double* __restrict__ v3, double dt,
@@ -674,7 +695,7 @@ __global__ void k_depart_remap_batch(StepGeom g, BliTable tab, const double* __r
   const long o = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (o >= n) return;
   const long m = blockIdx.y, vo = m * 3 * n, so = m * n;
-  depart_remap_body<D>(g, tab, o, x, y, z, v0 + vo, v1 + vo, v2 + vo, v3 + vo, dt, nullptr, vors + so, nullptr, 0,
+  depart_remap_body<D, VEC>(g, tab, o, x, y, z, v0 + vo, v1 + vo, v2 + vo, v3 + vo, dt, nullptr, vors + so, nullptr, 0,
                        new_vors + so, nullptr, 3);
 }
 
@@ -1186,26 +1207,47 @@ void launch_direct_leaves(const StepGeom& g, int precision, const double4* src, 
   SB_LAUNCH(k_reduce_groups, blocks_for(3 * n, 256), 256, 0, st, partial, groups, 3 * n, 3 * n, vout);
 }
 
+static bool aligned16(std::initializer_list<const double*> ps) {
+  for (const double* p : ps)
+    if (reinterpret_cast<uintptr_t>(p) % 16 != 0) return false;
+  return true;
+}
+
 void launch_depart_remap(const StepGeom& g, const BliTable* tab, const double* x, const double* y, const double* z,
                          const double* v0, const double* v1, const double* v2, const double* v3, double dt,
                          double* dep, const double* vors, const double* tracers, int T, double* new_vors,
                          double* new_tracers, int mode, cudaStream_t st, VelocityOut vel) {
   long n = (long)g.leaves * g.q;
   unsigned grid = blocks_for(n, 128);
-#define SB_DRM(D, MODE)                                                                                            \
-  SB_LAUNCH((k_depart_remap<D, MODE>), grid, 128, 0, st, g, *tab, x, y, z, v0, v1, v2, v3, dt, dep, vors, tracers, \
-            T, new_vors, new_tracers, vel)
-#define SB_DR(D)                     \
-  case D:                            \
-    if (mode == 1) SB_DRM(D, 1);     \
-    else if (mode == 2) SB_DRM(D, 2); \
-    else SB_DRM(D, 3);               \
+  // rows of an even q on 16-byte boundaries where every gathered field is
+  const bool vec = aligned16({v0, v1, v2, vors}) && n % 2 == 0;
+  const bool few = grid <= 4 * 148;
+#define SB_DRL(D, MODE, VEC, BLOCKS)                                                                                \
+  SB_LAUNCH((k_depart_remap<D, MODE, VEC, BLOCKS>), grid, 128, 0, st, g, *tab, x, y, z, v0, v1, v2, v3, dt, dep, \
+            vors, tracers, T, new_vors, new_tracers, vel)
+#define SB_DRM(D, MODE, BLOCKS)                                   \
+  if (((D + 1) * (D + 1)) % 2 == 0 && vec)                        \
+    SB_DRL(D, MODE, (((D + 1) * (D + 1)) % 2 == 0), BLOCKS);      \
+  else                                                            \
+    SB_DRL(D, MODE, false, BLOCKS)
+#define SB_DR(D)             \
+  case D:                    \
+    if (mode == 1) {         \
+      SB_DRM(D, 1, 8);       \
+    } else if (mode == 2) {  \
+      SB_DRM(D, 2, 8);       \
+    } else if (few) {        \
+      SB_DRM(D, 3, 4);       \
+    } else {                 \
+      SB_DRM(D, 3, 8);       \
+    }                        \
     break;
   switch (g.degree) {
     SB_DR(0) SB_DR(1) SB_DR(2) SB_DR(3) SB_DR(4) SB_DR(5) SB_DR(6) SB_DR(7) SB_DR(8) SB_DR(9) SB_DR(10)
   }
 #undef SB_DR
 #undef SB_DRM
+#undef SB_DRL
 }
 
 void launch_depart_remap_batch(const StepGeom& g, const BliTable* tab, int members, const double* x,
@@ -1214,9 +1256,15 @@ void launch_depart_remap_batch(const StepGeom& g, const BliTable* tab, int membe
                                cudaStream_t st) {
   const long n = (long)g.leaves * g.q;
   const dim3 grid(blocks_for(n, 128), (unsigned)members);
-#define SB_DRB(D)                                                                                               \
-  case D:                                                                                                       \
-    SB_LAUNCH(k_depart_remap_batch<D>, grid, 128, 0, st, g, *tab, x, y, z, v0, v1, v2, v3, dt, vors, new_vors); \
+  const bool vec = aligned16({v0, v1, v2, vors}) && n % 2 == 0;
+#define SB_DRB(D)                                                                                                  \
+  case D:                                                                                                          \
+    if (((D + 1) * (D + 1)) % 2 == 0 && vec)                                                                       \
+      SB_LAUNCH((k_depart_remap_batch<D, (((D + 1) * (D + 1)) % 2 == 0)>), grid, 128, 0, st, g, *tab, x, y, z, v0, \
+                v1, v2, v3, dt, vors, new_vors);                                                                   \
+    else                                                                                                           \
+      SB_LAUNCH((k_depart_remap_batch<D, false>), grid, 128, 0, st, g, *tab, x, y, z, v0, v1, v2, v3, dt, vors,    \
+                new_vors);                                                                                         \
     break;
   switch (g.degree) {
     SB_DRB(0) SB_DRB(1) SB_DRB(2) SB_DRB(3) SB_DRB(4) SB_DRB(5) SB_DRB(6) SB_DRB(7) SB_DRB(8) SB_DRB(9) SB_DRB(10)

@@ -27,6 +27,13 @@ __device__ __forceinline__ double recip_nr(double d) {
   return fma(r, fma(e, e, e), r);
 }
 
+// 1/d to within half a unit in the last place: recip_nr and one residual
+// step.  d of either sign, normal.
+__device__ __forceinline__ double recip_full(double d) {
+  const double r = recip_nr(d);
+  return fma(r, fma(-d, r, 1.0), r);
+}
+
 __device__ __forceinline__ float recip_f32(float d) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
@@ -287,67 +294,68 @@ __device__ __forceinline__ void bli_1d_common(double t, double lo, double hi, co
     den += f[i];
     suf *= dl[i];
   }
-  const double inv = 1.0 / den;
+  const double inv = recip_full(den);
 #pragma unroll
   for (int i = 0; i <= D; i++) f[i] *= inv;
 }
 
 __device__ __forceinline__ void project_to_sphere_rcp(double& x, double& y, double& z) {
   // written out: the single and the batched step's kernels must contract alike
-  const double inv = 1.0 / sqrt(fma(z, z, fma(y, y, x * x)));
+  const double inv = rsqrt(fma(z, z, fma(y, y, x * x)));
   x *= inv;
   y *= inv;
   z *= inv;
 }
 
+// The cell [b, b + 1] 2/n - 1 (times pi/4) of t along one direction of the
+// face's n = 2^(levels-1) leaves, t on a boundary belonging to the upper one.
+// The boundaries are those the tree descent compares with: fl(pi/4 * dyadic),
+// its 0.5 pi/4 (max + min) being the same number.  The guess is off by one at
+// most and corrected against them.
+__device__ __forceinline__ double leaf_edge(int b, int n) { return b * (2.0 / n) - 1.0; }
+
+__device__ __forceinline__ int leaf_cell(double t, int n) {
+  int b = (int)floor(fma(t, 4.0 / kPi, 1.0) * (0.5 * n));
+  b = max(0, min(n - 1, b));
+  if (b > 0 && t < kPi / 4.0 * leaf_edge(b, n)) b--;
+  else if (b < n - 1 && t >= kPi / 4.0 * leaf_edge(b + 1, n)) b++;
+  return b;
+}
+
+// Bits of b spread to the even positions.
+__device__ __forceinline__ unsigned spread_bits(unsigned b) {
+  b = (b | (b << 8)) & 0x00ff00ffu;
+  b = (b | (b << 4)) & 0x0f0f0f0fu;
+  b = (b | (b << 2)) & 0x33333333u;
+  return (b | (b << 1)) & 0x55555555u;
+}
+
+// locate_basis for the departure / remap kernel: one reciprocal for the face's
+// axis, the leaf from the cells of xi and eta instead of a descent through the
+// levels (child c of a level has xi bit bx, eta bit be: c = 2 (1 - be) + (bx
+// xor be)), the barycentric basis with one reciprocal per direction.
 template <int D>
 __device__ __forceinline__ void locate_basis_rcp(const StepGeom& g, const BliTable& tab, double x, double y, double z,
                                                  Basis<D>& b, unsigned& err) {
   const int face = face_from_xyz(x, y, z);
-  double xi, eta;
-  switch (face) {  // xieta_from_xyz_face with one reciprocal of the face's axis coordinate
-    case 0: { const double r = 1.0 / x; xi = atan(y * r); eta = atan(z * r); break; }
-    case 1: { const double r = 1.0 / y; xi = atan(-x * r); eta = atan(z * r); break; }
-    case 2: { const double r = 1.0 / x; xi = atan(y * r); eta = atan(-z * r); break; }
-    case 3: { const double r = 1.0 / y; xi = atan(-x * r); eta = atan(-z * r); break; }
-    case 4: { const double r = 1.0 / z; xi = atan(y * r); eta = atan(-x * r); break; }
-    default: { const double r = 1.0 / z; xi = atan(-y * r); eta = atan(-x * r); break; }
-  }
-  // tree descent of locate_leaf from the face's coordinates
-  Bounds bd{-1, 1, -1, 1};
-  int id = face;
-  for (int lev = 0; lev < g.levels - 1; lev++) {
-    const double mid_xi = 0.5 * kPi / 4.0 * (bd.max_xi + bd.min_xi);
-    const double mid_eta = 0.5 * kPi / 4.0 * (bd.max_eta + bd.min_eta);
-    const double ux = 0.5 * (bd.max_xi + bd.min_xi), ue = 0.5 * (bd.max_eta + bd.min_eta);
-    int c;
-    if ((xi >= mid_xi) && (eta >= mid_eta)) {
-      c = 0;
-      bd.min_xi = ux;
-      bd.min_eta = ue;
-    } else if ((xi <= mid_xi) && (eta >= mid_eta)) {
-      c = 1;
-      bd.max_xi = ux;
-      bd.min_eta = ue;
-    } else if ((xi <= mid_xi) && (eta <= mid_eta)) {
-      c = 2;
-      bd.max_xi = ux;
-      bd.max_eta = ue;
-    } else if ((xi >= mid_xi) && (eta <= mid_eta)) {
-      c = 3;
-      bd.min_xi = ux;
-      bd.max_eta = ue;
-    } else {
-      err |= kErrNonFinite;  // NaN coordinates
-      c = 0;
-      bd.min_xi = ux;
-      bd.min_eta = ue;
-    }
-    id = level_start(lev + 1) + 4 * (id - level_start(lev)) + c;
-  }
+  // xieta_from_xyz_face: face 0 (y, z)/x, 1 (-x, z)/y, 2 (y, -z)/x, 3 (-x, -z)/y, 4 (y, -x)/z, 5 (-y, -x)/z
+  const double den = face == 0 || face == 2 ? x : face == 1 || face == 3 ? y : z;
+  const double num_xi = face == 1 || face == 3 ? -x : face == 5 ? -y : y;
+  const double num_eta = face >= 4 ? -x : face >= 2 ? -z : z;
+  const double r = recip_full(den);
+  const double xi = atan(num_xi * r), eta = atan(num_eta * r);
+  if (!(xi == xi) || !(eta == eta)) err |= kErrNonFinite;  // NaN coordinates
+  const int n = 1 << (g.levels - 1);
+  int bx = leaf_cell(xi, n);
+  const int be = leaf_cell(eta, n);
+  // xi on a boundary: at the level that cuts there (bit ffs - 1 of the cells)
+  // the descent takes the upper half with the upper half of eta only
+  if (bx > 0 && xi == kPi / 4.0 * leaf_edge(bx, n) && !((be >> (__ffs(bx) - 1)) & 1)) bx--;
+  const Bounds bd{leaf_edge(bx, n), leaf_edge(bx + 1, n), leaf_edge(be, n), leaf_edge(be + 1, n)};
+  const unsigned leaf = (spread_bits(~be & (n - 1)) << 1) | spread_bits(bx ^ be);
   bli_1d_common<D>(xi, kPi / 4.0 * bd.min_xi, kPi / 4.0 * bd.max_xi, tab, b.fx, err);
   bli_1d_common<D>(eta, kPi / 4.0 * bd.min_eta, kPi / 4.0 * bd.max_eta, tab, b.fe, err);
-  b.row = (long)(id - g.offset) * g.q;
+  b.row = ((long)face * n * n + leaf) * g.q;
 }
 
 // sum_m field[row + m] * fx[i] fe[j] with m = i (D+1) + j, in m order.
@@ -360,6 +368,22 @@ __device__ __forceinline__ double gather(const Basis<D>& b, const double* __rest
   for (int i = 0; i <= D; i++)
 #pragma unroll
     for (int j = 0; j <= D; j++, m++) acc += f[(b.row + m) * stride + base] * (b.fx[i] * b.fe[j]);
+  return acc;
+}
+
+// The same for q even and rows on 16-byte boundaries, two values per load: a
+// particle's 160 loads (degree 3) otherwise fill the load/store unit.
+template <int D>
+__device__ __forceinline__ double gather_vec(const Basis<D>& b, const double* __restrict__ f) {
+  constexpr int n1 = D + 1, q = n1 * n1;
+  const double2* p = reinterpret_cast<const double2*>(f + b.row);
+  double acc = 0;
+#pragma unroll
+  for (int m = 0; m < q; m += 2) {
+    const double2 v = p[m / 2];
+    acc += v.x * (b.fx[m / n1] * b.fe[m % n1]);
+    acc += v.y * (b.fx[(m + 1) / n1] * b.fe[(m + 1) % n1]);
+  }
   return acc;
 }
 
