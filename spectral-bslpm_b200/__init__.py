@@ -13,6 +13,7 @@ There is no CPU fallback: without the library or a GPU the calls raise.
 from __future__ import annotations
 
 import ctypes
+import math
 import os
 from dataclasses import dataclass
 
@@ -391,7 +392,7 @@ def _dev(t, name, shape=None):
 
     if not isinstance(t, torch.Tensor) or not t.is_cuda or t.dtype != torch.float64 or not t.is_contiguous():
         raise TypeError(f"{name} must be a contiguous float64 CUDA tensor")
-    if shape is not None and t.numel() != int(np.prod(shape)):
+    if shape is not None and t.numel() != math.prod(shape):
         raise ValueError(f"{name} has {t.numel()} elements, expected {shape}")
     return t.data_ptr()
 
@@ -413,7 +414,7 @@ def _host(a, name, shape=None, write=False):
         if write and not a.flags["WRITEABLE"]:
             raise ValueError(f"{name} is read-only")
         n, ptr = a.size, a.ctypes.data
-    if shape is not None and n != int(np.prod(shape)):
+    if shape is not None and n != math.prod(shape):
         raise ValueError(f"{name} has {n} elements, expected {shape}")
     return ptr
 

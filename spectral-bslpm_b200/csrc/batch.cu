@@ -110,12 +110,10 @@ sbslpm_status bupload(sbslpm_batch* b, T** p, const std::vector<T>& h) {
 sbslpm_status batch_finish(sbslpm_batch* b) {
   cudaStream_t st = b->stream();
   SB_CUDA(cudaGetLastError());
-  SB_CUDA(cudaMemcpyAsync(b->h_err, b->err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
   SB_CUDA(cudaStreamSynchronize(st));
-  const unsigned e = *b->h_err;
+  unsigned e = 0;
+  SB_TRY(error_word(b->err, b->h_err, st, &e));
   if (e) {
-    SB_CUDA(cudaMemsetAsync(b->err, 0, sizeof(unsigned), st));
-    SB_CUDA(cudaStreamSynchronize(st));
     if (e & kErrTimeout)
       return set_last_error("a tensor-core interaction kernel's bounded wait ran out"), SBSLPM_ERR_TIMEOUT;
     if (e & kErrNonFinite) return set_last_error("non-finite point in a location step"), SBSLPM_ERR_NONFINITE;
@@ -135,9 +133,8 @@ sbslpm_status batch_setup(sbslpm_batch* b) {
   b->N = (long)b->A * b->q;
   build_panels(b->L, b->panels);
   bli_table(b->d, b->tab);
-  SB_TRY(balloc(b, &b->err, 1));
-  SB_CUDA(cudaMemset(b->err, 0, sizeof(unsigned)));
-  SB_CUDA(cudaMallocHost(reinterpret_cast<void**>(&b->h_err), sizeof(unsigned)));
+  SB_TRY(alloc_error_word(&b->err, &b->h_err));
+  b->bufs.push_back(b->err);
 
   StepGeom& g = b->g;
   g.levels = b->L;

@@ -252,9 +252,7 @@ sbslpm_status allocate_workspace(sbslpm_ctx* c) {
     c->groups = (int)(g < 1 ? 1 : (g > 64 ? 64 : g));
     SB_TRY(dalloc(&c->partial, (size_t)c->groups * 3 * ln));
   }
-  SB_TRY(dalloc(&c->err, 1));
-  SB_CUDA(cudaMemset(c->err, 0, sizeof(unsigned)));
-  SB_CUDA(cudaMallocHost(reinterpret_cast<void**>(&c->h_err), sizeof(unsigned)));
+  SB_TRY(alloc_error_word(&c->err, &c->h_err));
   return SBSLPM_OK;
 }
 
@@ -449,22 +447,44 @@ void enqueue_step(sbslpm_ctx* c, const double* x, const double* y, const double*
   if (T > 0) cudaMemcpyAsync(tracers, c->newtr, sizeof(double) * ln * T, cudaMemcpyDeviceToDevice, st);
 }
 
+sbslpm_status alloc_error_word(unsigned** err, unsigned** h_err) {
+  SB_CUDA(cudaMalloc(reinterpret_cast<void**>(err), 4 * sizeof(unsigned)));
+  SB_CUDA(cudaMallocHost(reinterpret_cast<void**>(h_err), 2 * sizeof(unsigned)));
+  (*h_err)[0] = (*h_err)[1] = 0;
+  void* flag = nullptr;
+  SB_CUDA(cudaHostGetDevicePointer(&flag, *h_err, 0));
+  unsigned words[4] = {0, 0, 0, 0};
+  std::memcpy(words + 2, &flag, sizeof flag);
+  SB_CUDA(cudaMemcpy(*err, words, sizeof words, cudaMemcpyHostToDevice));
+  return SBSLPM_OK;
+}
+
+sbslpm_status error_word(unsigned* err, unsigned* h_err, cudaStream_t st, unsigned* bits) {
+  volatile unsigned* h = h_err;
+  *bits = 0;
+  if (h[0] == 0) return SBSLPM_OK;
+  SB_CUDA(cudaMemcpyAsync(h_err + 1, err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+  SB_CUDA(cudaMemsetAsync(err, 0, sizeof(unsigned), st));
+  SB_CUDA(cudaStreamSynchronize(st));
+  *bits = h[1];
+  h[0] = 0;
+  return SBSLPM_OK;
+}
+
 // Waits for the stream, then turns launch errors and the device error word
 // into a status.
 sbslpm_status finish(sbslpm_ctx* c) {
   cudaStream_t st = c->stream();
   SB_CUDA(cudaGetLastError());
-  SB_CUDA(cudaMemcpyAsync(c->h_err, c->err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
   SB_CUDA(cudaStreamSynchronize(st));
-  unsigned e = *c->h_err;
   if (c->shard_status != SBSLPM_OK) {
     const sbslpm_status s = c->shard_status;
     c->shard_status = SBSLPM_OK;
     return set_last_error(c->shard_error), s;
   }
+  unsigned e = 0;
+  SB_TRY(error_word(c->err, c->h_err, st, &e));
   if (e) {
-    SB_CUDA(cudaMemsetAsync(c->err, 0, sizeof(unsigned), st));
-    SB_CUDA(cudaStreamSynchronize(st));
     if (e & kErrTimeout)
       return set_last_error("a well-separated kernel's bounded copy wait ran out"), SBSLPM_ERR_TIMEOUT;
     if (e & kErrNonFinite) return set_last_error("non-finite point in a location step"), SBSLPM_ERR_NONFINITE;

@@ -12,8 +12,14 @@
 namespace sbslpm {
 namespace dev {
 
+// The device error word (alloc_error_word): the bits, and at err + 2 the
+// address of a page-locked host word that any error sets, so that the host
+// reads the bits back only after one.
 __device__ __forceinline__ void flag(unsigned* err, unsigned bits) {
-  if (bits) atomicOr(err, bits);
+  if (bits) {
+    atomicOr(err, bits);
+    *static_cast<volatile unsigned*>(*reinterpret_cast<unsigned**>(err + 2)) = 1u;
+  }
 }
 
 // 1/d from the hardware approximation r and one third-order step

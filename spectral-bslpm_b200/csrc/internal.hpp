@@ -32,6 +32,14 @@ inline bool any_on_host(std::initializer_list<const void*> ps) {
   return false;
 }
 
+// Device error word of a context or batch: four words at *err (the bits, a
+// spare, and the address of h_err[0], which device code sets with any bit) and
+// two page-locked words at *h_err (that flag, and where the bits are copied).
+// error_word is called once the stream is idle: the bits of the errors since
+// the last call, cleared, without touching the device when there were none.
+sbslpm_status alloc_error_word(unsigned** err, unsigned** h_err);
+sbslpm_status error_word(unsigned* err, unsigned* h_err, cudaStream_t st, unsigned* bits);
+
 // setup_host.cpp
 int child_of(const sbslpm_panel& p, int c);
 void build_panels(int levels, std::vector<sbslpm_panel>& panels);
