@@ -121,7 +121,8 @@ sbslpm_status sbslpm_bve_adjoint_step(sbslpm_ctx* c, const double* x, const doub
       launch_bltc_sources(c->tgeom, c->fgeom, c->ftab, s, h[s], s ? v[s - 1] : nullptr, x, y, z, vors, area, c->psrc,
                           nullptr, c->fsrc, false, st);
       launch_tree_velocity_adjoint(c->tgeom, c->fgeom, c->ftab, tl, x, y, z, vb[s], c->psrc, c->adj_tbar, c->adj_qbl,
-                                   c->adj_q, c->adj_y, c->cfg.precision == SBSLPM_MIXED, st);
+                                   c->adj_q, c->adj_y, c->cfg.precision == SBSLPM_MIXED, st, c->aux_stream ? c->aux_stream : st,
+                                   c->ev_fork, c->ev_join);
     } else if (spectral) {
       launch_spectral_velocity_adjoint(c->geom, c->adj_cc_ts, c->adj_cc_tt, vb[s], c->adj_src + s * pn,
                                        c->adj_tbar, c->adj_qbl, c->adj_y, c->adj_ynl,

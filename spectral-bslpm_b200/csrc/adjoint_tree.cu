@@ -261,7 +261,8 @@ __global__ void __launch_bounds__(NT) k_tree_near_T(TreeGeom tg, const int* __re
       tile[i][2] = make_double2(c * px - a * pz, a * py - b * px);
     }
     __syncthreads();
-#pragma unroll 4
+    // not unrolled: 64 registers either way, and 195 us against 216 us with four
+#pragma unroll 1
     for (int i = 0; i < cnt; i++) {
       const double2 A = tile[i][0], B = tile[i][1], C = tile[i][2];
       // step by step for both sources: an operand held over from the
@@ -742,28 +743,36 @@ void launch_nonleaf_positions_adjoint(const StepGeom& g, double h, const double*
 void launch_tree_velocity_adjoint(const TreeGeom& tg, const StepGeom& fg, const BliTable& ftab,
                                   const TreeAdjointLists& tl, const double* x, const double* y, const double* z,
                                   const double* vbar, const double4* psrc, double* tbar, double* qbl, double* qbar,
-                                  double* ybar, bool mixed, cudaStream_t st) {
+                                  double* ybar, bool mixed, cudaStream_t st, cudaStream_t tree_st, cudaEvent_t fork,
+                                  cudaEvent_t join) {
   const int qx = fg.q, Pf = fg.panels;
   const long pn = (long)Pf * qx;
+  // the tree's passes need only vbar, the near field only vbar and the
+  // particle sources: the tree runs beside it
+  if (tree_st != st) {
+    cudaEventRecord(fork, st);
+    cudaStreamWaitEvent(tree_st, fork, 0);
+  }
   // leaf interpolation, transposed; non-leaf rows start at zero
-  cudaMemsetAsync(tbar, 0, sizeof(double) * 3 * pn, st);
+  cudaMemsetAsync(tbar, 0, sizeof(double) * 3 * pn, tree_st);
   const int n1 = tg.n + 1, groups = kLeafThreads / qx > 0 ? kLeafThreads / qx : 1;
   static std::atomic<unsigned long long> attr_t{0};
   raise_smem_once(attr_t, 128 * 1024, k_tree_to_particles_T);
   SB_LAUNCH(k_tree_to_particles_T, dim3((unsigned)fg.leaves, 3), kLeafThreads,
-            sizeof(double) * (tg.npl + 2 * tg.npl * n1 + groups * qx), st, tg, fg, vbar, tbar);
-  launch_up3(fg, tbar, st);
+            sizeof(double) * (tg.npl + 2 * tg.npl * n1 + groups * qx), tree_st, tg, fg, vbar, tbar);
+  launch_up3(fg, tbar, tree_st);
   // well-separated interactions, transposed
   if (mixed) {
-    if (fg.eps > 0) SB_LAUNCH(k_tree_cc_T32<false>, (unsigned)Pf, kT, 0, st, fg, tl.cc_tstart, tl.cc_ttgt, tbar, qbl);
-    else SB_LAUNCH(k_tree_cc_T32<true>, (unsigned)Pf, kT, 0, st, fg, tl.cc_tstart, tl.cc_ttgt, tbar, qbl);
+    if (fg.eps > 0) SB_LAUNCH(k_tree_cc_T32<false>, (unsigned)Pf, kT, 0, tree_st, fg, tl.cc_tstart, tl.cc_ttgt, tbar, qbl);
+    else SB_LAUNCH(k_tree_cc_T32<true>, (unsigned)Pf, kT, 0, tree_st, fg, tl.cc_tstart, tl.cc_ttgt, tbar, qbl);
   } else if (fg.eps > 0) {
-    launch_cluster(k_tree_cc_T<false>, Pf, split_ranks(Pf), kT, 0, st, fg, tl.cc_tstart, tl.cc_ttgt, tbar, qbl);
+    launch_cluster(k_tree_cc_T<false>, Pf, split_ranks(Pf), kT, 0, tree_st, fg, tl.cc_tstart, tl.cc_ttgt, tbar, qbl);
   } else {
-    launch_cluster(k_tree_cc_T<true>, Pf, split_ranks(Pf), kT, 0, st, fg, tl.cc_tstart, tl.cc_ttgt, tbar, qbl);
+    launch_cluster(k_tree_cc_T<true>, Pf, split_ranks(Pf), kT, 0, tree_st, fg, tl.cc_tstart, tl.cc_ttgt, tbar, qbl);
   }
   // upward pass, transposed: interpolate down the tree
-  launch_down1(fg, qbl, st);
+  launch_down1(fg, qbl, tree_st);
+  if (tree_st != st) cudaEventRecord(join, tree_st);
   // near field, transposed (writes qbar, ybar), then the anterpolation adjoint (adds)
   const int nth = tg.npl <= 256 ? 256 : 512;
   if (mixed) {
@@ -779,6 +788,7 @@ void launch_tree_velocity_adjoint(const TreeGeom& tg, const StepGeom& fg, const 
   } else {
     launch_near_T<128>(tg, fg.leaves, tl, x, y, z, vbar, psrc, qbar, ybar, st);
   }
+  if (tree_st != st) cudaStreamWaitEvent(st, join, 0);
   launch_sources_T(tg, fg, ftab, psrc, qbl, qbar, ybar, st);
 }
 

@@ -23,10 +23,13 @@ struct TreeAdjointLists {
 // [3][tree panels * q], qbl [tree panels * q].  mixed: the transposed near
 // and well-separated pair sums in float32 on packed coordinates (the
 // forward's mixed arithmetic), everything else float64.
+// tree_st: the stream of the tree passes (with fork and join events), which run
+// beside the transposed near field; st itself where there is none.
 void launch_tree_velocity_adjoint(const TreeGeom& tg, const StepGeom& fg, const BliTable& ftab,
                                   const TreeAdjointLists& tl, const double* x, const double* y, const double* z,
                                   const double* vbar, const double4* psrc, double* tbar, double* qbl, double* qbar,
-                                  double* ybar, bool mixed, cudaStream_t st);
+                                  double* ybar, bool mixed, cudaStream_t st,
+                                  cudaStream_t tree_st, cudaEvent_t fork, cudaEvent_t join);
 
 // The reference's spectral FMM (proxy = particle degree; float64, or mixed:
 // float32 transposed pairs on packed coordinates): given vbar
