@@ -29,6 +29,7 @@
 #include "adjoint_pair32.cuh"
 #include "adjoint_tree.cuh"
 #include "device_common.cuh"
+#include "leaf_moments.cuh"
 
 namespace sbslpm {
 namespace {
@@ -49,39 +50,16 @@ unsigned split_ranks(int units) {
 }
 
 // Tbar_leaf[c][k] = sum_i B_k(x_i) vbar_c,i over the leaf's particles, one
-// block per (leaf, component c): the leaf-box bases in shared memory, the
-// particles in G contiguous groups (a thread per group and proxy), the
-// groups' sums added in order.
+// block per (leaf, component c), a direction at a time.
 __global__ void __launch_bounds__(kLeafThreads) k_tree_to_particles_T(TreeGeom tg, StepGeom fg,
                                                                      const double* __restrict__ vbar,
                                                                      double* __restrict__ tbar) {
-  extern __shared__ double sh[];  // npl values, npl n1 of each basis, G qx partial sums
-  const int f = blockIdx.x, c = blockIdx.y, npl = tg.npl, n1 = tg.n + 1, qx = n1 * n1;
-  const long pn = (long)fg.panels * qx;
-  double* sv = sh;
-  double* lx = sv + npl;
-  double* ly = lx + npl * n1;
-  double* part = ly + npl * n1;
-  for (int i = threadIdx.x; i < npl; i += blockDim.x) sv[i] = vbar[c * tg.N + (long)f * npl + i];
-  for (int i = threadIdx.x; i < npl * n1; i += blockDim.x) {
-    lx[i] = tg.lx[i];
-    ly[i] = tg.ly[i];
-  }
+  extern __shared__ double sh[];  // npl values, side n1 half-contracted
+  const int f = blockIdx.x, c = blockIdx.y, npl = tg.npl, qx = (tg.n + 1) * (tg.n + 1);
+  double* to = tbar + c * (long)fg.panels * qx + (long)(fg.offset + f) * qx;
+  for (int i = threadIdx.x; i < npl; i += blockDim.x) sh[grid_slot(tg, i)] = vbar[c * tg.N + (long)f * npl + i];
   __syncthreads();
-  const int G = blockDim.x / qx > 0 ? blockDim.x / qx : 1, per = (npl + G - 1) / G;
-  for (int t = threadIdx.x; t < G * qx; t += blockDim.x) {
-    const int gi = t / qx, k = t - gi * qx, a = k / n1, b = k - a * n1;
-    const int i1 = min(npl, (gi + 1) * per);
-    double acc = 0;
-    for (int i = gi * per; i < i1; i++) acc = fma(lx[i * n1 + a] * ly[i * n1 + b], sv[i], acc);
-    part[t] = acc;
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < qx; k += blockDim.x) {
-    double acc = part[k];
-    for (int gi = 1; gi < G; gi++) acc += part[gi * qx + k];
-    tbar[c * pn + (long)(fg.offset + f) * qx + k] = acc;
-  }
+  grid_moments(tg, sh, sh + npl, [&](int m, double s) { to[m] = s; });
 }
 
 // One level of the transpose of the downward pass: a parent at `level` adds
@@ -755,11 +733,8 @@ void launch_tree_velocity_adjoint(const TreeGeom& tg, const StepGeom& fg, const 
   }
   // leaf interpolation, transposed; non-leaf rows start at zero
   cudaMemsetAsync(tbar, 0, sizeof(double) * 3 * pn, tree_st);
-  const int n1 = tg.n + 1, groups = kLeafThreads / qx > 0 ? kLeafThreads / qx : 1;
-  static std::atomic<unsigned long long> attr_t{0};
-  raise_smem_once(attr_t, 128 * 1024, k_tree_to_particles_T);
   SB_LAUNCH(k_tree_to_particles_T, dim3((unsigned)fg.leaves, 3), kLeafThreads,
-            sizeof(double) * (tg.npl + 2 * tg.npl * n1 + groups * qx), tree_st, tg, fg, vbar, tbar);
+            sizeof(double) * (tg.npl + tg.side * (tg.n + 1)), tree_st, tg, fg, vbar, tbar);
   launch_up3(fg, tbar, tree_st);
   // well-separated interactions, transposed
   if (mixed) {

@@ -43,6 +43,7 @@ struct sbslpm_batch {
     int n = -1, qx = 0;
     TreeTables t;
     double *fpx = nullptr, *fcentre = nullptr, *fbounds = nullptr, *fchild = nullptr, *flx = nullptr, *fly = nullptr;
+    int* fplace = nullptr;
     int* fface = nullptr;
     std::vector<int> members;
     int* d_idx = nullptr;
@@ -164,6 +165,7 @@ sbslpm_status batch_setup(sbslpm_batch* b) {
     if (!D.t.c1d.empty()) SB_TRY(bupload(b, &D.fchild, D.t.c1d));
     SB_TRY(bupload(b, &D.flx, D.t.lx));
     SB_TRY(bupload(b, &D.fly, D.t.ly));
+    SB_TRY(bupload(b, &D.fplace, D.t.place));
   }
   b->Lf = b->degs[0].t.Lf;
   b->Pf = b->degs[0].t.Pf;
@@ -280,6 +282,8 @@ sbslpm_status batch_setup(sbslpm_batch* b) {
     tg.omega = c.omega;
     tg.lx = D.flx;
     tg.ly = D.fly;
+    tg.place = D.fplace;
+    tg.side = D.t.side;
     tg.fbounds = D.fbounds;
     tg.fface = D.fface;
     tg.near_start = ns;
@@ -430,7 +434,7 @@ void batch_velocity(sbslpm_batch* b, int stage, double dt_s, const double* vprev
     launch_bltc_near_batch(b->d_mem, b->M, b->Af, b->npl, b->cfg.kernel_eps, prec, x, y, z, b->psrc, b->psrcf,
                            b->near, b->splits, b->nt, b->tpt, b->near_expanded, st);
   if (b->aux_stream) cudaStreamWaitEvent(st, b->ev_join, 0);
-  launch_bltc_to_particles_batch(b->d_mem, b->M, b->Af, b->nmax, b->near, b->splits, v, st);
+  launch_bltc_to_particles_batch(b->d_mem, b->M, b->Af, b->npl, b->nmax, b->near, b->splits, v, st);
 }
 
 void batch_enqueue_step(sbslpm_batch* b, const double* x, const double* y, const double* z, const double* area,

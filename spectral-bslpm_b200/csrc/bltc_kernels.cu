@@ -28,6 +28,7 @@
 #include "../../include/sbslpm.h"
 #include "bve_kernels.cuh"
 #include "device_common.cuh"
+#include "leaf_moments.cuh"
 
 namespace sbslpm {
 
@@ -35,49 +36,10 @@ namespace {
 
 using namespace dev;
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 32 * kMomentWarps;
 
-// Barycentric Lagrange basis of degree n on Chebyshev extrema of [lo, hi]
-// without the reference's range check: displaced sources may sit slightly
-// outside their leaf, where the interpolant extrapolates smoothly.  The
-// second barycentric form multiplied through by prod_j (t - c_j):
-// f_i = w_i P_i / sum_k w_k P_k with P_i = prod_{j != i} (t - c_j), one
-// division instead of n + 2 (nodes within 1e-15 are hit exactly).
-__device__ __forceinline__ void bli_1d_free(double t, double lo, double hi, int n, const double* cosv,
-                                            const double* w, double* f) {
-  if (n == 0) {
-    f[0] = 1;
-    return;
-  }
-  const double range = 0.5 * (hi - lo), offset = 0.5 * (hi + lo);
-  double dl[kMaxDegree + 1];
-  int hit = -1;
-#pragma unroll
-  for (int i = 0; i <= kMaxDegree; i++) {
-    dl[i] = i <= n ? t - (cosv[i] * range + offset) : 1.0;
-    if (i <= n && hit < 0 && fabs(dl[i]) < 1e-15) hit = i;
-  }
-  if (hit >= 0) {
-    for (int i = 0; i <= n; i++) f[i] = (i == hit) ? 1.0 : 0.0;
-    return;
-  }
-  double pre[kMaxDegree + 1];
-  pre[0] = 1.0;
-#pragma unroll
-  for (int i = 1; i <= kMaxDegree; i++) pre[i] = pre[i - 1] * dl[i - 1];
-  double suf = 1.0, den = 0.0, v[kMaxDegree + 1];
-#pragma unroll
-  for (int i = kMaxDegree; i >= 0; i--) {
-    v[i] = i <= n ? w[i] * (pre[i] * suf) : 0.0;
-    den += v[i];
-    suf *= dl[i];
-  }
-  const double inv = 1.0 / den;
-#pragma unroll
-  for (int i = 0; i <= kMaxDegree; i++)
-    if (i <= n) f[i] = v[i] * inv;
-}
-
+// One leaf's sources (see the file comment).  N1 = proxy degree + 1, or 0 for any.
+template <int N1>
 __device__ __forceinline__ void bltc_sources_body(const TreeGeom& tg, const StepGeom& fg, const BliTable& tab, int f,
                                                   int stage, double dt_s, const double* __restrict__ vprev,
                                                   const double* __restrict__ x, const double* __restrict__ y,
@@ -86,10 +48,11 @@ __device__ __forceinline__ void bltc_sources_body(const TreeGeom& tg, const Step
                                                   float4* __restrict__ psrcf, double4* __restrict__ proxy,
                                                   int mixed) {
   extern __shared__ double sh[];
-  const int n1 = tg.n + 1, npl = tg.npl;
-  double* lx = sh;              // [npl][n1]
-  double* ly = lx + npl * n1;   // [npl][n1]
-  double* sw = ly + npl * n1;   // [npl]
+  const int n1 = N1 ? N1 : tg.n + 1, npl = tg.npl, ls = leaf_stride(n1);
+  double* lx = sh;              // [npl][ls]
+  double* ly = lx + npl * ls;   // [npl][ls]
+  double* sw = ly + npl * ls;   // [npl]
+  double* part = sw + npl;      // [warps][n1][n1]
   const int panel = fg.offset + f;
   const double* bd = tg.fbounds + 4 * panel;
   const int face = tg.fface[panel];
@@ -116,42 +79,29 @@ __device__ __forceinline__ void bltc_sources_body(const TreeGeom& tg, const Step
                              (float)((zz - cc[2]) * kPackScale), (float)w);
     double xi, eta;
     xieta_from_xyz_face(xx, yy, zz, face, xi, eta);
-    bli_1d_free(xi, bd[0], bd[1], tg.n, tab.cosv, tab.w, lx + k * n1);
-    bli_1d_free(eta, bd[2], bd[3], tg.n, tab.cosv, tab.w, ly + k * n1);
+    bli_1d_free<N1>(xi, bd[0], bd[1], tg.n, tab.cosv, tab.w, lx + k * ls);
+    bli_1d_free<N1>(eta, bd[2], bd[3], tg.n, tab.cosv, tab.w, ly + k * ls);
     sw[k] = w;
   }
   __syncthreads();
-  // proxy strengths S[a][b] = sum_k lx[k][a] ly[k][b] w_k: the particles are
-  // cut into G contiguous groups (G = threads / q), one thread per (group,
-  // proxy), and the G partial sums are added in group order
-  const int qx = n1 * n1, G = blockDim.x / qx > 0 ? blockDim.x / qx : 1;
-  double* part = sw + npl;  // [G][qx]
-  const int per = (npl + G - 1) / G;
-  for (int t = threadIdx.x; t < G * qx; t += blockDim.x) {
-    const int gi = t / qx, m = t - gi * qx, a = m / n1, b = m % n1;
-    const int k0 = gi * per, k1 = min(npl, k0 + per);
-    double acc = 0;
-    for (int k = k0; k < k1; k++) acc = fma(lx[k * n1 + a] * ly[k * n1 + b], sw[k], acc);
-    part[t] = acc;
-  }
+  // proxy strengths S[a][b] = sum_k lx[k][a] ly[k][b] w_k
+  const int qx = n1 * n1;
+  leaf_moments<N1>(lx, ly, ls, sw, npl, n1, part);
   __syncthreads();
-  for (int m = threadIdx.x; m < qx; m += blockDim.x) {
-    double acc = part[m];
-    for (int gi = 1; gi < G; gi++) acc += part[gi * qx + m];
-    proxy[(long)panel * qx + m].w = acc;
-  }
+  for (int m = threadIdx.x; m < qx; m += blockDim.x) proxy[(long)panel * qx + m].w = leaf_moment(part, qx, m);
 }
 
-__global__ void __launch_bounds__(kThreads)
+template <int N1>
+__global__ void __launch_bounds__(kThreads, N1 >= 6 && N1 <= 9 ? 4 : 2)
     k_bltc_sources(TreeGeom tg, StepGeom fg, BliTable tab, int stage, double dt_s, const double* __restrict__ vprev,
                    const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
                    const double* __restrict__ vors, const double* __restrict__ area, double4* __restrict__ psrc,
                    float4* __restrict__ psrcf, double4* __restrict__ proxy, int mixed) {
-  bltc_sources_body(tg, fg, tab, blockIdx.x, stage, dt_s, vprev, x, y, z, vors, area, psrc, psrcf, proxy, mixed);
+  bltc_sources_body<N1>(tg, fg, tab, blockIdx.x, stage, dt_s, vprev, x, y, z, vors, area, psrc, psrcf, proxy, mixed);
 }
 
 // Batched members (member blockIdx.y) on one particle grid.
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 4)
     k_bltc_sources_batch(const BatchMember* __restrict__ mem, int stage, double dt_s, const double* __restrict__ vprev,
                          const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
                          const double* __restrict__ vors, const double* __restrict__ area,
@@ -160,8 +110,11 @@ __global__ void __launch_bounds__(kThreads)
   const TreeGeom tg = m.tg;
   const StepGeom fg = m.fg;
   const long N = tg.N, mo = (long)blockIdx.y;
-  bltc_sources_body(tg, fg, m.tab, blockIdx.x, stage, dt_s, vprev ? vprev + mo * 3 * N : nullptr, x, y, z,
-                    vors + mo * N, area, psrc + mo * N, psrcf ? psrcf + mo * N : nullptr, m.fsrc, mixed);
+#define SB_SRC(N1)                                                                                            \
+  bltc_sources_body<N1>(tg, fg, m.tab, blockIdx.x, stage, dt_s, vprev ? vprev + mo * 3 * N : nullptr, x, y, z, \
+                        vors + mo * N, area, psrc + mo * N, psrcf ? psrcf + mo * N : nullptr, m.fsrc, mixed)
+  SB_LEAF_N1(tg.n + 1, SB_SRC)
+#undef SB_SRC
 }
 
 // Near leaf pairs: one CTA of NT threads per (target leaf, source split),
@@ -601,14 +554,23 @@ __global__ void k_near_slot_sum(TreeGeom tg, const float* __restrict__ slot, con
 }
 
 // Leaf proxy targets -> particles: v_i = (near-field splits summed in order)
-// + sum_a lx[k][a] sum_b ly[k][b] T[a][b], with the leaf-box basis of
-// particle k of the (uniform) leaf.
+// + sum_a lx[column][a] sum_b ly[row][b] T[a][b].  The inner sums depend on
+// the particle's row alone, so they are formed once per row of the leaf's
+// grid: 3 n1^2 side + 3 n1 npl FMAs per leaf where every particle of its own
+// took 3 n1^2 npl, bound by the shared-memory reads of T (a broadcast read
+// still fills 32 registers).  393,216 particles, 81 proxies: 21.5 us -> 12.0,
+// of which the velocities, near sums and targets are 6 at the memory's rate;
+// the results are the same bits.
+template <int N1>
 __device__ __forceinline__ void bltc_to_particles_body(const TreeGeom& tg, const StepGeom& fg, int f,
                                                        const double* __restrict__ tgt,
                                                        const double* __restrict__ near, int splits,
                                                        double* __restrict__ v) {
-  extern __shared__ double tsh[];  // 3 x qx
-  const int n1 = tg.n + 1, qx = n1 * n1, npl = tg.npl;
+  extern __shared__ double tsh[];
+  const int n1 = N1 ? N1 : tg.n + 1, qx = n1 * n1, npl = tg.npl, side = tg.side;
+  double* half = tsh + 3 * qx;           // [3][n1][side]
+  double* lx = half + 3 * n1 * side;     // [side][n1]
+  double* ly = lx + side * n1;           // [side][n1]
   const long pn = (long)fg.panels * qx;
   const long base = (long)(fg.offset + f) * qx;
   for (int m = threadIdx.x; m < qx; m += blockDim.x) {
@@ -616,37 +578,38 @@ __device__ __forceinline__ void bltc_to_particles_body(const TreeGeom& tg, const
     tsh[qx + m] = tgt[pn + base + m];
     tsh[2 * qx + m] = tgt[2 * pn + base + m];
   }
+  for (int m = threadIdx.x; m < side * n1; m += blockDim.x) {
+    lx[m] = tg.lx[m];
+    ly[m] = tg.ly[m];
+  }
+  __syncthreads();
+  for (int o = threadIdx.x; o < 3 * n1 * side; o += blockDim.x) {
+    const int ca = o / side, row = o - ca * side;  // component and a
+    double s = 0;
+#pragma unroll
+    for (int b = 0; b < n1; b++) s = fma(ly[row * n1 + b], tsh[ca * n1 + b], s);
+    half[o] = s;
+  }
   __syncthreads();
   for (int k = threadIdx.x; k < npl; k += blockDim.x) {
-    const double* lxk = tg.lx + k * n1;
-    const double* lyk = tg.ly + k * n1;
-    // the particle's eta basis in registers (n1 <= kMaxDegree + 1), read once
-    double lb[kMaxDegree + 1];
-#pragma unroll
-    for (int b = 0; b <= kMaxDegree; b++) lb[b] = b < n1 ? __ldg(lyk + b) : 0.0;
+    const int p = __ldg(tg.place + k);
+    const double* lxk = lx + (p & 0xffff) * n1;
+    const double* h = half + (p >> 16);
     double u0 = 0, u1 = 0, u2 = 0;
-    for (int a = 0; a < n1; a++) {
-      double s0 = 0, s1 = 0, s2 = 0;
 #pragma unroll
-      for (int b = 0; b <= kMaxDegree; b++) {
-        if (b < n1) {
-          s0 = fma(lb[b], tsh[a * n1 + b], s0);
-          s1 = fma(lb[b], tsh[qx + a * n1 + b], s1);
-          s2 = fma(lb[b], tsh[2 * qx + a * n1 + b], s2);
-        }
-      }
-      double la = __ldg(lxk + a);
-      u0 = fma(la, s0, u0);
-      u1 = fma(la, s1, u1);
-      u2 = fma(la, s2, u2);
+    for (int a = 0; a < n1; a++) {
+      const double la = lxk[a];
+      u0 = fma(la, h[a * side], u0);
+      u1 = fma(la, h[(n1 + a) * side], u1);
+      u2 = fma(la, h[(2 * n1 + a) * side], u2);
     }
     const long i = (long)f * npl + k;
     double n0 = 0, n1s = 0, n2 = 0;
     for (int y = 0; y < splits; y++) {
-      const double* p = near + (long)y * 3 * tg.N;
-      n0 += p[i];
-      n1s += p[tg.N + i];
-      n2 += p[2 * tg.N + i];
+      const double* nr = near + (long)y * 3 * tg.N;
+      n0 += nr[i];
+      n1s += nr[tg.N + i];
+      n2 += nr[2 * tg.N + i];
     }
     v[i] = n0 + u0;
     v[tg.N + i] = n1s + u1;
@@ -654,20 +617,24 @@ __device__ __forceinline__ void bltc_to_particles_body(const TreeGeom& tg, const
   }
 }
 
-__global__ void __launch_bounds__(kThreads)
+template <int N1>
+__global__ void __launch_bounds__(kThreads, 4)
     k_bltc_to_particles(TreeGeom tg, StepGeom fg, const double* __restrict__ tgt, const double* __restrict__ near,
                         int splits, double* __restrict__ v) {
-  bltc_to_particles_body(tg, fg, tg.leaf0 + blockIdx.x, tgt, near, splits, v);
+  bltc_to_particles_body<N1>(tg, fg, tg.leaf0 + blockIdx.x, tgt, near, splits, v);
 }
 
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 4)
     k_bltc_to_particles_batch(const BatchMember* __restrict__ mem, const double* __restrict__ near, int splits,
                               double* __restrict__ v) {
   const BatchMember& m = mem[blockIdx.y];
   const TreeGeom tg = m.tg;
   const StepGeom fg = m.fg;
   const long mo = blockIdx.y;
-  bltc_to_particles_body(tg, fg, blockIdx.x, m.ftgt, near + mo * splits * 3 * tg.N, splits, v + mo * 3 * tg.N);
+#define SB_TOP(N1)                                                                                           \
+  bltc_to_particles_body<N1>(tg, fg, blockIdx.x, m.ftgt, near + mo * splits * 3 * tg.N, splits, v + mo * 3 * tg.N)
+  SB_LEAF_N1(tg.n + 1, SB_TOP)
+#undef SB_TOP
 }
 
 }  // namespace
@@ -678,20 +645,26 @@ void launch_bltc_sources(const TreeGeom& tg, const StepGeom& fg, const BliTable&
                          const double* vprev, const double* x, const double* y, const double* z, const double* vors,
                          const double* area, double4* psrc, float4* psrcf, double4* proxy, bool mixed,
                          cudaStream_t st) {
-  size_t smem = sizeof(double) * ((size_t)tg.npl * (tg.n + 1) * 2 + tg.npl + kThreads);
-  static std::atomic<unsigned long long> attr{0};
-  raise_smem_once(attr, 200 * 1024, k_bltc_sources);
-  SB_LAUNCH(k_bltc_sources, (unsigned)fg.leaves, kThreads, smem, st, tg, fg, tab, stage, dt_s, vprev, x, y, z, vors,
-            area, psrc, psrcf, proxy, mixed ? 1 : 0);
+  const int n1 = tg.n + 1;
+  const size_t smem = leaf_smem(tg.npl, n1, 1);
+#define SB_SRC(N1)                                                                                                  \
+  {                                                                                                                 \
+    static std::atomic<unsigned long long> attr{0};                                                                 \
+    raise_smem_once(attr, kLeafSmem, k_bltc_sources<N1>);                                                           \
+    SB_LAUNCH(k_bltc_sources<N1>, (unsigned)fg.leaves, kThreads, smem, st, tg, fg, tab, stage, dt_s, vprev, x, y, z, \
+              vors, area, psrc, psrcf, proxy, mixed ? 1 : 0);                                                       \
+  }
+  SB_LEAF_N1(n1, SB_SRC)
+#undef SB_SRC
 }
 
 void launch_bltc_sources_batch(const BatchMember* mem, int members, int leaves, int npl, int nmax, int stage,
                                double dt_s, const double* vprev, const double* x, const double* y, const double* z,
                                const double* vors, const double* area, double4* psrc, float4* psrcf, bool mixed,
                                cudaStream_t st) {
-  size_t smem = sizeof(double) * ((size_t)npl * (nmax + 1) * 2 + npl + kThreads);
+  const size_t smem = leaf_smem(npl, nmax + 1, 1);
   static std::atomic<unsigned long long> attr{0};
-  raise_smem_once(attr, 200 * 1024, k_bltc_sources_batch);
+  raise_smem_once(attr, kLeafSmem, k_bltc_sources_batch);
   SB_LAUNCH(k_bltc_sources_batch, dim3((unsigned)leaves, (unsigned)members), kThreads, smem, st, mem, stage, dt_s,
             vprev, x, y, z, vors, area, psrc, mixed ? psrcf : nullptr, mixed ? 1 : 0);
 }
@@ -756,18 +729,26 @@ void launch_bltc_near_mutual(const TreeGeom& tg, const StepGeom& fg, const int4*
   SB_LAUNCH(k_near_slot_sum, blocks_for(tg.N, 256), 256, 0, st, tg, slot, x, y, z, near);
 }
 
-void launch_bltc_to_particles_batch(const BatchMember* mem, int members, int leaves, int nmax, const double* near,
-                                    int splits, double* v, cudaStream_t st) {
-  const int qx = (nmax + 1) * (nmax + 1);
+// proxy targets, their sums per row of the leaf's grid, the bases of its columns and rows
+static size_t to_particles_smem(int n1, int npl) {
+  int side = 1;
+  while (side * side < npl) side++;
+  return sizeof(double) * (3 * n1 * n1 + 5 * n1 * side);
+}
+
+void launch_bltc_to_particles_batch(const BatchMember* mem, int members, int leaves, int npl, int nmax,
+                                    const double* near, int splits, double* v, cudaStream_t st) {
   SB_LAUNCH(k_bltc_to_particles_batch, dim3((unsigned)leaves, (unsigned)members), kThreads,
-            sizeof(double) * 3 * qx, st, mem, near, splits, v);
+            to_particles_smem(nmax + 1, npl), st, mem, near, splits, v);
 }
 
 void launch_bltc_to_particles(const TreeGeom& tg, const StepGeom& fg, const double* tgt, const double* near,
                               int splits, double* v, cudaStream_t st) {
-  int qx = (tg.n + 1) * (tg.n + 1);
-  SB_LAUNCH(k_bltc_to_particles, (unsigned)(tg.owned > 0 ? tg.owned : fg.leaves), kThreads, sizeof(double) * 3 * qx,
-            st, tg, fg, tgt, near, splits, v);
+#define SB_TOP(N1)                                                                                    \
+  SB_LAUNCH(k_bltc_to_particles<N1>, (unsigned)(tg.owned > 0 ? tg.owned : fg.leaves), kThreads,       \
+            to_particles_smem(tg.n + 1, tg.npl), st, tg, fg, tgt, near, splits, v)
+  SB_LEAF_N1(tg.n + 1, SB_TOP)
+#undef SB_TOP
 }
 
 }  // namespace sbslpm

@@ -19,6 +19,7 @@
 
 #include "../../include/sbslpm.h"
 #include "device_common.cuh"
+#include "leaf_moments.cuh"
 #include "swe_kernels.cuh"
 
 namespace sbslpm {
@@ -26,45 +27,7 @@ namespace {
 
 using namespace dev;
 
-constexpr int kThreads = 256;
-
-// Barycentric basis of degree n on Chebyshev extrema of [lo, hi], extended
-// past the interval (displaced sources may leave their leaf); one division
-// (the second barycentric form multiplied through by prod_j (t - c_j)).
-__device__ __forceinline__ void swe_bli_free(double t, double lo, double hi, int n, const double* cosv,
-                                             const double* w, double* f) {
-  if (n == 0) {
-    f[0] = 1;
-    return;
-  }
-  const double range = 0.5 * (hi - lo), offset = 0.5 * (hi + lo);
-  double dl[kMaxDegree + 1];
-  int hit = -1;
-#pragma unroll
-  for (int i = 0; i <= kMaxDegree; i++) {
-    dl[i] = i <= n ? t - (cosv[i] * range + offset) : 1.0;
-    if (i <= n && hit < 0 && fabs(dl[i]) < 1e-15) hit = i;
-  }
-  if (hit >= 0) {
-    for (int i = 0; i <= n; i++) f[i] = (i == hit) ? 1.0 : 0.0;
-    return;
-  }
-  double pre[kMaxDegree + 1];
-  pre[0] = 1.0;
-#pragma unroll
-  for (int i = 1; i <= kMaxDegree; i++) pre[i] = pre[i - 1] * dl[i - 1];
-  double suf = 1.0, den = 0.0, v[kMaxDegree + 1];
-#pragma unroll
-  for (int i = kMaxDegree; i >= 0; i--) {
-    v[i] = i <= n ? w[i] * (pre[i] * suf) : 0.0;
-    den += v[i];
-    suf *= dl[i];
-  }
-  const double inv = 1.0 / den;
-#pragma unroll
-  for (int i = 0; i <= kMaxDegree; i++)
-    if (i <= n) f[i] = v[i] * inv;
-}
+constexpr int kThreads = 32 * kMomentWarps;
 
 // One CTA per treecode leaf: both fields' particle sources and their
 // anterpolation onto the leaf's proxies.  Step mode (no displacement arrays): the
@@ -73,7 +36,8 @@ __device__ __forceinline__ void swe_bli_free(double t, double lo, double hi, int
 // area (1 + dts div)(vor + dts tv) at x + dtd vprev (re-projected), w_div =
 // area (div + dts td) at x; stage 0: area vor and area div, undisplaced.
 // Piecewise mode: positions x + disp (re-projected) and strengths given.
-__global__ void __launch_bounds__(kThreads)
+template <int N1>
+__global__ void __launch_bounds__(kThreads, N1 >= 6 && N1 <= 9 ? 4 : 2)
     k_bltc_swe_sources(TreeGeom tg, StepGeom fg, BliTable tab, int stage, double dtd, double dts,
                        const double* __restrict__ vprev, const double* __restrict__ tprev,
                        const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
@@ -85,12 +49,12 @@ __global__ void __launch_bounds__(kThreads)
                        double4* __restrict__ proxy, double4* __restrict__ proxy2, int mixed,
                        const double* __restrict__ gcentre, int gq) {
   extern __shared__ double sh[];
-  const int f = blockIdx.x, n1 = tg.n + 1, npl = tg.npl;
-  double* lx = sh;              // [npl][n1] basis of the displaced vorticity sources
-  double* ly = lx + npl * n1;   // [npl][n1]
-  double* sw = ly + npl * n1;   // [npl] vorticity strengths
-  double* sd = sw + npl;        // [npl] divergence strengths
-  double* part = sd + npl;      // [2][G][qx] group partials
+  const int f = blockIdx.x, n1 = N1 ? N1 : tg.n + 1, npl = tg.npl, ls = leaf_stride(n1);
+  double* lx = sh;              // [npl][ls] basis of the displaced vorticity sources
+  double* ly = lx + npl * ls;   // [npl][ls]
+  double* sw = ly + npl * ls;   // [npl] vorticity strengths
+  double* sd = sw + npl;        // [npl] divergence strengths in the leaf grid's order
+  double* part = sd + npl;      // [warps][n1][n1]
   const int panel = fg.offset + f;
   const double* bd = tg.fbounds + 4 * panel;
   const int face = tg.fface[panel];
@@ -130,35 +94,20 @@ __global__ void __launch_bounds__(kThreads)
     }
     double xi, eta;
     xieta_from_xyz_face(xx, yy, zz, face, xi, eta);
-    swe_bli_free(xi, bd[0], bd[1], tg.n, tab.cosv, tab.w, lx + k * n1);
-    swe_bli_free(eta, bd[2], bd[3], tg.n, tab.cosv, tab.w, ly + k * n1);
+    bli_1d_free<N1>(xi, bd[0], bd[1], tg.n, tab.cosv, tab.w, lx + k * ls);
+    bli_1d_free<N1>(eta, bd[2], bd[3], tg.n, tab.cosv, tab.w, ly + k * ls);
     sw[k] = wv;
-    sd[k] = wd;
+    sd[grid_slot(tg, k)] = wd;
   }
   __syncthreads();
-  // S[a][b] = sum_k lx[k][a] ly[k][b] w_k over G contiguous particle groups,
-  // the partials added in group order (as k_bltc_sources); the divergence
-  // uses the grid's leaf-box basis tg.lx / tg.ly
-  const int qx = n1 * n1, G = blockDim.x / qx > 0 ? blockDim.x / qx : 1;
-  const int per = (npl + G - 1) / G;
-  for (int t = threadIdx.x; t < 2 * G * qx; t += blockDim.x) {
-    const int fld = t / (G * qx), tt = t - fld * G * qx;
-    const int gi = tt / qx, m = tt - gi * qx, a = m / n1, b = m % n1;
-    const int k0 = gi * per, k1 = min(npl, k0 + per);
-    double acc = 0;
-    if (fld == 0)
-      for (int k = k0; k < k1; k++) acc = fma(lx[k * n1 + a] * ly[k * n1 + b], sw[k], acc);
-    else
-      for (int k = k0; k < k1; k++) acc = fma(__ldg(tg.lx + k * n1 + a) * __ldg(tg.ly + k * n1 + b), sd[k], acc);
-    part[t] = acc;
-  }
+  // S[a][b] = sum_k lx[k][a] ly[k][b] w_k; the divergence's sources are the
+  // grid's particles
+  const int qx = n1 * n1;
+  leaf_moments<N1>(lx, ly, ls, sw, npl, n1, part);
   __syncthreads();
-  for (int m = threadIdx.x; m < 2 * qx; m += blockDim.x) {
-    const int fld = m / qx, mm = m - fld * qx;
-    double acc = part[fld * G * qx + mm];
-    for (int gi = 1; gi < G; gi++) acc += part[fld * G * qx + gi * qx + mm];
-    (fld == 0 ? proxy : proxy2)[(long)panel * qx + mm].w = acc;
-  }
+  for (int m = threadIdx.x; m < qx; m += blockDim.x) proxy[(long)panel * qx + m].w = leaf_moment(part, qx, m);
+  // (the displaced bases are done with: their space takes the half-contracted sums)
+  grid_moments(tg, sd, lx, [&](int m, double s) { proxy2[(long)panel * qx + m].w = s; });
 }
 
 // u = K x cross A - K (B - x (x.B)) (swe_kernels.cu's epilogue)
@@ -466,13 +415,18 @@ void launch_bltc_swe_sources(const TreeGeom& tg, const StepGeom& fg, const BliTa
                              const double* wd, double4* psrc, float4* psrcf,
                              double4* psrc2, float4* psrcf2, double4* proxy, double4* proxy2, bool mixed,
                              const double* gcentre, int gq, cudaStream_t st) {
-  const int n1 = tg.n + 1, qx = n1 * n1, G = kThreads / qx > 0 ? kThreads / qx : 1;
-  const size_t smem = sizeof(double) * ((size_t)tg.npl * n1 * 2 + 2 * (size_t)tg.npl + 2 * (size_t)G * qx);
-  static std::atomic<unsigned long long> attr{0};
-  raise_smem_once(attr, 200 * 1024, k_bltc_swe_sources);
-  SB_LAUNCH(k_bltc_swe_sources, (unsigned)fg.leaves, kThreads, smem, st, tg, fg, tab, stage, dtd, dts, vprev, tprev,
-            x, y, z, vors, divs, area, dispx, dispy, dispz, wv, wd, psrc, psrcf, psrc2, psrcf2, proxy, proxy2,
-            mixed ? 1 : 0, gcentre, gq);
+  const int n1 = tg.n + 1;
+  const size_t smem = leaf_smem(tg.npl, n1, 2);
+#define SB_SRC(N1)                                                                                             \
+  {                                                                                                            \
+    static std::atomic<unsigned long long> attr{0};                                                            \
+    raise_smem_once(attr, kLeafSmem, k_bltc_swe_sources<N1>);                                                  \
+    SB_LAUNCH(k_bltc_swe_sources<N1>, (unsigned)fg.leaves, kThreads, smem, st, tg, fg, tab, stage, dtd, dts,   \
+              vprev, tprev, x, y, z, vors, divs, area, dispx, dispy, dispz, wv, wd, psrc, psrcf, psrc2, psrcf2, \
+              proxy, proxy2, mixed ? 1 : 0, gcentre, gq);                                                      \
+  }
+  SB_LEAF_N1(n1, SB_SRC)
+#undef SB_SRC
 }
 
 void launch_bltc_swe_near(const TreeGeom& tg, const StepGeom& fg, int precision, const double* x, const double* y,

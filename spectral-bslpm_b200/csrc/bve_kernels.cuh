@@ -56,8 +56,11 @@ struct TreeGeom {
   int npl;                // particles per treecode leaf
   long N;                 // particles
   double eps, omega;
-  const double* lx;       // [npl][n+1]: leaf-box BLI basis of each particle's xi (same for every leaf)
-  const double* ly;       // [npl][n+1]: the same for eta
+  // the particles of a leaf are a tensor grid (the same for every leaf):
+  int side;               // its columns (and rows), side^2 = npl
+  const double* lx;       // [side][n+1]: leaf-box BLI basis of each column's xi
+  const double* ly;       // [side][n+1]: of each row's eta
+  const int* place;       // [npl]: particle's row << 16 | column
   const double* fbounds;  // [tree panels][4]: min_xi, max_xi, min_eta, max_eta (radians)
   const int* fface;       // [tree panels]
   const int* near_start;  // [tree leaves + 1]: CSR of near leaf pairs by target leaf
@@ -206,8 +209,8 @@ void launch_bltc_near_batch(const BatchMember* mem, int members, int leaves, int
                             const double* x, const double* y, const double* z, const double4* psrc,
                             const float4* psrcf, double* near, int splits, int nt, int tpt, bool expanded,
                             cudaStream_t st);
-void launch_bltc_to_particles_batch(const BatchMember* mem, int members, int leaves, int nmax, const double* near,
-                                    int splits, double* v, cudaStream_t st);
+void launch_bltc_to_particles_batch(const BatchMember* mem, int members, int leaves, int npl, int nmax,
+                                    const double* near, int splits, double* v, cudaStream_t st);
 void launch_depart_remap_batch(const StepGeom& g, const BliTable* tab, int members, const double* x,
                                const double* y, const double* z, const double* v0, const double* v1,
                                const double* v2, const double* v3, double dt, const double* vors, double* new_vors,

@@ -181,6 +181,8 @@ sbslpm_status precompute_tree(sbslpm_ctx* c) {
   if (!t.c1d.empty()) SB_TRY(upload(&c->fchild, t.c1d));
   SB_TRY(upload(&c->flx, t.lx));
   SB_TRY(upload(&c->fly, t.ly));
+  SB_TRY(upload(&c->fplace, t.place));
+  c->fside = t.side;
 
   // the traversal of the tree on the GPU (the same list, in the same order, as on the host)
   std::vector<TreeLists> lv;
@@ -302,6 +304,8 @@ void fill_geom(sbslpm_ctx* c) {
     t.omega = c->cfg.omega;
     t.lx = c->flx;
     t.ly = c->fly;
+    t.place = c->fplace;
+    t.side = c->fside;
     t.fbounds = c->fbounds;
     t.fface = c->fface;
     t.near_start = c->near_start;
@@ -862,7 +866,7 @@ sbslpm_status sbslpm_destroy(sbslpm_ctx* c) {
   if (c->swe_graph) cudaGraphExecDestroy(c->swe_graph);
   void* bufs[] = {c->px, c->il_basis, c->child_mat, c->centre, c->tgt_start, c->src_panel, c->il_row, c->src,
                   c->srcf, c->tgt, c->vbuf, c->partial, c->newvor, c->newtr, c->dep, c->err, c->fpx, c->fchild,
-                  c->fcentre, c->flx, c->fly, c->fbounds, c->fface, c->near_start, c->near_src, c->cc_start,
+                  c->fcentre, c->flx, c->fly, c->fplace, c->fbounds, c->fface, c->near_start, c->near_src, c->cc_start,
                   c->cc_src, c->fsrc, c->psrc, c->fsrcf, c->psrcf, c->ftgt, c->gx, c->near, c->s_fd,
                   c->s_ntan, c->s_pow15, c->s_filt, c->s_ptan, c->s_pface, c->s_ustart, c->s_umem, c->src2,
                   c->srcf2, c->tend, c->avor, c->adj_src, c->adj_vbar, c->adj_q, c->adj_y, c->adj_part,

@@ -60,6 +60,8 @@ struct sbslpm_ctx {
   long n_near = 0, n_cc = 0;
   std::vector<sbslpm_panel> fpanels;
   double *fpx = nullptr, *fchild = nullptr, *fcentre = nullptr, *flx = nullptr, *fly = nullptr, *fbounds = nullptr;
+  int* fplace = nullptr;
+  int fside = 0;
   int *fface = nullptr, *near_start = nullptr, *near_src = nullptr, *cc_start = nullptr, *cc_src = nullptr;
   int4* fentry32 = nullptr;  // the same entry table over the well-separated list (mixed, q <= 32)
   double4 *fsrc = nullptr, *psrc = nullptr;
@@ -218,6 +220,8 @@ struct TreeTables {
   int Lf = 0, Pf = 0, Af = 0, npl = 0, n = 0, qx = 0;
   std::vector<sbslpm_panel> fpanels;
   std::vector<double> fpx, centre, bounds, c1d, lx, ly;
+  std::vector<int> place;
+  int side = 0;
   std::vector<int> face;
   BliTable ftab{};
 };

@@ -3,7 +3,9 @@
 // quadtree truncated so that a leaf holds at most leaf_size particles, degree-n
 // Chebyshev proxies on every tree panel, the leaf-box 1-D bases of the
 // particle grid, and the near / well-separated interaction lists.
+#include <algorithm>
 #include <cmath>
+#include <utility>
 #include <vector>
 
 #include "context_internal.hpp"
@@ -85,24 +87,45 @@ sbslpm_status build_tree_tables(int L, int d, const std::vector<sbslpm_panel>& g
   t.c1d.clear();
   if (t.Lf > 1) child_basis_1d(t.fpanels, t.ftab, n, t.c1d, err);
 
-  // leaf-box basis of the particles of the first tree leaf (the same for every leaf)
+  // Leaf-box basis of the particles of the first tree leaf (the same for every
+  // leaf).  They form a tensor grid: a particle's xi is that of its grid
+  // panel's column and its node's column, its eta that of the rows, so a row of
+  // n1 values per column and per row, and each particle's (row, column).
   std::vector<double> interp_p;
   build_interp(d, false, interp_p);
-  t.lx.assign((size_t)npl * n1, 0.0);
-  t.ly.assign((size_t)npl * n1, 0.0);
+  const int side = (1 << m) * (d + 1);
+  t.side = side;
+  t.lx.assign((size_t)side * n1, 0.0);
+  t.ly.assign((size_t)side * n1, 0.0);
+  t.place.assign((size_t)npl, 0);
   const sbslpm_panel& leaf = t.fpanels[offf];
   const double lo_x = kPi / 4.0 * leaf.min_xi, hi_x = kPi / 4.0 * leaf.max_xi;
   const double lo_e = kPi / 4.0 * leaf.min_eta, hi_e = kPi / 4.0 * leaf.max_eta;
   const int first_dp = level_start(L - 1);  // the first leaf's descendants come first
+  using Key = std::pair<double, double>;    // the grid panel's lower bound, the node's position in it
+  std::vector<Key> cols, rows;
+  std::vector<char> seen((size_t)npl, 0);
+  auto index = [](std::vector<Key>& keys, const Key& key) {
+    const size_t i = std::find(keys.begin(), keys.end(), key) - keys.begin();
+    if (i == keys.size()) keys.push_back(key);
+    return (int)i;
+  };
   for (long k = 0; k < npl; k++) {
     const sbslpm_panel& dp = grid[first_dp + k / qp];
     const int j = (int)(k % qp);
+    const int ix = index(cols, {dp.min_xi, interp_p[4 * j]}), iy = index(rows, {dp.min_eta, interp_p[4 * j + 1]});
+    if (ix >= side || iy >= side || seen[iy * side + ix]) {
+      set_last_error("treecode set-up: a leaf's particles are not a tensor grid");
+      return SBSLPM_ERR_OUT_OF_PANEL;
+    }
+    seen[iy * side + ix] = 1;
+    t.place[k] = iy << 16 | ix;
     double max_xi = kPi / 4.0 * dp.max_xi, min_xi = kPi / 4.0 * dp.min_xi;
     double max_eta = kPi / 4.0 * dp.max_eta, min_eta = kPi / 4.0 * dp.min_eta;
     double xi = 0.5 * (max_xi + min_xi) + 0.5 * (max_xi - min_xi) * interp_p[4 * j];
     double eta = 0.5 * (max_eta + min_eta) + 0.5 * (max_eta - min_eta) * interp_p[4 * j + 1];
-    bli_1d(xi, lo_x, hi_x, n, t.ftab.cosv, t.ftab.w, &t.lx[k * n1], err);
-    bli_1d(eta, lo_e, hi_e, n, t.ftab.cosv, t.ftab.w, &t.ly[k * n1], err);
+    bli_1d(xi, lo_x, hi_x, n, t.ftab.cosv, t.ftab.w, &t.lx[(size_t)ix * n1], err);
+    bli_1d(eta, lo_e, hi_e, n, t.ftab.cosv, t.ftab.w, &t.ly[(size_t)iy * n1], err);
   }
   if (err) {
     set_last_error("treecode set-up: a particle fell outside its leaf");
