@@ -252,7 +252,7 @@ sbslpm_status batch_setup(sbslpm_batch* b) {
     SB_TRY(balloc(b, &fsrc, pn));
     std::vector<double4> init(pn);
     for (size_t i = 0; i < pn; i++) init[i] = make_double4(D.t.fpx[i], D.t.fpx[pn + i], D.t.fpx[2 * pn + i], 0.0);
-    SB_CUDA(cudaMemcpy(fsrc, init.data(), sizeof(double4) * pn, cudaMemcpyHostToDevice));
+    SB_TRY(copy_in(fsrc, init.data(), sizeof(double4) * pn));
     if (mixed) SB_TRY(balloc(b, &fsrcf, pn));
     SB_TRY(balloc(b, &ftgt, 3 * pn));
 

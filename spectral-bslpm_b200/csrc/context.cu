@@ -223,7 +223,7 @@ sbslpm_status precompute_tree(sbslpm_ctx* c) {
   SB_TRY(dalloc(&c->fsrc, pn));
   std::vector<double4> init(pn);
   for (size_t i = 0; i < pn; i++) init[i] = make_double4(fpx[i], fpx[pn + i], fpx[2 * pn + i], 0.0);
-  SB_CUDA(cudaMemcpy(c->fsrc, init.data(), sizeof(double4) * pn, cudaMemcpyHostToDevice));
+  SB_TRY(copy_in(c->fsrc, init.data(), sizeof(double4) * pn));
   SB_TRY(dalloc(&c->ftgt, 3 * pn));
   SB_TRY(dalloc(&c->psrc, N));
   // up to four near-field splits; on trees of few leaves as many as give the
@@ -459,8 +459,7 @@ sbslpm_status alloc_error_word(unsigned** err, unsigned** h_err) {
   SB_CUDA(cudaHostGetDevicePointer(&flag, *h_err, 0));
   unsigned words[4] = {0, 0, 0, 0};
   std::memcpy(words + 2, &flag, sizeof flag);
-  SB_CUDA(cudaMemcpy(*err, words, sizeof words, cudaMemcpyHostToDevice));
-  return SBSLPM_OK;
+  return copy_in(*err, words, sizeof words);
 }
 
 sbslpm_status error_word(unsigned* err, unsigned* h_err, cudaStream_t st, unsigned* bits) {
@@ -828,7 +827,7 @@ sbslpm_status sbslpm_create(const sbslpm_config* cfg, sbslpm_ctx** out) {
   if (s == SBSLPM_OK && cfg->forcing != SBSLPM_FORCING_NONE) {
     s = dalloc(&c->force, (size_t)c->A * c->q);
     if (s == SBSLPM_OK) s = dalloc(&c->d_time, 1);
-    if (s == SBSLPM_OK && cudaMemset(c->force, 0, sizeof(double) * c->A * c->q) != cudaSuccess) s = SBSLPM_ERR_CUDA;
+    if (s == SBSLPM_OK) s = zero_fill(c->force, sizeof(double) * c->A * c->q);
   }
   c->I = (long)c->list.size();
   if (s != SBSLPM_OK) {

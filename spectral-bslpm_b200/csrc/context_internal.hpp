@@ -172,23 +172,34 @@ sbslpm_status dalloc(T** p, size_t count) {
   return SBSLPM_OK;
 }
 
+// Set-up work on the legacy stream, waited for: a copy from pageable memory may
+// return once its bytes are staged and a memset at once, and the streams that
+// read the buffers (created non-blocking, or a caller's own) do not wait for
+// the legacy one.
+inline sbslpm_status copy_in(void* to, const void* from, size_t bytes) {
+  SB_CUDA(cudaMemcpy(to, from, bytes, cudaMemcpyHostToDevice));
+  SB_CUDA(cudaStreamSynchronize(nullptr));
+  return SBSLPM_OK;
+}
+
+inline sbslpm_status zero_fill(void* to, size_t bytes) {
+  SB_CUDA(cudaMemset(to, 0, bytes));
+  SB_CUDA(cudaStreamSynchronize(nullptr));
+  return SBSLPM_OK;
+}
+
 // Packed float32 sources of a tree (StepGeom::srcf), zeroed: the places that
 // close odd counts stay zero.
 inline sbslpm_status alloc_packed(float4** p, int panels, int q) {
   const size_t n = (size_t)panels * packed_stride(q);
   const sbslpm_status s = dalloc(p, n);
-  if (s != SBSLPM_OK) return s;
-  SB_CUDA(cudaMemset(*p, 0, sizeof(float4) * n));
-  SB_CUDA(cudaStreamSynchronize(nullptr));  // the context's streams do not wait for the legacy one
-  return SBSLPM_OK;
+  return s != SBSLPM_OK ? s : zero_fill(*p, sizeof(float4) * n);
 }
 
 template <class T>
 sbslpm_status upload(T** p, const std::vector<T>& h) {
-  sbslpm_status s = dalloc(p, h.size());
-  if (s != SBSLPM_OK) return s;
-  if (!h.empty()) SB_CUDA(cudaMemcpy(*p, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
-  return SBSLPM_OK;
+  const sbslpm_status s = dalloc(p, h.size());
+  return s != SBSLPM_OK || h.empty() ? s : copy_in(*p, h.data(), sizeof(T) * h.size());
 }
 
 #define SB_TRY(expr)                           \

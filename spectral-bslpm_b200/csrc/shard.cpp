@@ -267,7 +267,7 @@ sbslpm_status sbslpm_set_shard(sbslpm_ctx* c, int rank, int nranks, const unsign
   m.tab = c->ftab;
   m.fsrc = c->fsrc;
   m.ftgt = c->ftgt;
-  SB_CUDA(cudaMemcpy(c->self, &m, sizeof m, cudaMemcpyHostToDevice));
+  SB_TRY(copy_in(c->self, &m, sizeof m));
   // launch shapes are timed again on the new lists (the two-sided first-stage
   // kernel writes both leaves of a pair: unsharded contexts only)
   c->near_tuned = false;

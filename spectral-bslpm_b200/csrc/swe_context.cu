@@ -61,7 +61,7 @@ sbslpm_status swe_setup(sbslpm_ctx* c) {
     std::vector<double> fpx(3 * fpn);
     SB_CUDA(cudaMemcpy(fpx.data(), c->fpx, sizeof(double) * 3 * fpn, cudaMemcpyDeviceToHost));
     for (size_t i = 0; i < fpn; i++) init[i] = make_double4(fpx[i], fpx[fpn + i], fpx[2 * fpn + i], 0.0);
-    SB_CUDA(cudaMemcpy(c->fsrc2, init.data(), sizeof(double4) * fpn, cudaMemcpyHostToDevice));
+    SB_TRY(copy_in(c->fsrc2, init.data(), sizeof(double4) * fpn));
     if (c->cfg.precision == SBSLPM_MIXED) {
       SB_TRY(dalloc(&c->psrcf2, (size_t)ln));
       SB_TRY(alloc_packed(&c->fsrcf2, c->Pf, c->qx));
