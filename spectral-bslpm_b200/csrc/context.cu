@@ -824,6 +824,7 @@ sbslpm_status sbslpm_create(const sbslpm_config* cfg, sbslpm_ctx** out) {
       s = SBSLPM_ERR_CUDA;
   }
   if (s == SBSLPM_OK) s = allocate_workspace(c);
+  if (s == SBSLPM_OK && cfg->velocity == SBSLPM_VEL_FMM && !c->tree) s = poisson_setup(c);
   if (s == SBSLPM_OK && cfg->forcing != SBSLPM_FORCING_NONE) {
     s = dalloc(&c->force, (size_t)c->A * c->q);
     if (s == SBSLPM_OK) s = dalloc(&c->d_time, 1);

@@ -92,7 +92,7 @@ struct sbslpm_ctx {
   int* cc_cstart[4] = {};
   int cc_nchunks[4] = {};
   double* cc_partial = nullptr;  // [n_cc][3][qx] chunk sums
-  double* log_table = nullptr;      // Poisson: k_poisson_interact's logarithm table, built on the first solve
+  double* log_table = nullptr;   // Poisson: k_poisson_interact's logarithm table (contexts with the spectral FMM)
   double* swe_cc_partial = nullptr;  // [n_cc][6][qx] chunk sums of both SWE fields (mixed treecode)
   int cc_slots = 1, cc_len = 2;  // chunk slots per block (0: one block per target panel), entries per chunk
   int cc_tpt = 0;                 // 0: sources staged in shared memory; 1 | 2: barrier-free, targets per thread
@@ -217,6 +217,8 @@ void velocity_eval(sbslpm_ctx* c, int stage, double dt_s, const double* vprev, c
                    const double* z, const double* area, const double* vors, double* v, double* keep = nullptr);
 void launch_add3(const double* t, long n, double* a, double* b, double* cc, cudaStream_t st);
 sbslpm_status install_cc_lists(sbslpm_ctx* c, const std::vector<int>& cs, const std::vector<int>& csrc);
+// poisson.cu: the tables of the Poisson solve
+sbslpm_status poisson_setup(sbslpm_ctx* c);
 // shard.cpp: all-gathers a stage velocity [3][particles] over the context's
 // ranks (a no-op on an unsharded context); failures land in shard_status
 void shard_exchange(sbslpm_ctx* c, double* v);

@@ -206,10 +206,6 @@ sbslpm_status need_spectral_fmm(const sbslpm_ctx* c) {
   return SBSLPM_OK;
 }
 
-sbslpm_status need_log_table(sbslpm_ctx* c) {
-  return c->log_table ? SBSLPM_OK : upload(&c->log_table, log_table());
-}
-
 bool bad(const void* p) { return p == nullptr; }
 
 // downward_pass of one field through the three-field device pass: the
@@ -223,12 +219,13 @@ void downward_one(sbslpm_ctx* c, cudaStream_t st) {
 
 }  // namespace
 
+sbslpm_status sbslpm::poisson_setup(sbslpm_ctx* c) { return upload(&c->log_table, log_table()); }
+
 extern "C" {
 
 sbslpm_status sbslpm_poisson_fmm_interactions(sbslpm_ctx* c, const double* source, double* target) {
   if (!c || bad(source) || bad(target)) return SBSLPM_ERR_ARG;
   SB_TRY(need_spectral_fmm(c));
-  SB_TRY(need_log_table(c));
   cudaStream_t st = c->stream();
   launch_poisson(c->geom, c->log_table, source, target, st);
   return finish(c);
@@ -249,7 +246,6 @@ sbslpm_status sbslpm_downward_pass(sbslpm_ctx* c, double* proxy_target, double* 
 sbslpm_status sbslpm_poisson_fmm(sbslpm_ctx* c, const double* area, const double* pots, double* soln) {
   if (!c || bad(area) || bad(pots) || bad(soln)) return SBSLPM_ERR_ARG;
   SB_TRY(need_spectral_fmm(c));
-  SB_TRY(need_log_table(c));
   cudaStream_t st = c->stream();
   const size_t pn = (size_t)c->P * c->q, ln = (size_t)c->A * c->q, off = (size_t)c->off * c->q;
   // upward pass: proxy source weights into component 1 of the proxy-target buffer
