@@ -747,9 +747,15 @@ __device__ __forceinline__ void direct_reduce(double* red, double* bsum, long nt
   cl.sync();  // the blocks' sums stay until every rank has read them
 }
 
+// Where eps is at least kPlainEps and a tile's strengths are at most
+// kPlainStrength in magnitude, a pair's g is finite and a coincident pair adds
+// g * 0; any other tile (infinite strengths and NaN among them) takes the
+// guarded pairs, which leave a coincident pair out whatever its g.
+constexpr double kPlainEps = 1e-100, kPlainStrength = 1e200;
+
 // float64: two targets per lane (64 per block), each warp sweeping its own
 // `per` sources 32 at a time through its own tile, the next 32 loaded during
-// the current ones.
+// the current ones.  GUARD: eps below kPlainEps (negative or NaN among them).
 template <bool GUARD>
 __global__ void __cluster_dims__(1, kDirectRanks, 1) __launch_bounds__(kDirectThreads, 4)
     k_direct_bve64(long nt, const double* __restrict__ tx, const double* __restrict__ ty,
@@ -784,12 +790,21 @@ __global__ void __cluster_dims__(1, kDirectRanks, 1) __launch_bounds__(kDirectTh
     tile[warp][2 * lane] = a;
     tile[warp][2 * lane + 1] = b;
     __syncwarp();
+    const bool plain = !GUARD && __all_sync(0xffffffffu, fabs(b.y) <= kPlainStrength);
     load(k + 32 + lane);
     const int cnt = (int)min(32L, s1 - k);
+    if (plain) {
 #pragma unroll 8
-    for (int m = 0; m < cnt; m++) {
-      const double2 p = tile[warp][2 * m], q = tile[warp][2 * m + 1];
-      pairs64<GUARD>(x, y, z, p.x, p.y, q.x, q.y, eps2, ax, ay, az);
+      for (int m = 0; m < cnt; m++) {
+        const double2 p = tile[warp][2 * m], q = tile[warp][2 * m + 1];
+        pairs64<false>(x, y, z, p.x, p.y, q.x, q.y, eps2, ax, ay, az);
+      }
+    } else {
+#pragma unroll 2
+      for (int m = 0; m < cnt; m++) {
+        const double2 p = tile[warp][2 * m], q = tile[warp][2 * m + 1];
+        pairs64<true>(x, y, z, p.x, p.y, q.x, q.y, eps2, ax, ay, az);
+      }
     }
   }
 #pragma unroll
@@ -1293,9 +1308,7 @@ void launch_direct_bve(long nt, const double* tx, const double* ty, const double
   // a warp's share of the sources, at least one tile
   const long parts = kDirectRanks * (kDirectThreads / 32), per = std::max(32L, (ns + parts - 1) / parts);
   const dim3 grid(blocks_for(nt, 64), kDirectRanks);
-  // with eps > 0 a coincident pair adds g * 0; the guard is for eps = 0 and for
-  // eps so small that g would overflow
-  if (eps >= 1e-100)
+  if (eps >= kPlainEps)
     SB_LAUNCH(k_direct_bve64<false>, grid, kDirectThreads, 0, st, nt, tx, ty, tz, ns, sx, sy, sz, s, per, eps, ux, uy,
               uz);
   else

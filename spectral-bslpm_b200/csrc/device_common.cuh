@@ -51,17 +51,25 @@ __device__ __forceinline__ float recip_f32(float d) {
 // a = sum (g / 2) d gives u = -2/(4 pi) x cross a (kBiotSavartTwice): the
 // denominator is taken as |d|^2 + 2 eps, one chain of fused multiply-adds
 // with eps2 = twice_eps(eps), 13 FP64 operations in all.  Coincident points
-// add nothing: with eps > 0 because d = 0; with eps = 0 (GUARD) because g is
-// zeroed.
+// add nothing: because d = 0 where g is finite, which an eps > 0 of ordinary
+// size and a finite strength give; otherwise (GUARD: eps = 0, eps so small
+// that g overflows, any other eps) because g is zeroed where |d|^2 is not
+// positive, the eps added to it afterwards.
 __host__ __device__ __forceinline__ double twice_eps(double eps) { return eps < 8e307 ? 2.0 * eps : eps; }
+
+template <bool GUARD>
+__device__ __forceinline__ double pair_weight64(double dx, double dy, double dz, double sw, double eps2) {
+  if (!GUARD) return sw * recip_nr(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))));
+  const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+  const double g = sw * recip_nr(r2 + eps2);
+  return r2 > 0.0 ? g : 0.0;
+}
 
 template <bool GUARD>
 __device__ __forceinline__ void pair64(double tx, double ty, double tz, double sx, double sy, double sz, double sw,
                                        double eps2, double& ax, double& ay, double& az) {
   const double dx = sx - tx, dy = sy - ty, dz = sz - tz;
-  const double den = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
-  double g = sw * recip_nr(den);
-  if (GUARD) g = den > 0.0 ? g : 0.0;
+  const double g = pair_weight64<GUARD>(dx, dy, dz, sw, eps2);
   ax = fma(g, dx, ax);
   ay = fma(g, dy, ay);
   az = fma(g, dz, az);
@@ -90,11 +98,7 @@ __device__ __forceinline__ void pairs64(const double (&tx)[T], const double (&ty
 #pragma unroll
   for (int r = 0; r < T; r++) dx[r] = sx - tx[r];
 #pragma unroll
-  for (int r = 0; r < T; r++) {
-    const double den = fma(dx[r], dx[r], fma(dy[r], dy[r], fma(dz[r], dz[r], eps2)));
-    g[r] = sw * recip_nr(den);
-    if (GUARD) g[r] = den > 0.0 ? g[r] : 0.0;
-  }
+  for (int r = 0; r < T; r++) g[r] = pair_weight64<GUARD>(dx[r], dy[r], dz[r], sw, eps2);
 #pragma unroll
   for (int r = 0; r < T; r++) {
     ax[r] = fma(g[r], dx[r], ax[r]);
