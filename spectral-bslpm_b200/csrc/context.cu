@@ -591,9 +591,14 @@ sbslpm_status cc_autotune(sbslpm_ctx* c) {
   return SBSLPM_OK;
 }
 
-// Times every near-field launch shape (threads x targets per thread covering a
-// treecode leaf, 1..4 source-list splits, on small trees up to 16) on the stage-0 sources and keeps the
-// fastest.  Runs once per context, before the first step, outside any capture.
+// Times the near-field launch shapes (threads x targets per thread covering a
+// treecode leaf, 1..4 source-list splits, on trees of few leaves 2..near_max_splits)
+// on the stage-0 sources and keeps the fastest.  Runs once per context, before
+// the first step, outside any capture.  One split is left out on trees of few
+// leaves: us per launch at 1 / 2 / the best split count, leaves of 256, theta
+// 0.7, float64 and mixed: 96 leaves 277 / 170 / 92 and 81 / 68 / 41, 384 leaves
+// 506 / 410 / 369 and 192 / 160 / 142 (theta 0.5 to 0.85, leaves of 64 and 6 or
+// 24 leaves alike: one split 1.07 to 6 times the best).
 sbslpm_status near_autotune(sbslpm_ctx* c, const double* x, const double* y, const double* z, const double* area,
                             const double* vors) {
   if (!c->tree || (c->near_tuned && c->cc_tuned)) return SBSLPM_OK;
@@ -1247,7 +1252,7 @@ sbslpm_status sbslpm_set_near_tuning(sbslpm_ctx* c, int threads, int targets_per
   const bool ok = ((threads == 64 && (targets_per_thread == 1 || targets_per_thread == 2 || targets_per_thread == 4)) ||
                    (threads == 128 && (targets_per_thread == 1 || targets_per_thread == 2)) ||
                    (threads == 256 && (targets_per_thread == 1 || targets_per_thread == 2))) &&
-                  threads * targets_per_thread >= c->npl && splits >= 1 && splits <= 4;
+                  threads * targets_per_thread >= c->npl && splits >= 1 && splits <= c->near_max_splits;
   if (!ok) return set_last_error("unsupported near-field launch shape"), SBSLPM_ERR_ARG;
   c->near_nt = threads;
   c->near_tpt = targets_per_thread;
