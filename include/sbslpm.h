@@ -535,7 +535,8 @@ sbslpm_status sbslpm_nc_close(sbslpm_nc* nc);
  *   u_i = -1/(4 pi) sum_j (x_i x y_j) s_j / (1 - x_i.y_j + eps)
  * evaluated as x_i x sum_j s_j (y_j - x_i) / (|y_j - x_i|^2/2 + eps).
  * Pairs with y_j == x_i contribute nothing.  precision: SBSLPM_FP64 or
- * SBSLPM_MIXED.  stream: cudaStream_t or NULL. */
+ * SBSLPM_MIXED.  stream: cudaStream_t or NULL.  The results may overlay the
+ * inputs (they then pass through a stream-ordered temporary). */
 sbslpm_status sbslpm_direct_sum_bve(long n_targets, const double* tx, const double* ty, const double* tz,
                                     long n_sources, const double* sx, const double* sy, const double* sz,
                                     const double* strength, double eps, int precision, double* u_x, double* u_y,
@@ -550,8 +551,10 @@ sbslpm_status sbslpm_direct_sum_inv_lap(long n, const double* x, const double* y
  * sbslpm_direct_sum_bve, for callers that cannot let a library allocate
  * device memory: a host model that fixes its device footprint at start-up, or
  * that routes every device allocation through its own allocator.  Neither
- * entry point allocates device memory (their partial sums stay in shared
- * memory); this one promises it.
+ * entry point allocates device memory for its sums (they stay in shared
+ * memory); this one never does: results that overlay the inputs pass through
+ * one fixed 16 MiB array of the library, so such calls whose kernels overlap
+ * on a device (different streams or host threads) race: serialise them.
  * Limit: n_targets <= 699,050; larger calls return SBSLPM_ERR_ARG with a
  * message and do nothing.  Results equal sbslpm_direct_sum_bve's; in mixed
  * precision from about 100,000 targets up to the order of the sources'

@@ -451,6 +451,23 @@ void enqueue_step(sbslpm_ctx* c, const double* x, const double* y, const double*
   if (T > 0) cudaMemcpyAsync(tracers, c->newtr, sizeof(double) * ln * T, cudaMemcpyDeviceToDevice, st);
 }
 
+bool direct_in_place(long nt, std::initializer_list<const double*> targets, long ns,
+                     std::initializer_list<const double*> sources, std::initializer_list<const double*> results) {
+  auto shared = [](const double* a, long na, const double* b, long nb) {
+    const auto p = reinterpret_cast<uintptr_t>(a), q = reinterpret_cast<uintptr_t>(b);
+    return p < q + sizeof(double) * nb && q < p + sizeof(double) * na;
+  };
+  for (const double* const* r = results.begin(); r != results.end(); r++) {
+    for (const double* t : targets)
+      if (shared(*r, nt, t, nt)) return true;
+    for (const double* s : sources)
+      if (shared(*r, nt, s, ns)) return true;
+    for (const double* const* o = results.begin(); o != r; o++)
+      if (shared(*r, nt, *o, nt)) return true;
+  }
+  return false;
+}
+
 sbslpm_status alloc_error_word(unsigned** err, unsigned** h_err) {
   SB_CUDA(cudaMalloc(reinterpret_cast<void**>(err), 4 * sizeof(unsigned)));
   SB_CUDA(cudaMallocHost(reinterpret_cast<void**>(h_err), 2 * sizeof(unsigned)));
@@ -1184,8 +1201,22 @@ sbslpm_status sbslpm_direct_sum_bve(long nt, const double* tx, const double* ty,
     SB_CUDA(cudaStreamSynchronize(st));
     return SBSLPM_OK;
   }
-  launch_direct_bve(nt, tx, ty, tz, ns, sx, sy, sz, s, eps, precision, direct_groups(nt, ns), ux, uy, uz, st);
-  SB_CUDA(cudaGetLastError());
+  double* out[3] = {ux, uy, uz};
+  double* apart = nullptr;
+  if (direct_in_place(nt, {tx, ty, tz}, ns, {sx, sy, sz, s}, {ux, uy, uz})) {
+    SB_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&apart), sizeof(double) * 3 * nt, st));
+    for (int k = 0; k < 3; k++) out[k] = apart + k * nt;
+  }
+  launch_direct_bve(nt, tx, ty, tz, ns, sx, sy, sz, s, eps, precision, direct_groups(nt, ns), out[0], out[1], out[2],
+                    st);
+  cudaError_t e = cudaGetLastError();
+  if (apart) {
+    double* to[3] = {ux, uy, uz};
+    for (int k = 0; k < 3 && e == cudaSuccess; k++)
+      e = cudaMemcpyAsync(to[k], out[k], sizeof(double) * nt, cudaMemcpyDeviceToDevice, st);
+    cudaFreeAsync(apart, st);
+  }
+  SB_CUDA(e);
   SB_CUDA(cudaStreamSynchronize(st));
   return SBSLPM_OK;
 }

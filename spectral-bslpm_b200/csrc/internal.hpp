@@ -32,6 +32,12 @@ inline bool any_on_host(std::initializer_list<const void*> ps) {
   return false;
 }
 
+// True where one of a direct sum's results (nt values each) shares memory with
+// an input or with another result: its kernels write results while others still
+// read the sources, so such a call's results go through a buffer of their own.
+bool direct_in_place(long nt, std::initializer_list<const double*> targets, long ns,
+                     std::initializer_list<const double*> sources, std::initializer_list<const double*> results);
+
 // Device error word of a context or batch: four words at *err (the bits, a
 // spare, and the address of h_err[0], which device code sets with any bit) and
 // two page-locked words at *h_err (that flag, and where the bits are copied).

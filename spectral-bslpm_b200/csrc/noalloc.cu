@@ -5,9 +5,11 @@
 // through its own allocator, must not see cudaMalloc / cudaMallocAsync /
 // cudaFree calls appear inside the time loop.  The direct-sum kernels add
 // their partial sums within a cluster's shared memory, so neither direct-sum
-// entry point needs device scratch; this one keeps its own limits (its target
-// count, and fewer source groups in mixed precision for large ones), which its
-// callers' results and error handling depend on.
+// entry point needs device scratch for them; this one keeps its own limits (its
+// target count, and fewer source groups in mixed precision for large ones),
+// which its callers' results and error handling depend on.  Results that
+// overlay an input pass through a fixed array of this module (16 MiB, on the
+// GPU once this file's code is loaded there); such calls share it.
 #include <cuda_runtime.h>
 
 #include <string>
@@ -19,6 +21,7 @@
 namespace sbslpm {
 namespace {
 constexpr long kPartialDoubles = 1L << 21;  // 3 x targets x groups never exceeds this: 699,050 targets at most
+__device__ __align__(256) double g_apart[kPartialDoubles];
 }
 }  // namespace sbslpm
 
@@ -44,7 +47,7 @@ extern "C" sbslpm_status sbslpm_direct_sum_bve_noalloc(long nt, const double* tx
   }
   if (nt == 0) return SBSLPM_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  cudaError_t e;
+  cudaError_t e = cudaSuccess;
   if (ns == 0) {
     double* outs[3] = {ux, uy, uz};
     for (double* o : outs)
@@ -53,8 +56,18 @@ extern "C" sbslpm_status sbslpm_direct_sum_bve_noalloc(long nt, const double* tx
     long groups = direct_groups(nt, ns);
     const long fit = kPartialDoubles / (3 * nt);
     if (groups > fit) groups = fit;
-    launch_direct_bve(nt, tx, ty, tz, ns, sx, sy, sz, s, eps, precision, (int)groups, ux, uy, uz, st);
-    e = cudaGetLastError();
+    double *out[3] = {ux, uy, uz}, *to[3] = {ux, uy, uz};
+    void* apart = nullptr;
+    if (direct_in_place(nt, {tx, ty, tz}, ns, {sx, sy, sz, s}, {ux, uy, uz})) {
+      e = cudaGetSymbolAddress(&apart, g_apart);
+      for (int k = 0; k < 3 && e == cudaSuccess; k++) out[k] = static_cast<double*>(apart) + k * nt;
+    }
+    if (e == cudaSuccess) {
+      launch_direct_bve(nt, tx, ty, tz, ns, sx, sy, sz, s, eps, precision, (int)groups, out[0], out[1], out[2], st);
+      e = cudaGetLastError();
+    }
+    for (int k = 0; k < 3 && apart && e == cudaSuccess; k++)
+      e = cudaMemcpyAsync(to[k], out[k], sizeof(double) * nt, cudaMemcpyDeviceToDevice, st);
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
