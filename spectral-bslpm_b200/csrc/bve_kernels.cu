@@ -700,8 +700,8 @@ __global__ void __launch_bounds__(128, 8) k_depart_remap_batch(StepGeom g, BliTa
 }
 
 // ---------------------------------------------------------------------------
-// Stand-alone direct sums over arbitrary points.  A cluster of kDirectRanks
-// blocks owns a tile of targets; its blocks, and the warps (float64) or
+// Stand-alone direct sums over arbitrary points.  A cluster of blocks (one to
+// kDirectRanks) owns a tile of targets; its blocks, and the warps (float64) or
 // 64-thread groups (mixed) within a block, split the sources, and the partial
 // sums are added in a fixed order over shared memory and distributed shared
 // memory.  Nothing goes through device memory: with partial sums there, a call
@@ -711,29 +711,28 @@ __global__ void __launch_bounds__(128, 8) k_depart_remap_batch(StepGeom g, BliTa
 constexpr int kDirectThreads = 256, kDirectRanks = 8;
 constexpr int kInvLapThreads = 128;
 
-// Adds the partial sums red[PARTS][3][TB] of the cluster's blocks, part by
+// Adds the partial sums red[parts][3][TB] of the cluster's blocks, part by
 // part and rank by rank, and writes u = cb x cross a for the targets.
-template <int PARTS, int TB>
-__device__ __forceinline__ void direct_reduce(double* red, double* bsum, long nt, const double* __restrict__ tx,
-                                              const double* __restrict__ ty, const double* __restrict__ tz, double cb,
-                                              double* __restrict__ ux, double* __restrict__ uy,
-                                              double* __restrict__ uz) {
+template <int TB>
+__device__ __forceinline__ void direct_reduce(const double* red, double* bsum, int parts, long nt,
+                                              const double* __restrict__ tx, const double* __restrict__ ty,
+                                              const double* __restrict__ tz, double cb, double* __restrict__ ux,
+                                              double* __restrict__ uy, double* __restrict__ uz) {
   cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
   __syncthreads();
-  for (int k = threadIdx.x; k < 3 * TB; k += kDirectThreads) {
+  for (int k = threadIdx.x; k < 3 * TB; k += blockDim.x) {
     double a = red[k];
-#pragma unroll
-    for (int p = 1; p < PARTS; p++) a += red[p * 3 * TB + k];
+    for (int p = 1; p < parts; p++) a += red[p * 3 * TB + k];
     bsum[k] = a;
   }
   cl.sync();
-  constexpr int SHARE = TB / kDirectRanks;  // each rank finishes its share of the targets
-  if (threadIdx.x < SHARE) {
-    const int k = (int)cl.block_rank() * SHARE + threadIdx.x;
+  const int ranks = gridDim.y, share = TB / ranks;  // each rank finishes its share of the targets
+  for (int j = threadIdx.x; j < share; j += blockDim.x) {
+    const int k = blockIdx.y * share + j;
     const long i = (long)blockIdx.x * TB + k;
     if (i < nt) {
       double a[3] = {0, 0, 0};
-      for (int r = 0; r < kDirectRanks; r++) {
+      for (int r = 0; r < ranks; r++) {
         const double* b = cl.map_shared_rank(bsum, r);
 #pragma unroll
         for (int c = 0; c < 3; c++) a[c] += b[c * TB + k];
@@ -755,17 +754,23 @@ constexpr double kPlainEps = 1e-100, kPlainStrength = 1e200;
 
 // float64: two targets per lane (64 per block), each warp sweeping its own
 // `per` sources 32 at a time through its own tile, the next 32 loaded during
-// the current ones.  GUARD: eps below kPlainEps (negative or NaN among them).
+// the current ones.  The loop over a whole tile knows its length (1 x 300,000:
+// 494 us against 535 with one loop for every length).  GUARD: eps below kPlainEps (negative or NaN among them).
+constexpr int kDirectTile64 = 64;
+constexpr size_t direct_smem64(int parts) { return sizeof(double) * (parts * (128 + 3 * kDirectTile64) + 3 * kDirectTile64); }
+
 template <bool GUARD>
-__global__ void __cluster_dims__(1, kDirectRanks, 1) __launch_bounds__(kDirectThreads, 4)
+__global__ void __launch_bounds__(kDirectThreads, 4)
     k_direct_bve64(long nt, const double* __restrict__ tx, const double* __restrict__ ty,
                    const double* __restrict__ tz, long ns, const double* __restrict__ sx,
                    const double* __restrict__ sy, const double* __restrict__ sz, const double* __restrict__ sw,
                    long per, double eps, double* __restrict__ ux, double* __restrict__ uy, double* __restrict__ uz) {
-  constexpr int TPT = 2, TB = 32 * TPT, PARTS = kDirectThreads / 32;
-  __shared__ __align__(16) double2 tile[PARTS][64];
-  __shared__ double red[PARTS * 3 * TB], bsum[3 * TB];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int TPT = 2, TB = 32 * TPT;
+  static_assert(TB == kDirectTile64, "direct_smem64");
+  extern __shared__ __align__(16) double dsh[];  // a tile of 32 sources per warp, partial sums, the block's sums
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, parts = blockDim.x >> 5;
+  double2* tile = reinterpret_cast<double2*>(dsh) + warp * 64;
+  double* red = dsh + parts * 128;
   double x[TPT], y[TPT], z[TPT], ax[TPT], ay[TPT], az[TPT];
 #pragma unroll
   for (int r = 0; r < TPT; r++) {
@@ -776,7 +781,7 @@ __global__ void __cluster_dims__(1, kDirectRanks, 1) __launch_bounds__(kDirectTh
     ax[r] = ay[r] = az[r] = 0;
   }
   const double eps2 = twice_eps(eps);
-  const long s0 = (blockIdx.y * PARTS + warp) * per, s1 = min(ns, s0 + per);
+  const long s0 = (blockIdx.y * parts + warp) * per, s1 = min(ns, s0 + per);
   double2 a = make_double2(0, 0), b = a;
   auto load = [&](long k) {
     if (k < s1) {
@@ -787,22 +792,28 @@ __global__ void __cluster_dims__(1, kDirectRanks, 1) __launch_bounds__(kDirectTh
   load(s0 + lane);
   for (long k = s0; k < s1; k += 32) {
     __syncwarp();
-    tile[warp][2 * lane] = a;
-    tile[warp][2 * lane + 1] = b;
+    tile[2 * lane] = a;
+    tile[2 * lane + 1] = b;
     __syncwarp();
     const bool plain = !GUARD && __all_sync(0xffffffffu, fabs(b.y) <= kPlainStrength);
     load(k + 32 + lane);
     const int cnt = (int)min(32L, s1 - k);
-    if (plain) {
+    if (plain && cnt == 32) {
 #pragma unroll 8
+      for (int m = 0; m < 32; m++) {
+        const double2 p = tile[2 * m], q = tile[2 * m + 1];
+        pairs64<false>(x, y, z, p.x, p.y, q.x, q.y, eps2, ax, ay, az);
+      }
+    } else if (plain) {
+#pragma unroll 1
       for (int m = 0; m < cnt; m++) {
-        const double2 p = tile[warp][2 * m], q = tile[warp][2 * m + 1];
+        const double2 p = tile[2 * m], q = tile[2 * m + 1];
         pairs64<false>(x, y, z, p.x, p.y, q.x, q.y, eps2, ax, ay, az);
       }
     } else {
-#pragma unroll 2
+#pragma unroll 1
       for (int m = 0; m < cnt; m++) {
-        const double2 p = tile[warp][2 * m], q = tile[warp][2 * m + 1];
+        const double2 p = tile[2 * m], q = tile[2 * m + 1];
         pairs64<true>(x, y, z, p.x, p.y, q.x, q.y, eps2, ax, ay, az);
       }
     }
@@ -814,24 +825,30 @@ __global__ void __cluster_dims__(1, kDirectRanks, 1) __launch_bounds__(kDirectTh
     p[TB] = ay[r];
     p[2 * TB] = az[r];
   }
-  direct_reduce<PARTS, TB>(red, bsum, nt, tx, ty, tz, kBiotSavartTwice, ux, uy, uz);
+  direct_reduce<TB>(red, red + parts * 3 * TB, parts, nt, tx, ty, tz, kBiotSavartTwice, ux, uy, uz);
 }
 
 // Mixed: 128 targets per block, two per thread (the paired float32
 // instructions take one source against both), groups of 64 threads walking
-// the source groups; both tiles are measured relative to their first point
-// (in float64), so float32 carries only the small in-tile offsets.  A
-// target's sources are added in order, per tile of 128 in float32 and over
-// the tiles in float64.
-__global__ void __cluster_dims__(1, kDirectRanks, 1) __launch_bounds__(kDirectThreads)
+// shares of the source tiles; both tiles are measured relative to their first
+// point (in float64), so float32 carries only the small in-tile offsets.  The
+// sources are cut into `groups`, each into tiles of 128 from its first source
+// on; a tile is summed in float32, the tiles in float64.
+constexpr int kDirectTile32 = 128, kDirectPart32 = 64;
+constexpr size_t direct_smem32(int parts) {
+  return parts * (sizeof(float4) + 3 * sizeof(double)) * kDirectTile32 + 3 * sizeof(double) * kDirectTile32;
+}
+
+__global__ void __launch_bounds__(kDirectThreads)
     k_direct_bve32(long nt, const double* __restrict__ tx, const double* __restrict__ ty,
                    const double* __restrict__ tz, long ns, const double* __restrict__ sx,
                    const double* __restrict__ sy, const double* __restrict__ sz, const double* __restrict__ sw,
                    int groups, double eps, double* __restrict__ ux, double* __restrict__ uy, double* __restrict__ uz) {
-  constexpr int TB = 128, NT = 64, PARTS = kDirectThreads / NT;
-  __shared__ float4 tile[PARTS][TB];
-  __shared__ double red[PARTS * 3 * TB], bsum[3 * TB];
-  const int part = threadIdx.x / NT, th = threadIdx.x % NT;
+  constexpr int TB = kDirectTile32, NT = kDirectPart32;
+  extern __shared__ __align__(16) double dsh[];  // a source tile per part, partial sums, the block's sums
+  const int part = threadIdx.x / NT, th = threadIdx.x % NT, parts = blockDim.x / NT;
+  float4* tile = reinterpret_cast<float4*>(dsh) + part * TB;
+  double* red = dsh + parts * 2 * TB;
   const long i0 = blockIdx.x * (long)TB;
   const double tcx = tx[i0], tcy = ty[i0], tcz = tz[i0];
   float dtx[2], dty[2], dtz[2];
@@ -845,40 +862,44 @@ __global__ void __cluster_dims__(1, kDirectRanks, 1) __launch_bounds__(kDirectTh
   }
   const float feps = (float)eps;
   const float2 eps2 = make_float2(feps, feps);
-  const long per = (ns + groups - 1) / groups;
-  for (int grp = blockIdx.y * PARTS + part; grp < groups; grp += kDirectRanks * PARTS) {
-    const long s0 = grp * per, s1 = min(ns, s0 + per);
-    for (long b = s0; b < s1; b += TB) {
-      const double scx = sx[b], scy = sy[b], scz = sz[b];
-      const int cnt = (int)min((long)TB, s1 - b);
-      asm volatile("bar.sync %0, %1;" : : "r"(1 + part), "n"(NT) : "memory");
+  // tile u of the sources: number u % tiles of group u / tiles (the last groups may be short or empty)
+  const long per = (ns + groups - 1) / groups, tiles = (per + TB - 1) / TB, units = groups * tiles;
+  const long p0 = blockIdx.y * parts + part, shares = (long)gridDim.y * parts;
+  const long u0 = units * p0 / shares, u1 = units * (p0 + 1) / shares;
+  long s0 = u0 / tiles * per, b = s0 + u0 % tiles * TB;
+  for (long u = u0; u < u1; u++, b += TB) {
+    if (b >= s0 + per) s0 += per, b = s0;
+    const long s1 = min(ns, s0 + per);
+    if (b >= s1) continue;
+    const double scx = sx[b], scy = sy[b], scz = sz[b];
+    const int cnt = (int)min((long)TB, s1 - b);
+    asm volatile("bar.sync %0, %1;" : : "r"(1 + part), "n"(NT) : "memory");
 #pragma unroll
-      for (int r = 0; r < 2; r++) {
-        const int m = th + NT * r;
-        const long k = b + m;
-        if (m < cnt)
-          tile[part][m] = make_float4((float)((sx[k] - scx) * kPackScale), (float)((sy[k] - scy) * kPackScale),
-                                      (float)((sz[k] - scz) * kPackScale), (float)sw[k]);
-      }
-      asm volatile("bar.sync %0, %1;" : : "r"(1 + part), "n"(NT) : "memory");
-      const float cx = (float)((scx - tcx) * kPackScale), cy = (float)((scy - tcy) * kPackScale),
-                  cz = (float)((scz - tcz) * kPackScale);
-      const float2 bx = make_float2(cx - dtx[0], cx - dtx[1]), by = make_float2(cy - dty[0], cy - dty[1]),
-                   bz = make_float2(cz - dtz[0], cz - dtz[1]);
-      float2 fx = make_float2(0.f, 0.f), fy = fx, fz = fx;
-#pragma unroll 8
-      for (int m = 0; m < cnt; m++) {
-        const float4 v = tile[part][m];
-        pair32x2<true>(bx, by, bz, make_float2(v.x, v.x), make_float2(v.y, v.y), make_float2(v.z, v.z),
-                       make_float2(v.w, v.w), eps2, fx, fy, fz);
-      }
-      ax[0] += fx.x;
-      ay[0] += fy.x;
-      az[0] += fz.x;
-      ax[1] += fx.y;
-      ay[1] += fy.y;
-      az[1] += fz.y;
+    for (int r = 0; r < 2; r++) {
+      const int m = th + NT * r;
+      const long k = b + m;
+      if (m < cnt)
+        tile[m] = make_float4((float)((sx[k] - scx) * kPackScale), (float)((sy[k] - scy) * kPackScale),
+                              (float)((sz[k] - scz) * kPackScale), (float)sw[k]);
     }
+    asm volatile("bar.sync %0, %1;" : : "r"(1 + part), "n"(NT) : "memory");
+    const float cx = (float)((scx - tcx) * kPackScale), cy = (float)((scy - tcy) * kPackScale),
+                cz = (float)((scz - tcz) * kPackScale);
+    const float2 bx = make_float2(cx - dtx[0], cx - dtx[1]), by = make_float2(cy - dty[0], cy - dty[1]),
+                 bz = make_float2(cz - dtz[0], cz - dtz[1]);
+    float2 fx = make_float2(0.f, 0.f), fy = fx, fz = fx;
+#pragma unroll 8
+    for (int m = 0; m < cnt; m++) {
+      const float4 v = tile[m];
+      pair32x2<true>(bx, by, bz, make_float2(v.x, v.x), make_float2(v.y, v.y), make_float2(v.z, v.z),
+                     make_float2(v.w, v.w), eps2, fx, fy, fz);
+    }
+    ax[0] += fx.x;
+    ay[0] += fy.x;
+    az[0] += fz.x;
+    ax[1] += fx.y;
+    ay[1] += fy.y;
+    az[1] += fz.y;
   }
 #pragma unroll
   for (int r = 0; r < 2; r++) {
@@ -887,7 +908,7 @@ __global__ void __cluster_dims__(1, kDirectRanks, 1) __launch_bounds__(kDirectTh
     p[TB] = ay[r];
     p[2 * TB] = az[r];
   }
-  direct_reduce<PARTS, TB>(red, bsum, nt, tx, ty, tz, kBiotSavartPacked, ux, uy, uz);
+  direct_reduce<TB>(red, red + parts * 3 * TB, parts, nt, tx, ty, tz, kBiotSavartPacked, ux, uy, uz);
 }
 
 // inv_lap (src/direct_sum_impl.hpp:20-27): soln_i += sum_{j != i}
@@ -1297,23 +1318,42 @@ int direct_groups(long nt, long ns) {
   return (int)(gsel < 1 ? 1 : (gsel > 64 ? 64 : gsel));
 }
 
+// Shares of the sources per tile of targets, a power of two: as many as give
+// the GPU `want` parts (warps or 64-thread groups) in all, none without a
+// source tile of its own, kDirectRanks blocks of max_parts at most; a block
+// takes them before the cluster does.  Few targets need all 64 shares to reach
+// every SM, many targets none, and a share without sources only waits and is
+// added: us per call with eight full blocks for every tile of targets and by
+// this rule, 10,007 x 24,577 points 260 / 256 (float64), 191 / 165 (mixed);
+// 100,000 x 12,000 1,106 / 1,116, 1,984 / 682; 600,000 x 33 756 / 64, 418 / 62;
+// 2,000,000 x 3,000 5,695 / 5,220, 42,200 / 2,660.
+struct DirectShape {
+  unsigned parts, ranks;
+};
+static DirectShape direct_shape(long target_tiles, long source_tiles, long want, unsigned max_parts) {
+  unsigned shares = 1;
+  while (shares < kDirectRanks * max_parts && shares < source_tiles && target_tiles * shares < want) shares *= 2;
+  const unsigned parts = std::min(shares, max_parts);
+  return {parts, shares / parts};
+}
+
 void launch_direct_bve(long nt, const double* tx, const double* ty, const double* tz, long ns, const double* sx,
                        const double* sy, const double* sz, const double* s, double eps, int precision, int groups,
                        double* ux, double* uy, double* uz, cudaStream_t st) {
+  const long waves = 16L * 148;  // of 32 warps (float64) or 16 64-thread groups per SM
   if (precision == SBSLPM_MIXED) {
-    SB_LAUNCH(k_direct_bve32, dim3(blocks_for(nt, 128), kDirectRanks), kDirectThreads, 0, st, nt, tx, ty, tz, ns, sx,
-              sy, sz, s, groups, eps, ux, uy, uz);
+    const unsigned blocks = blocks_for(nt, kDirectTile32);
+    const long per = (ns + groups - 1) / groups, units = groups * ((per + kDirectTile32 - 1) / kDirectTile32);
+    const DirectShape d = direct_shape(blocks, units, 16 * waves, kDirectThreads / kDirectPart32);
+    launch_cluster(k_direct_bve32, blocks, d.ranks, d.parts * kDirectPart32, direct_smem32(d.parts), st, nt, tx, ty, tz,
+                   ns, sx, sy, sz, s, groups, eps, ux, uy, uz);
     return;
   }
-  // a warp's share of the sources, at least one tile
-  const long parts = kDirectRanks * (kDirectThreads / 32), per = std::max(32L, (ns + parts - 1) / parts);
-  const dim3 grid(blocks_for(nt, 64), kDirectRanks);
-  if (eps >= kPlainEps)
-    SB_LAUNCH(k_direct_bve64<false>, grid, kDirectThreads, 0, st, nt, tx, ty, tz, ns, sx, sy, sz, s, per, eps, ux, uy,
-              uz);
-  else
-    SB_LAUNCH(k_direct_bve64<true>, grid, kDirectThreads, 0, st, nt, tx, ty, tz, ns, sx, sy, sz, s, per, eps, ux, uy,
-              uz);
+  const unsigned blocks = blocks_for(nt, kDirectTile64);
+  const DirectShape d = direct_shape(blocks, (ns + 31) / 32, 32 * waves, kDirectThreads / 32);
+  const long per = (ns + d.parts * d.ranks - 1) / (d.parts * d.ranks);  // sources of a warp
+  launch_cluster(eps >= kPlainEps ? k_direct_bve64<false> : k_direct_bve64<true>, blocks, d.ranks, 32 * d.parts,
+                 direct_smem64(d.parts), st, nt, tx, ty, tz, ns, sx, sy, sz, s, per, eps, ux, uy, uz);
 }
 
 void launch_ssw_forcing(int leaves, int q, int type, double omega, const double* time, const double* x,
