@@ -317,33 +317,10 @@ __device__ __forceinline__ void project_to_sphere_rcp(double& x, double& y, doub
   z *= inv;
 }
 
-// The cell [b, b + 1] 2/n - 1 (times pi/4) of t along one direction of the
-// face's n = 2^(levels-1) leaves, t on a boundary belonging to the upper one.
-// The boundaries are those the tree descent compares with: fl(pi/4 * dyadic),
-// its 0.5 pi/4 (max + min) being the same number.  The guess is off by one at
-// most and corrected against them.
-__device__ __forceinline__ double leaf_edge(int b, int n) { return b * (2.0 / n) - 1.0; }
-
-__device__ __forceinline__ int leaf_cell(double t, int n) {
-  int b = (int)floor(fma(t, 4.0 / kPi, 1.0) * (0.5 * n));
-  b = max(0, min(n - 1, b));
-  if (b > 0 && t < kPi / 4.0 * leaf_edge(b, n)) b--;
-  else if (b < n - 1 && t >= kPi / 4.0 * leaf_edge(b + 1, n)) b++;
-  return b;
-}
-
-// Bits of b spread to the even positions.
-__device__ __forceinline__ unsigned spread_bits(unsigned b) {
-  b = (b | (b << 8)) & 0x00ff00ffu;
-  b = (b | (b << 4)) & 0x0f0f0f0fu;
-  b = (b | (b << 2)) & 0x33333333u;
-  return (b | (b << 1)) & 0x55555555u;
-}
-
 // locate_basis for the departure / remap kernel: one reciprocal for the face's
-// axis, the leaf from the cells of xi and eta instead of a descent through the
-// levels (child c of a level has xi bit bx, eta bit be: c = 2 (1 - be) + (bx
-// xor be)), the barycentric basis with one reciprocal per direction.
+// axis, the leaf from the cells of xi and eta (leaf_by_cells) instead of a
+// descent through the levels, the barycentric basis with one reciprocal per
+// direction.
 template <int D>
 __device__ __forceinline__ void locate_basis_rcp(const StepGeom& g, const BliTable& tab, double x, double y, double z,
                                                  Basis<D>& b, unsigned& err) {
@@ -355,17 +332,11 @@ __device__ __forceinline__ void locate_basis_rcp(const StepGeom& g, const BliTab
   const double r = recip_full(den);
   const double xi = atan(num_xi * r), eta = atan(num_eta * r);
   if (!(xi == xi) || !(eta == eta)) err |= kErrNonFinite;  // NaN coordinates
-  const int n = 1 << (g.levels - 1);
-  int bx = leaf_cell(xi, n);
-  const int be = leaf_cell(eta, n);
-  // xi on a boundary: at the level that cuts there (bit ffs - 1 of the cells)
-  // the descent takes the upper half with the upper half of eta only
-  if (bx > 0 && xi == kPi / 4.0 * leaf_edge(bx, n) && !((be >> (__ffs(bx) - 1)) & 1)) bx--;
-  const Bounds bd{leaf_edge(bx, n), leaf_edge(bx + 1, n), leaf_edge(be, n), leaf_edge(be + 1, n)};
-  const unsigned leaf = (spread_bits(~be & (n - 1)) << 1) | spread_bits(bx ^ be);
+  Bounds bd;
+  const unsigned leaf = leaf_by_cells(xi, eta, g.levels, bd);
   bli_1d_common<D>(xi, kPi / 4.0 * bd.min_xi, kPi / 4.0 * bd.max_xi, tab, b.fx, err);
   bli_1d_common<D>(eta, kPi / 4.0 * bd.min_eta, kPi / 4.0 * bd.max_eta, tab, b.fe, err);
-  b.row = ((long)face * n * n + leaf) * g.q;
+  b.row = (((long)face << (2 * (g.levels - 1))) + leaf) * g.q;
 }
 
 // sum_m field[row + m] * fx[i] fe[j] with m = i (D+1) + j, in m order.

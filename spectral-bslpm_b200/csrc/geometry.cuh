@@ -77,15 +77,8 @@ struct Bounds {
   double min_xi, max_xi, min_eta, max_eta;
 };
 
-// Point location by tree descent (point_locate_panel,
-// src/interp_funcs_impl.hpp:114-142), with child ids and bounds computed from
-// the uniform quadtree's numbering (refine_cube,
-// src/initialize_cubed_sphere.cpp:64-141) instead of read from a panel table.
-// Returns the leaf panel id; xi/eta are the point's coordinates on its face.
-SB_HD int locate_leaf(double x, double y, double z, int levels, double& xi, double& eta, Bounds& b,
-                      unsigned& err) {
-  int face = face_from_xyz(x, y, z);
-  xieta_from_xyz_face(x, y, z, face, xi, eta);
+// Descent from the face's panel to the leaf that holds (xi, eta).
+SB_HD int descend_to_leaf(int face, double xi, double eta, int levels, Bounds& b, unsigned& err) {
   b.min_xi = -1;
   b.max_xi = 1;
   b.min_eta = -1;
@@ -121,6 +114,60 @@ SB_HD int locate_leaf(double x, double y, double z, int levels, double& xi, doub
     id = level_start(lev + 1) + 4 * (id - level_start(lev)) + c;
   }
   return id;
+}
+
+// Point location by tree descent (point_locate_panel,
+// src/interp_funcs_impl.hpp:114-142), with child ids and bounds computed from
+// the uniform quadtree's numbering (refine_cube,
+// src/initialize_cubed_sphere.cpp:64-141) instead of read from a panel table.
+// Returns the leaf panel id; xi/eta are the point's coordinates on its face.
+SB_HD int locate_leaf(double x, double y, double z, int levels, double& xi, double& eta, Bounds& b,
+                      unsigned& err) {
+  const int face = face_from_xyz(x, y, z);
+  xieta_from_xyz_face(x, y, z, face, xi, eta);
+  return descend_to_leaf(face, xi, eta, levels, b, err);
+}
+
+// The cell [b, b + 1] 2/n - 1 (times pi/4) of t along one direction of the
+// face's n = 2^(levels-1) leaves, t on a boundary belonging to the upper one.
+// The boundaries are those the tree descent compares with: fl(pi/4 * dyadic),
+// its 0.5 pi/4 (max + min) being the same number.  The guess is off by one at
+// most and corrected against them.
+SB_HD double leaf_edge(int b, int n) { return b * (2.0 / n) - 1.0; }
+
+SB_HD int leaf_cell(double t, int n) {
+  int b = (int)floor(fma(t, 4.0 / kPi, 1.0) * (0.5 * n));
+  b = b < 0 ? 0 : b > n - 1 ? n - 1 : b;
+  if (b > 0 && t < kPi / 4.0 * leaf_edge(b, n)) b--;
+  else if (b < n - 1 && t >= kPi / 4.0 * leaf_edge(b + 1, n)) b++;
+  return b;
+}
+
+// Bits of b spread to the even positions.
+SB_HD unsigned spread_bits(unsigned b) {
+  b = (b | (b << 8)) & 0x00ff00ffu;
+  b = (b | (b << 4)) & 0x0f0f0f0fu;
+  b = (b | (b << 2)) & 0x33333333u;
+  return (b | (b << 1)) & 0x55555555u;
+}
+
+// descend_to_leaf without the descent, for xi and eta that are numbers: the
+// leaf's number within the face from the cells of xi and eta (child c of a
+// level has xi bit bx, eta bit be: c = 2 (1 - be) + (bx xor be)), and its
+// bounds.
+SB_HD unsigned leaf_by_cells(double xi, double eta, int levels, Bounds& b) {
+  const int n = 1 << (levels - 1);
+  int bx = leaf_cell(xi, n);
+  const int be = leaf_cell(eta, n);
+  // xi on a boundary: at the level that cuts there (the cells' bit that is
+  // bx's lowest one) the descent takes the upper half with the upper half of
+  // eta only
+  if (bx > 0 && xi == kPi / 4.0 * leaf_edge(bx, n) && !(be & bx & -bx)) bx--;
+  b.min_xi = leaf_edge(bx, n);
+  b.max_xi = leaf_edge(bx + 1, n);
+  b.min_eta = leaf_edge(be, n);
+  b.max_eta = leaf_edge(be + 1, n);
+  return (spread_bits(~be & (n - 1)) << 1) | spread_bits(bx ^ be);
 }
 
 // One direction of interp_vals_bli (src/interp_funcs_impl.hpp:11-112):
