@@ -24,8 +24,9 @@ __device__ __forceinline__ void flag(unsigned* err, unsigned bits) {
 
 // 1/d from the hardware approximation r and one third-order step
 // (Householder's iteration for 1/d): with e = 1 - d r, r (1 + e + e^2) leaves
-// an error of e^3 -- below 2^-56 from the approximation's 2^-20 or better --
-// in three FP64 operations instead of the four of two Newton steps.  d > 0.
+// an error of e^3 -- at most 2^-60 from the approximation's 2^-20 or better --
+// before the last rounding, in three FP64 operations instead of the four of two
+// Newton steps.  d of either sign, 1/d normal.
 __device__ __forceinline__ double recip_nr(double d) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
@@ -33,8 +34,9 @@ __device__ __forceinline__ double recip_nr(double d) {
   return fma(r, fma(e, e, e), r);
 }
 
-// 1/d to within half a unit in the last place: recip_nr and one residual
-// step.  d of either sign, normal.
+// 1/d with a residual step on recip_nr: what is left of the error before the
+// last rounding is its square (below 2^-105), so the result is off by that
+// rounding alone, 2^-53 (1 + 2^-50) relative.  d of either sign, 1/d normal.
 __device__ __forceinline__ double recip_full(double d) {
   const double r = recip_nr(d);
   return fma(r, fma(-d, r, 1.0), r);

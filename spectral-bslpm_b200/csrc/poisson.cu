@@ -7,71 +7,16 @@
 // the solve is u with -Laplacian(u) = f for mean-zero f.
 #include <cuda_runtime.h>
 
-#include <cmath>
-#include <cstring>
-#include <vector>
-
 #include "context_internal.hpp"
 #include "device_common.cuh"
 #include "list64.cuh"
+#include "log_table.cuh"
 
 using namespace sbslpm;
 
 namespace {
 
 constexpr double kInvLapConst = -0.07957747154594767;  // -1/(4 pi), as the reference writes it
-
-// log(a) of a positive normal a by table (P. T. P. Tang, "Table-driven
-// implementation of the logarithm function in IEEE floating-point
-// arithmetic", ACM TOMS 16, 1990): a = 2^k m with m in [0.6875, 1.375), the
-// interval of m gives c close to 1/m, r = m c - 1 is exact in one fused
-// multiply-add up to its rounding, and log a = k log 2 - log c + log(1 + r)
-// with |r| <= 2^-7 and the series of log(1 + r) to r^8.  log c and log 2 are
-// held in two parts, the high ones short enough that k log 2 - log c is exact;
-// c = 1 on both sides of 1.  Against long double over (0, 2], powers of two
-// down to 2^-49 and near 1: relative error rms 4.8e-17 as CUDA's log, at most
-// 1.6e-16 (log: 1.1e-16), far below that of its argument 1 - x.y (1e-16
-// absolute); 6.4e11 against 3.3e11 per second.
-constexpr int kLogBits = 7, kLogN = 1 << kLogBits, kLogFirst = 0x3fe60000;  // the high word of 0.6875
-constexpr double kLn2Hi = 0x1.62e42fefap-1, kLn2Lo = 0x1.cf79abc9e3b3ap-40;
-
-__device__ __forceinline__ double table_log(double a, const double2* __restrict__ cv, const double* __restrict__ lo) {
-  const int hi = __double2hiint(a), t = hi - kLogFirst, k = t >> 20, i = (t >> (20 - kLogBits)) & (kLogN - 1);
-  const double m = __hiloint2double(hi - (k << 20), __double2loint(a));
-  const double2 c = cv[i];
-  const double r = fma(m, c.x, -1.0);
-  const double kd = (double)k;
-  double p = fma(r, -1.0 / 8, 1.0 / 7);
-  p = fma(r, p, -1.0 / 6);
-  p = fma(r, p, 1.0 / 5);
-  p = fma(r, p, -1.0 / 4);
-  p = fma(r, p, 1.0 / 3);
-  p = fma(r, p, -1.0 / 2);
-  const double tail = fma(r * r, p, fma(kd, kLn2Lo, lo[i]));
-  const double big = fma(kd, kLn2Hi, c.y), sum = big + r;  // |big| > |r| or big = 0: the remainder is exact
-  return sum + ((r - (sum - big)) + tail);
-}
-
-// [kLogN] (c, high part of -log c), then [kLogN] its low part.
-std::vector<double> log_table() {
-  std::vector<double> t(3 * kLogN);
-  auto edge = [](int i) {
-    const unsigned long long bits = (unsigned long long)(kLogFirst + (i << (20 - kLogBits))) << 32;
-    double d;
-    std::memcpy(&d, &bits, sizeof d);
-    return d;
-  };
-  for (int i = 0; i < kLogN; i++) {
-    const double a = edge(i), b = edge(i + 1);
-    const double c = a == 1.0 || b == 1.0 ? 1.0 : 2.0 / (a + b);
-    const long double v = -std::log((long double)c);
-    const double hi = (double)(std::nearbyint(v * 0x1p40L) * 0x1p-40L);  // k log 2's high part ends at 2^-40 as well
-    t[2 * i] = c;
-    t[2 * i + 1] = hi;
-    t[2 * kLogN + i] = (double)(v - hi);
-  }
-  return t;
-}
 
 // poisson_panel_interaction (src/fmm_interactions/inverse_poisson_impl.hpp:22-52)
 // owner-computes, on the list organisation of list64.cuh: S source splits of
