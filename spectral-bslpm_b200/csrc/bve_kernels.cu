@@ -579,8 +579,14 @@ __global__ void k_reduce_groups(const double* __restrict__ partial, int groups, 
 // kernel is bound by float64 division and atan latency, not by its 136 bytes
 // of traffic per particle.
 
-// VEC: the gathered fields are read two values at a time (q even, rows on
-// 16-byte boundaries).
+// Whether a build with two values per load exists: rows of an even q of at most
+// 16 values.  From 36 values on, the loads of a row that the compiler keeps in
+// flight spill 1.5 to 5.6 KB of registers (degree 7, 393,216 particles: 388 us
+// with them, 176 with one value per load at the same register bound).
+constexpr bool depart_vec(int D) { return D <= 3 && (D + 1) * (D + 1) % 2 == 0; }
+
+// VEC: the gathered fields are read two values at a time (rows on 16-byte
+// boundaries).
 template <int D, bool VEC>
 __device__ __forceinline__ void gather_velocity(const Basis<D>& b, const double* __restrict__ v, long n, double& x,
                                                 double& y, double& z) {
@@ -657,13 +663,19 @@ __device__ __forceinline__ void depart_remap_body(const StepGeom& g, const BliTa
   flag(g.err, err);
 }
 
-// 128 threads; held to 64 registers (BLOCKS = 8 per SM) where the grid fills
-// the SMs that often: the chain of four locate -> gather rounds per particle
-// is latency-bound, and the extra resident warps measured 9 us per launch
-// faster at 393,216 particles than a 76-register build.  A grid of at most
-// four blocks per SM has the registers to keep a round's loads in flight.
-// 393,216 particles: 74 us with a descent per location and one value per
-// load, 65 us now.
+// Blocks of 128 threads per SM, which bound the registers of a thread.  The
+// chain of four locate -> gather rounds per particle is latency-bound: up to
+// degree 3, 64 registers (eight blocks) where the grid fills the SMs that
+// often, and a grid of at most four blocks per SM has the registers to keep a
+// round's loads in flight; above, the basis and the row's values need them at
+// any size.  us per launch at 8 / 6 / 4 / 3 blocks, degree 4 at 153,600
+// particles 48 / 42 / 33 / 35, 5 at 221,184 50 / 45 / 49 / 55, 6 at 301,056 95 /
+// 104 / 84 / 97, 7 at 98,304 54 / 51 / 58 / 49, 9 at 153,600 111 / 100 / 88 /
+// 80, 10 at 185,856 181 / 161 / 124 / 126; degree 3 at 393,216 65 / 69 / 74 /
+// -.  Before (a descent per location, eight blocks throughout): degree 3 at
+// 393,216 72 us, 4 42, 5 58, 6 90, 7 51, 9 118, 10 173.
+constexpr int depart_blocks(int D, bool few) { return D > 6 ? 3 : D > 3 ? 4 : few ? 4 : 8; }
+
 template <int D, int MODE, bool VEC, int BLOCKS>
 __global__ void __launch_bounds__(128, BLOCKS) k_depart_remap(StepGeom g, BliTable tab, const double* __restrict__ x, const double* __restrict__ y,
                                const double* __restrict__ z, const double* __restrict__ v0,
@@ -685,8 +697,8 @@ __global__ void __launch_bounds__(128, BLOCKS) k_depart_remap(StepGeom g, BliTab
 
 // Batched members on one particle grid (member blockIdx.y): departure and
 // remap in one pass (mode 3), stage velocities v_k + m * 3n, vorticity + m * n.
-template <int D, bool VEC>
-__global__ void __launch_bounds__(128, 8) k_depart_remap_batch(StepGeom g, BliTable tab, const double* __restrict__ x,
+template <int D, bool VEC, int BLOCKS>
+__global__ void __launch_bounds__(128, BLOCKS) k_depart_remap_batch(StepGeom g, BliTable tab, const double* __restrict__ x,
                                      const double* __restrict__ y, const double* __restrict__ z,
                                      const double* __restrict__ v0, const double* __restrict__ v1,
                                      const double* __restrict__ v2, const double* __restrict__ v3, double dt,
@@ -1249,41 +1261,45 @@ static bool aligned16(std::initializer_list<const double*> ps) {
   return true;
 }
 
+// f(std::integral_constant<int, degree>).
+template <class F>
+static void with_degree(int degree, F f) {
+  switch (degree) {
+#define SB_DEGREE(D)                            \
+  case D:                                       \
+    f(std::integral_constant<int, D>());        \
+    break;
+    SB_DEGREE(0) SB_DEGREE(1) SB_DEGREE(2) SB_DEGREE(3) SB_DEGREE(4) SB_DEGREE(5) SB_DEGREE(6) SB_DEGREE(7)
+    SB_DEGREE(8) SB_DEGREE(9) SB_DEGREE(10)
+#undef SB_DEGREE
+  }
+}
+
 void launch_depart_remap(const StepGeom& g, const BliTable* tab, const double* x, const double* y, const double* z,
                          const double* v0, const double* v1, const double* v2, const double* v3, double dt,
                          double* dep, const double* vors, const double* tracers, int T, double* new_vors,
                          double* new_tracers, int mode, cudaStream_t st, VelocityOut vel) {
   long n = (long)g.leaves * g.q;
-  unsigned grid = blocks_for(n, 128);
-  // rows of an even q on 16-byte boundaries where every gathered field is
-  const bool vec = aligned16({v0, v1, v2, vors}) && n % 2 == 0;
-  const bool few = grid <= 4 * 148;
-#define SB_DRL(D, MODE, VEC, BLOCKS)                                                                                \
-  SB_LAUNCH((k_depart_remap<D, MODE, VEC, BLOCKS>), grid, 128, 0, st, g, *tab, x, y, z, v0, v1, v2, v3, dt, dep, \
-            vors, tracers, T, new_vors, new_tracers, vel)
-#define SB_DRM(D, MODE, BLOCKS)                                   \
-  if (((D + 1) * (D + 1)) % 2 == 0 && vec)                        \
-    SB_DRL(D, MODE, (((D + 1) * (D + 1)) % 2 == 0), BLOCKS);      \
-  else                                                            \
-    SB_DRL(D, MODE, false, BLOCKS)
-#define SB_DR(D)             \
-  case D:                    \
-    if (mode == 1) {         \
-      SB_DRM(D, 1, 8);       \
-    } else if (mode == 2) {  \
-      SB_DRM(D, 2, 8);       \
-    } else if (few) {        \
-      SB_DRM(D, 3, 4);       \
-    } else {                 \
-      SB_DRM(D, 3, 8);       \
-    }                        \
-    break;
-  switch (g.degree) {
-    SB_DR(0) SB_DR(1) SB_DR(2) SB_DR(3) SB_DR(4) SB_DR(5) SB_DR(6) SB_DR(7) SB_DR(8) SB_DR(9) SB_DR(10)
-  }
-#undef SB_DR
-#undef SB_DRM
-#undef SB_DRL
+  const unsigned grid = blocks_for(n, 128);
+  const bool vec = aligned16({v0, v1, v2, vors}) && n % 2 == 0, few = grid <= 4 * 148;
+  with_degree(g.degree, [&](auto d) {
+    constexpr int D = d.value;
+    auto launch = [&](auto m, auto v, auto f) {
+      SB_LAUNCH((k_depart_remap<D, m.value, v.value, depart_blocks(D, f.value)>), grid, 128, 0, st, g, *tab, x, y, z, v0,
+                v1, v2, v3, dt, dep, vors, tracers, T, new_vors, new_tracers, vel);
+    };
+    auto sized = [&](auto m, auto v) {
+      if (few) launch(m, v, std::true_type());
+      else launch(m, v, std::false_type());
+    };
+    auto loads = [&](auto m) {
+      if (depart_vec(D) && vec) sized(m, std::bool_constant<depart_vec(D)>());
+      else sized(m, std::false_type());
+    };
+    if (mode == 1) loads(std::integral_constant<int, 1>());
+    else if (mode == 2) loads(std::integral_constant<int, 2>());
+    else loads(std::integral_constant<int, 3>());
+  });
 }
 
 void launch_depart_remap_batch(const StepGeom& g, const BliTable* tab, int members, const double* x,
@@ -1292,20 +1308,20 @@ void launch_depart_remap_batch(const StepGeom& g, const BliTable* tab, int membe
                                cudaStream_t st) {
   const long n = (long)g.leaves * g.q;
   const dim3 grid(blocks_for(n, 128), (unsigned)members);
-  const bool vec = aligned16({v0, v1, v2, vors}) && n % 2 == 0;
-#define SB_DRB(D)                                                                                                  \
-  case D:                                                                                                          \
-    if (((D + 1) * (D + 1)) % 2 == 0 && vec)                                                                       \
-      SB_LAUNCH((k_depart_remap_batch<D, (((D + 1) * (D + 1)) % 2 == 0)>), grid, 128, 0, st, g, *tab, x, y, z, v0, \
-                v1, v2, v3, dt, vors, new_vors);                                                                   \
-    else                                                                                                           \
-      SB_LAUNCH((k_depart_remap_batch<D, false>), grid, 128, 0, st, g, *tab, x, y, z, v0, v1, v2, v3, dt, vors,    \
-                new_vors);                                                                                         \
-    break;
-  switch (g.degree) {
-    SB_DRB(0) SB_DRB(1) SB_DRB(2) SB_DRB(3) SB_DRB(4) SB_DRB(5) SB_DRB(6) SB_DRB(7) SB_DRB(8) SB_DRB(9) SB_DRB(10)
-  }
-#undef SB_DRB
+  const bool vec = aligned16({v0, v1, v2, vors}) && n % 2 == 0, few = (long)grid.x * members <= 4 * 148;
+  with_degree(g.degree, [&](auto d) {
+    constexpr int D = d.value;
+    auto launch = [&](auto v, auto f) {
+      SB_LAUNCH((k_depart_remap_batch<D, v.value, depart_blocks(D, f.value)>), grid, 128, 0, st, g, *tab, x, y, z, v0,
+                v1, v2, v3, dt, vors, new_vors);
+    };
+    auto sized = [&](auto v) {
+      if (few) launch(v, std::true_type());
+      else launch(v, std::false_type());
+    };
+    if (depart_vec(D) && vec) sized(std::bool_constant<depart_vec(D)>());
+    else sized(std::false_type());
+  });
 }
 
 // Source groups of the mixed direct sum (a group's tiles start at its own
