@@ -92,7 +92,7 @@ __device__ __forceinline__ void bltc_sources_body(const TreeGeom& tg, const Step
 }
 
 template <int N1>
-__global__ void __launch_bounds__(kThreads, N1 >= 6 && N1 <= 9 ? 4 : 2)
+__global__ void __launch_bounds__(kThreads, 4)
     k_bltc_sources(TreeGeom tg, StepGeom fg, BliTable tab, int stage, double dt_s, const double* __restrict__ vprev,
                    const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
                    const double* __restrict__ vors, const double* __restrict__ area, double4* __restrict__ psrc,

@@ -37,7 +37,7 @@ constexpr int kThreads = 32 * kMomentWarps;
 // area (div + dts td) at x; stage 0: area vor and area div, undisplaced.
 // Piecewise mode: positions x + disp (re-projected) and strengths given.
 template <int N1>
-__global__ void __launch_bounds__(kThreads, N1 >= 6 && N1 <= 9 ? 4 : 2)
+__global__ void __launch_bounds__(kThreads, 4)
     k_bltc_swe_sources(TreeGeom tg, StepGeom fg, BliTable tab, int stage, double dtd, double dts,
                        const double* __restrict__ vprev, const double* __restrict__ tprev,
                        const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,

@@ -120,13 +120,9 @@ __device__ __forceinline__ void leaf_moments(const double* lx, const double* ly,
                                              int n1, double* part) {
   if constexpr (N1 > 0) {
     leaf_moments_t<(N1 + 2) / 3>(lx, ly, ls, w, npl, N1, part);
-  } else {
-    switch ((n1 + 2) / 3) {
-      case 1: leaf_moments_t<1>(lx, ly, ls, w, npl, n1, part); break;
-      case 2: leaf_moments_t<2>(lx, ly, ls, w, npl, n1, part); break;
-      case 3: leaf_moments_t<3>(lx, ly, ls, w, npl, n1, part); break;
-      default: leaf_moments_t<4>(lx, ly, ls, w, npl, n1, part); break;
-    }
+  } else {  // n1 <= 5 (SB_LEAF_N1)
+    if (n1 <= 3) leaf_moments_t<1>(lx, ly, ls, w, npl, n1, part);
+    else leaf_moments_t<2>(lx, ly, ls, w, npl, n1, part);
   }
 }
 
@@ -169,10 +165,12 @@ __device__ __forceinline__ int grid_slot(const TreeGeom& tg, int k) {
 }  // namespace sbslpm::dev
 
 // Proxy degrees 5..10 (the well-separated kernels' range) run with the degree
-// as a constant, which bounds the basis' products and keeps the sources at 64
-// registers, four blocks per SM (98,304 particles in 384 blocks: one wave, 21.6
-// -> 13.9 us); below, one general form.  In a batch each block finds its
-// member's.
+// as a constant, which bounds the basis' products; below, one general form.
+// Every form is held to 64 registers, four blocks per SM (98,304 particles in
+// 384 blocks: one wave, 21.6 -> 13.9 us).  Source kernels at two and at four
+// blocks, us: degree 10, 393,216 particles in leaves of 256 35.4 / 27.4, 13,824
+// in leaves of 9 24.2 / 15.5; degree 4, 393,216 particles 31 / 22.  In a batch
+// each block finds its member's.
 #define SB_LEAF_N1(n1, CALL)     \
   switch (n1) {                  \
     case 6: CALL(6); break;      \
