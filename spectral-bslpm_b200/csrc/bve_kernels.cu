@@ -424,7 +424,7 @@ template <int Q, bool ALL_LEAVES, bool GUARD, bool MIXED>
 __device__ __forceinline__ void interact_wide_body(const StepGeom& g, int tix, int gy, int ngy,
                                                    const double4* __restrict__ src, const float4* __restrict__ srcf,
                                                    double* __restrict__ out, long out_stride) {
-  constexpr int TPL = (Q + 31) / 32, NW = 4, Q2 = (Q + 1) / 2;
+  constexpr int TPL = (Q + 31) / 32, NW = 4, Q2 = (Q + 1) / 2, kRow = row_of(Q);
   using Src = typename std::conditional<MIXED, float4, double4>::type;
   // MIXED: sources staged two at a time, transposed, (x0,x1,y0,y1),(z0,z1,w0,w1)
   __shared__ Src stage[NW][MIXED ? 2 * Q2 : Q];
@@ -503,7 +503,7 @@ __device__ __forceinline__ void interact_wide_body(const StepGeom& g, int tix, i
         az[r] += (double)fz[r].x + (double)fz[r].y;
       }
     } else {
-#pragma unroll 3
+#pragma unroll kRow
       for (int k = 0; k < Q; k++) {
         const double4 s = stage[warp][k];
         pairs64<GUARD>(tx, ty, tz, s.x, s.y, s.z, s.w, eps2, ax, ay, az);
@@ -1154,7 +1154,7 @@ void interact_qg(const StepGeom& g, int precision, const double4* src, double* o
   } else {
     if (precision == SBSLPM_MIXED) {
       constexpr int NW = dev::ListShape32<Q, 1>::NW, threads = 32 * NW;
-      const int wpt = dev::list_warps<Q, 1>(tp);
+      const int wpt = dev::list_warps<Q, 1, true>(tp);
       if (pack) SB_LAUNCH(k_pack_mixed, blocks_for((long)g.panels * g.q, 256), 256, 0, st, g, src, g.srcf);
       if (all_leaves)
         SB_LAUNCH((k_interact32<Q, 1, true, GUARD>), dim3(blocks_for(tp, NW), groups), threads, 0, st, g, g.srcf, out,
@@ -1167,7 +1167,7 @@ void interact_qg(const StepGeom& g, int precision, const double4* src, double* o
         SB_LAUNCH((k_interact32<Q, 1, false, GUARD>), blocks_for(tp, NW), threads, 0, st, g, g.srcf, out, out_stride);
     } else {
       constexpr int NW = dev::ListShape<Q, 1>::NW, threads64 = 32 * NW;
-      const int wpt = dev::list_warps<Q, 1>(tp);
+      const int wpt = dev::list_warps<Q, 1, false>(tp);
       if (all_leaves)
         SB_LAUNCH((k_interact64<Q, 1, true, GUARD>), dim3(blocks_for(tp, NW), groups), threads64, 0, st, g, src, out,
                   out_stride);

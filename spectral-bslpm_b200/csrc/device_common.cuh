@@ -213,6 +213,14 @@ __device__ __forceinline__ void store_packed(float4* srcf, int q, long panel, in
   store_packed_w(srcf, q, panel, j, (float)w);
 }
 
+// Nodes per direction of a panel of q = n^2 nodes: the length to which loops
+// over a panel of more than 25 sources are unrolled (whole rounds at any q).
+constexpr int row_of(int q) {
+  int n = 1;
+  while (n * n < q) n++;
+  return n;
+}
+
 // First panel id of the k-th level below the subtree root (level, root_rel).
 __device__ __forceinline__ int subtree_first(int level, int root_rel, int k) {
   return level_start(level + k) + (root_rel << (2 * k));

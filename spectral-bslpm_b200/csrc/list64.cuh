@@ -47,15 +47,23 @@ struct ListShape {
 
 // Warps per target panel: a whole block while the tree has fewer panels than
 // 16 warps per SM would take, else two (lists are then short enough for the
-// splits of two warps), one where a warp alone already splits the list ten
-// ways or more.  BVE step, degree 3, theta 0.7, us per step at 1 / 2 / 4 warps:
-// levels 3 198 / 180 / 172, levels 5 269 / 251 / 247, levels 7 1625 / 1605 /
-// 1649; degree 2, levels 6: 353 / 361 / 376.
-template <int Q, int FIELDS>
+// splits of two warps).  BVE step, degree 3, theta 0.7, us per step at 1 / 2 / 4
+// warps: levels 3 198 / 180 / 172, levels 5 269 / 251 / 247, levels 7 1625 /
+// 1605 / 1649.  Where one warp alone splits the list ten ways or more, a list
+// of some 40 entries leaves the splits of more warps without any: list kernels
+// of a step, us at 1 / 2 / 4 warps, theta 0.7, q = 9 at levels 4 41 / 30 / 27
+// (float64), 21 / 19 / 19 (mixed), levels 5 61 / 59 / 62, 35 / 40 / 50, levels 6
+// 168 / 168 / 197, 100 / 119 / 166; q = 4 levels 3 16 / 14 / 12, levels 5 26 /
+// 24 / 34, 20 / 24 / 37; q = 1 levels 3 10 / 10 / 12, levels 5 15 / 18 / 28.
+template <int Q, int FIELDS, bool MIXED>
 inline int list_warps(int target_panels) {
   using W = ListShape<Q, FIELDS>;
-  if (target_panels <= 148 * 16) return W::NW;
-  return W::S >= 10 ? 1 : 2;
+  constexpr int NW = MIXED ? 4 : W::NW;
+  const bool few = target_panels <= 148 * 4, some = target_panels <= 148 * 16;
+  if (W::S >= 32) return 1;
+  if (W::S >= 16) return few ? 2 : 1;
+  if (W::S >= 10) return few ? NW : some && !MIXED ? 2 : 1;
+  return some ? NW : 2;
 }
 
 __device__ __forceinline__ void copy_async16(void* dst, const void* src) {

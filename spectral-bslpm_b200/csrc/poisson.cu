@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(32 * dev::ListShape<Q, 1>::NW)
 template <int Q>
 void launch_poisson_q(const StepGeom& g, const double* table, const double* src, double* tgt, cudaStream_t st) {
   constexpr int NW = dev::ListShape<Q, 1>::NW, threads = 32 * NW;
-  const int wpt = dev::list_warps<Q, 1>(g.panels);
+  const int wpt = dev::list_warps<Q, 1, false>(g.panels);
   if (wpt == NW) SB_LAUNCH((k_poisson_interact<Q, NW>), g.panels, threads, 0, st, g, table, src, tgt);
   else if (wpt == 2) SB_LAUNCH((k_poisson_interact<Q, 2>), dev::blocks_for(g.panels, NW / 2), threads, 0, st, g, table, src, tgt);
   else SB_LAUNCH((k_poisson_interact<Q, 1>), dev::blocks_for(g.panels, NW), threads, 0, st, g, table, src, tgt);

@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(32 * kWarps)
   // mixed: the Q proxies as ceil(Q/2) source pairs of two float4
   // (x0,x1,y0,y1),(z0,z1,w0,w1), an odd Q closing on a zero-strength source
   // at the panel's centre (which adds exactly zero)
-  constexpr int HQ = (Q + 1) / 2;
+  constexpr int HQ = (Q + 1) / 2, kRow = row_of(Q);
   __shared__ Src stage[kWarps][2][MIXED ? 2 * HQ : Q];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tp_first = ALL_LEAVES ? g.offset : 0;
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(32 * kWarps)
           bz[r] += (double)(fb[r][2].x + fb[r][2].y);
         }
       } else {
-#pragma unroll 4
+#pragma unroll kRow
         for (int k = 0; k < Q; k++) {
           const double4 v1 = st1[k], v2 = st2[k];
           pairs64<GUARD>(tx, ty, tz, v1.x, v1.y, v1.z, v1.w, deps2, ax, ay, az);
@@ -449,11 +449,11 @@ void swe_interact_qg(const StepGeom& g, const SweGeom& s, int precision, const d
   if constexpr (Q <= 32) {
     if (mixed) {
       constexpr int NW = ListShape32<Q, 2>::NW, threads = 32 * NW;
-      const int wpt = dev::list_warps<Q, 2>(tp);
+      const int wpt = dev::list_warps<Q, 2, true>(tp);
       if (all_leaves)
         SB_LAUNCH((k_swe_interact32<Q, 1, true, GUARD>), dim3(blocks_for(tp, NW), groups), threads, 0, st, g, s, out,
                   out_stride);
-      else if (tp <= 148 * 16)
+      else if (wpt == NW)
         SB_LAUNCH((k_swe_interact32<Q, NW, false, GUARD>), tp, threads, 0, st, g, s, out, out_stride);
       else if (wpt == 2)
         SB_LAUNCH((k_swe_interact32<Q, 2, false, GUARD>), blocks_for(tp, NW / 2), threads, 0, st, g, s, out, out_stride);
@@ -462,7 +462,7 @@ void swe_interact_qg(const StepGeom& g, const SweGeom& s, int precision, const d
       return;
     }
     constexpr int NW = ListShape<Q, 2>::NW, threads = 32 * NW;
-    const int wpt = dev::list_warps<Q, 2>(tp);
+    const int wpt = dev::list_warps<Q, 2, false>(tp);
     if (all_leaves)
       SB_LAUNCH((k_swe_interact64<Q, 1, true, GUARD>), dim3(blocks_for(tp, NW), groups), threads, 0, st, g, src, src2,
                 out, out_stride);
