@@ -4,8 +4,9 @@
 //   src   : double4 [panels*q]  displaced source position (x, y, z) and
 //           strength w = area * vorticity (leaves) or its anterpolation
 //           (non-leaf proxies).  32 B per proxy point, one load per pair block.
-//   srcf  : float4  [panels*q]  mixed precision: position relative to the
-//           panel centre (float) and strength (float).
+//   srcf  : float4  [panels][packed_stride(q)]  mixed precision: position
+//           relative to the panel centre (float) and strength (float), up to
+//           25 sources two by two (store_packed_xyz).
 //   tgt   : double  [3][panels*q] proxy-target velocities.
 //   v_k   : double  [3][leaves*q] stage velocities (x, y, z blocks).
 // Every kernel is owner-computes (no atomics), so results are deterministic.
@@ -352,34 +353,30 @@ __global__ void k_downward_subtree_batch(const BatchMember* __restrict__ mem, in
 // ---------------------------------------------------------------------------
 // Interactions (bve_vel_panel_interaction, src/fmm_interactions/bve_vel_impl.hpp:85-122).
 //
-// One warp owns one target panel and walks its sources (CSR list, or all
-// leaves in direct mode).  For q <= 16 the warp's lanes are (split h,
-// target node j): split h takes every S-th source panel, stages its q
-// points in shared memory and every lane of the split runs over them.  For
-// q > 32 each lane owns ceil(q/32) target nodes and the whole warp stages
-// one source panel at a time.  Partial sums of the splits are combined in a
-// fixed order, so the result is deterministic.
+// Panels of up to 25 points by list64.cuh and list32.cuh (a warp or more per
+// target panel, its lists split over the lanes); larger ones by four warps per
+// target panel (interact_wide_body).  Partial sums are combined in a fixed
+// order, so the result is deterministic.
 //
-// Direct mode (ALL_LEAVES) splits the source leaves into gridDim.y groups
-// and writes per-group partials that k_reduce_groups sums in order.
+// Direct velocity: in float64, and mixed for panels of few points, the
+// stand-alone direct sum's kernel over the leaf points; else every leaf against
+// every leaf (ALL_LEAVES), the source leaves split into gridDim.y groups whose
+// partials k_reduce_groups sums in order.
 
 // Float64, q <= 25 (list64.cuh).
-template <int Q, int WPT, bool ALL_LEAVES, bool GUARD>
+template <int Q, int WPT, bool GUARD>
 __global__ void __launch_bounds__(32 * ListShape<Q, 1>::NW)
-    k_interact64(StepGeom g, const double4* __restrict__ src, double* __restrict__ out, long out_stride) {
+    k_interact64(StepGeom g, const double4* __restrict__ src, double* __restrict__ out) {
   using W = ListShape<Q, 1>;
   __shared__ __align__(16) double2 tiles[W::NW * W::WARP];
   const long pn = (long)g.panels * Q;
-  list64_sweep<Q, 1, WPT, ALL_LEAVES, GUARD>(
-      g, src, nullptr, tiles, [&](int t, int tix, int j, const double* a) {
-        const long i = (long)t * Q + j;
-        const double x = g.px[i], y = g.px[pn + i], z = g.px[2 * pn + i];
-        const long o = ALL_LEAVES ? (long)blockIdx.y * 3 * out_stride + (long)tix * Q + j : i;
-        const long s = ALL_LEAVES ? out_stride : pn;
-        out[o] = kBiotSavartTwice * (y * a[2] - z * a[1]);
-        out[s + o] = kBiotSavartTwice * (z * a[0] - x * a[2]);
-        out[2 * s + o] = kBiotSavartTwice * (x * a[1] - y * a[0]);
-      });
+  list64_sweep<Q, 1, WPT, false, GUARD>(g, src, nullptr, tiles, [&](int t, int, int j, const double* a) {
+    const long i = (long)t * Q + j;
+    const double x = g.px[i], y = g.px[pn + i], z = g.px[2 * pn + i];
+    out[i] = kBiotSavartTwice * (y * a[2] - z * a[1]);
+    out[pn + i] = kBiotSavartTwice * (z * a[0] - x * a[2]);
+    out[2 * pn + i] = kBiotSavartTwice * (x * a[1] - y * a[0]);
+  });
 }
 
 // Mixed precision: positions relative to panel centres in float, pair
@@ -771,12 +768,28 @@ constexpr double kPlainEps = 1e-100, kPlainStrength = 1e200;
 constexpr int kDirectTile64 = 64;
 constexpr size_t direct_smem64(int parts) { return sizeof(double) * (parts * (128 + 3 * kDirectTile64) + 3 * kDirectTile64); }
 
-template <bool GUARD>
+// The sources of a direct sum: four arrays of a caller, or a grid's sources.
+struct SourceArrays {
+  const double *x, *y, *z, *w;
+  __device__ __forceinline__ void get(long k, double2& a, double2& b) const {
+    a = make_double2(__ldg(x + k), __ldg(y + k));
+    b = make_double2(__ldg(z + k), __ldg(w + k));
+  }
+};
+struct SourceRecords {
+  const double4* s;
+  __device__ __forceinline__ void get(long k, double2& a, double2& b) const {
+    const double2* p = reinterpret_cast<const double2*>(s + k);
+    a = __ldg(p);
+    b = __ldg(p + 1);
+  }
+};
+
+template <bool GUARD, class Sources>
 __global__ void __launch_bounds__(kDirectThreads, 4)
     k_direct_bve64(long nt, const double* __restrict__ tx, const double* __restrict__ ty,
-                   const double* __restrict__ tz, long ns, const double* __restrict__ sx,
-                   const double* __restrict__ sy, const double* __restrict__ sz, const double* __restrict__ sw,
-                   long per, double eps, double* __restrict__ ux, double* __restrict__ uy, double* __restrict__ uz) {
+                   const double* __restrict__ tz, long ns, Sources sources, long per, double eps,
+                   double* __restrict__ ux, double* __restrict__ uy, double* __restrict__ uz) {
   constexpr int TPT = 2, TB = 32 * TPT;
   static_assert(TB == kDirectTile64, "direct_smem64");
   extern __shared__ __align__(16) double dsh[];  // a tile of 32 sources per warp, partial sums, the block's sums
@@ -796,10 +809,7 @@ __global__ void __launch_bounds__(kDirectThreads, 4)
   const long s0 = (blockIdx.y * parts + warp) * per, s1 = min(ns, s0 + per);
   double2 a = make_double2(0, 0), b = a;
   auto load = [&](long k) {
-    if (k < s1) {
-      a = make_double2(sx[k], sy[k]);
-      b = make_double2(sz[k], sw[k]);
-    }
+    if (k < s1) sources.get(k, a, b);
   };
   load(s0 + lane);
   for (long k = s0; k < s1; k += 32) {
@@ -1134,72 +1144,75 @@ void launch_downward_fused(const StepGeom& g, double* tgt, double* leaf_out, cud
 
 namespace {
 template <int Q, bool GUARD>
-void interact_qg(const StepGeom& g, int precision, const double4* src, double* out, bool all_leaves, int groups,
-                 long out_stride, cudaStream_t st, bool pack) {
-  int tp = all_leaves ? g.leaves : g.panels;
+void interact_qg(const StepGeom& g, int precision, const double4* src, double* out, cudaStream_t st, bool pack) {
+  const int tp = g.panels;
+  if (precision == SBSLPM_MIXED && pack)
+    SB_LAUNCH(k_pack_mixed, blocks_for((long)g.panels * g.q, 256), 256, 0, st, g, src, g.srcf);
   if constexpr (Q > 32) {
-    dim3 wgrid((unsigned)tp, all_leaves ? groups : 1);
-    const bool mixed = precision == SBSLPM_MIXED;
-    if (mixed && pack) {
-      long pn = (long)g.panels * g.q;
-      SB_LAUNCH(k_pack_mixed, blocks_for(pn, 256), 256, 0, st, g, src, g.srcf);
-    }
-    if (mixed) {
-      if (all_leaves) SB_LAUNCH((k_interact_wide<Q, true, GUARD, true>), wgrid, 128, 0, st, g, src, g.srcf, out, out_stride);
-      else SB_LAUNCH((k_interact_wide<Q, false, GUARD, true>), wgrid, 128, 0, st, g, src, g.srcf, out, out_stride);
-    } else {
-      if (all_leaves) SB_LAUNCH((k_interact_wide<Q, true, GUARD, false>), wgrid, 128, 0, st, g, src, g.srcf, out, out_stride);
-      else SB_LAUNCH((k_interact_wide<Q, false, GUARD, false>), wgrid, 128, 0, st, g, src, g.srcf, out, out_stride);
-    }
+    if (precision == SBSLPM_MIXED)
+      SB_LAUNCH((k_interact_wide<Q, false, GUARD, true>), tp, 128, 0, st, g, src, g.srcf, out, 0L);
+    else
+      SB_LAUNCH((k_interact_wide<Q, false, GUARD, false>), tp, 128, 0, st, g, src, g.srcf, out, 0L);
+  } else if (precision == SBSLPM_MIXED) {
+    constexpr int NW = dev::ListShape32<Q, 1>::NW, threads = 32 * NW;
+    const int wpt = dev::list_warps<Q, 1, true>(tp);
+    if (wpt == NW)
+      SB_LAUNCH((k_interact32<Q, NW, false, GUARD>), tp, threads, 0, st, g, g.srcf, out, 0L);
+    else if (wpt == 2)
+      SB_LAUNCH((k_interact32<Q, 2, false, GUARD>), blocks_for(tp, NW / 2), threads, 0, st, g, g.srcf, out, 0L);
+    else
+      SB_LAUNCH((k_interact32<Q, 1, false, GUARD>), blocks_for(tp, NW), threads, 0, st, g, g.srcf, out, 0L);
   } else {
-    if (precision == SBSLPM_MIXED) {
-      constexpr int NW = dev::ListShape32<Q, 1>::NW, threads = 32 * NW;
-      const int wpt = dev::list_warps<Q, 1, true>(tp);
-      if (pack) SB_LAUNCH(k_pack_mixed, blocks_for((long)g.panels * g.q, 256), 256, 0, st, g, src, g.srcf);
-      if (all_leaves)
-        SB_LAUNCH((k_interact32<Q, 1, true, GUARD>), dim3(blocks_for(tp, NW), groups), threads, 0, st, g, g.srcf, out,
-                  out_stride);
-      else if (wpt == NW)
-        SB_LAUNCH((k_interact32<Q, NW, false, GUARD>), tp, threads, 0, st, g, g.srcf, out, out_stride);
-      else if (wpt == 2)
-        SB_LAUNCH((k_interact32<Q, 2, false, GUARD>), blocks_for(tp, NW / 2), threads, 0, st, g, g.srcf, out, out_stride);
-      else
-        SB_LAUNCH((k_interact32<Q, 1, false, GUARD>), blocks_for(tp, NW), threads, 0, st, g, g.srcf, out, out_stride);
-    } else {
-      constexpr int NW = dev::ListShape<Q, 1>::NW, threads64 = 32 * NW;
-      const int wpt = dev::list_warps<Q, 1, false>(tp);
-      if (all_leaves)
-        SB_LAUNCH((k_interact64<Q, 1, true, GUARD>), dim3(blocks_for(tp, NW), groups), threads64, 0, st, g, src, out,
-                  out_stride);
-      else if (wpt == NW)
-        SB_LAUNCH((k_interact64<Q, NW, false, GUARD>), tp, threads64, 0, st, g, src, out, out_stride);
-      else if (wpt == 2)
-        SB_LAUNCH((k_interact64<Q, 2, false, GUARD>), blocks_for(tp, NW / 2), threads64, 0, st, g, src, out, out_stride);
-      else
-        SB_LAUNCH((k_interact64<Q, 1, false, GUARD>), blocks_for(tp, NW), threads64, 0, st, g, src, out, out_stride);
-    }
+    constexpr int NW = dev::ListShape<Q, 1>::NW, threads = 32 * NW;
+    const int wpt = dev::list_warps<Q, 1, false>(tp);
+    if (wpt == NW)
+      SB_LAUNCH((k_interact64<Q, NW, GUARD>), tp, threads, 0, st, g, src, out);
+    else if (wpt == 2)
+      SB_LAUNCH((k_interact64<Q, 2, GUARD>), blocks_for(tp, NW / 2), threads, 0, st, g, src, out);
+    else
+      SB_LAUNCH((k_interact64<Q, 1, GUARD>), blocks_for(tp, NW), threads, 0, st, g, src, out);
+  }
+}
+
+// Every leaf against every leaf, mixed precision, `groups` groups of source
+// leaves whose partial sums go to out [group][3][leaves*q].
+template <int Q, bool GUARD>
+void leaves_qg(const StepGeom& g, double* out, int groups, cudaStream_t st) {
+  const long n = (long)g.leaves * Q;
+  if constexpr (Q > 32) {
+    SB_LAUNCH((k_interact_wide<Q, true, GUARD, true>), dim3((unsigned)g.leaves, groups), 128, 0, st, g, nullptr, g.srcf,
+              out, n);
+  } else {
+    constexpr int NW = dev::ListShape32<Q, 1>::NW;
+    SB_LAUNCH((k_interact32<Q, 1, true, GUARD>), dim3(blocks_for(g.leaves, NW), groups), 32 * NW, 0, st, g, g.srcf, out,
+              n);
   }
 }
 
 // The coincident-point guard is compiled in only when kernel_eps = 0.
-template <int Q>
-void interact_q(const StepGeom& g, int precision, const double4* src, double* out, bool, bool all_leaves,
-                int groups, long out_stride, cudaStream_t st, bool pack = true) {
-  if (g.eps > 0)
-    interact_qg<Q, false>(g, precision, src, out, all_leaves, groups, out_stride, st, pack);
-  else
-    interact_qg<Q, true>(g, precision, src, out, all_leaves, groups, out_stride, st, pack);
-}
-
-void interact_dispatch(const StepGeom& g, int precision, const double4* src, double* out, bool accumulate,
-                       bool all_leaves, int groups, long out_stride, cudaStream_t st, bool pack = true) {
-#define SB_IQ(Q) \
-  case Q: interact_q<Q>(g, precision, src, out, accumulate, all_leaves, groups, out_stride, st, pack); break;
+void interact_dispatch(const StepGeom& g, int precision, const double4* src, double* out, cudaStream_t st,
+                       bool pack) {
+#define SB_IQ(Q)                                                             \
+  case Q:                                                                    \
+    if (g.eps > 0) interact_qg<Q, false>(g, precision, src, out, st, pack);  \
+    else interact_qg<Q, true>(g, precision, src, out, st, pack);             \
+    break;
   switch (g.q) {
-    SB_IQ(1) SB_IQ(4) SB_IQ(9) SB_IQ(16) SB_IQ(25) SB_IQ(36) SB_IQ(49) SB_IQ(64) SB_IQ(81) SB_IQ(100)
-    default: interact_q<121>(g, precision, src, out, accumulate, all_leaves, groups, out_stride, st, pack); break;
+    SB_IQ(1) SB_IQ(4) SB_IQ(9) SB_IQ(16) SB_IQ(25) SB_IQ(36) SB_IQ(49) SB_IQ(64) SB_IQ(81) SB_IQ(100) SB_IQ(121)
   }
 #undef SB_IQ
+}
+
+void leaves_dispatch(const StepGeom& g, double* out, int groups, cudaStream_t st) {
+#define SB_LQ(Q)                                                 \
+  case Q:                                                        \
+    if (g.eps > 0) leaves_qg<Q, false>(g, out, groups, st);      \
+    else leaves_qg<Q, true>(g, out, groups, st);                 \
+    break;
+  switch (g.q) {
+    SB_LQ(16) SB_LQ(25) SB_LQ(36) SB_LQ(49) SB_LQ(64) SB_LQ(81) SB_LQ(100) SB_LQ(121)
+  }
+#undef SB_LQ
 }
 
 // Independent FMA chains (8 per thread) so the pipe, not latency, limits throughput.
@@ -1229,11 +1242,11 @@ __global__ void k_fma_probe64(int iters, double* out) {
 
 void launch_interactions(const StepGeom& g, int precision, const double4* src, double* tgt, bool accumulate,
                          cudaStream_t st) {
-  interact_dispatch(g, precision, src, tgt, accumulate, false, 1, 0, st);
+  interact_dispatch(g, precision, src, tgt, st, true);
 }
 
 void launch_interactions_only(const StepGeom& g, int precision, const double4* src, double* tgt, cudaStream_t st) {
-  interact_dispatch(g, precision, src, tgt, false, false, 1, 0, st, false);
+  interact_dispatch(g, precision, src, tgt, st, false);
 }
 
 void launch_pack_mixed(const StepGeom& g, const double4* src, cudaStream_t st) {
@@ -1246,13 +1259,6 @@ void launch_fma_probe(int kind, int blocks, int iters, float* out32, double* out
     SB_LAUNCH(k_fma_probe32, blocks, 256, 0, st, iters, out32);
   else
     SB_LAUNCH(k_fma_probe64, blocks, 256, 0, st, iters, out64);
-}
-
-void launch_direct_leaves(const StepGeom& g, int precision, const double4* src, double* vout, double* partial,
-                          int groups, cudaStream_t st) {
-  long n = (long)g.leaves * g.q;
-  interact_dispatch(g, precision, src, partial, false, true, groups, n, st);
-  SB_LAUNCH(k_reduce_groups, blocks_for(3 * n, 256), 256, 0, st, partial, groups, 3 * n, 3 * n, vout);
 }
 
 static bool aligned16(std::initializer_list<const double*> ps) {
@@ -1353,23 +1359,63 @@ static DirectShape direct_shape(long target_tiles, long source_tiles, long want,
   return {parts, shares / parts};
 }
 
+constexpr long kDirectWaves = 16L * 148;  // of 32 warps (float64) or 16 64-thread groups per SM
+
+template <class Sources>
+static void launch_direct64(long nt, const double* tx, const double* ty, const double* tz, long ns,
+                            const Sources& sources, double eps, double* ux, double* uy, double* uz, cudaStream_t st) {
+  const unsigned blocks = blocks_for(nt, kDirectTile64);
+  const DirectShape d = direct_shape(blocks, (ns + 31) / 32, 32 * kDirectWaves, kDirectThreads / 32);
+  const long per = (ns + d.parts * d.ranks - 1) / (d.parts * d.ranks);  // sources of a warp
+  launch_cluster(eps >= kPlainEps ? k_direct_bve64<false, Sources> : k_direct_bve64<true, Sources>, blocks, d.ranks,
+                 32 * d.parts, direct_smem64(d.parts), st, nt, tx, ty, tz, ns, sources, per, eps, ux, uy, uz);
+}
+
 void launch_direct_bve(long nt, const double* tx, const double* ty, const double* tz, long ns, const double* sx,
                        const double* sy, const double* sz, const double* s, double eps, int precision, int groups,
                        double* ux, double* uy, double* uz, cudaStream_t st) {
-  const long waves = 16L * 148;  // of 32 warps (float64) or 16 64-thread groups per SM
   if (precision == SBSLPM_MIXED) {
     const unsigned blocks = blocks_for(nt, kDirectTile32);
     const long per = (ns + groups - 1) / groups, units = groups * ((per + kDirectTile32 - 1) / kDirectTile32);
-    const DirectShape d = direct_shape(blocks, units, 16 * waves, kDirectThreads / kDirectPart32);
+    const DirectShape d = direct_shape(blocks, units, 16 * kDirectWaves, kDirectThreads / kDirectPart32);
     launch_cluster(k_direct_bve32, blocks, d.ranks, d.parts * kDirectPart32, direct_smem32(d.parts), st, nt, tx, ty, tz,
                    ns, sx, sy, sz, s, groups, eps, ux, uy, uz);
     return;
   }
-  const unsigned blocks = blocks_for(nt, kDirectTile64);
-  const DirectShape d = direct_shape(blocks, (ns + 31) / 32, 32 * waves, kDirectThreads / 32);
-  const long per = (ns + d.parts * d.ranks - 1) / (d.parts * d.ranks);  // sources of a warp
-  launch_cluster(eps >= kPlainEps ? k_direct_bve64<false> : k_direct_bve64<true>, blocks, d.ranks, 32 * d.parts,
-                 direct_smem64(d.parts), st, nt, tx, ty, tz, ns, sx, sy, sz, s, per, eps, ux, uy, uz);
+  launch_direct64(nt, tx, ty, tz, ns, SourceArrays{sx, sy, sz, s}, eps, ux, uy, uz, st);
+}
+
+// Source groups of a grid's direct sum by panels: blocks of four warps for
+// about 12 per SM, no fewer leaves in a group than a warp has source splits (a
+// warp's rounds are then full).  us of a step's sums with 64 * 148 / leaves
+// groups and with this rule: shallow water, q = 9 at levels 3 77 / 41, q = 16 74
+// / 45, q = 25 189 / 83 (float64), 70 / 36, 60 / 35, 84 / 57 (mixed).
+int direct_leaf_groups(int leaves, int q) {
+  const int most = 64;
+  if (q > 25) return std::max(1, std::min(most, 148 * 64 / leaves));
+  const int splits = q <= 1 ? ListShape<1, 1>::S : q <= 4 ? ListShape<4, 1>::S : q <= 9 ? ListShape<9, 1>::S
+                     : q <= 16 ? ListShape<16, 1>::S : ListShape<25, 1>::S;
+  const int want = std::max(1, std::min(most, 148 * 48 / leaves)), per = (leaves + want - 1) / want;
+  const int full = (per + splits - 1) / splits * splits;
+  return (leaves + full - 1) / full;
+}
+
+// The grid's direct velocity.  In float64, and mixed up to nine points a panel,
+// as a direct sum over points (mixed pairs need a panel's common centre, which
+// costs more than they save on few points); else by panels, in source groups.
+// us per step by panels / by points, float64 at levels 5, 4 points a panel 475 /
+// 185, levels 4, 9 points 154 / 96, 49 points 1,710 / 1,323.
+void launch_direct_leaves(const StepGeom& g, int precision, const double4* src, double* vout, double* partial,
+                          int groups, cudaStream_t st) {
+  const long n = (long)g.leaves * g.q, pn = (long)g.panels * g.q, off = (long)g.offset * g.q;
+  if (precision != SBSLPM_MIXED || g.q <= 9) {
+    launch_direct64(n, g.px + off, g.px + pn + off, g.px + 2 * pn + off, n, SourceRecords{src + off}, g.eps, vout,
+                    vout + n, vout + 2 * n, st);
+    return;
+  }
+  launch_pack_mixed(g, src, st);
+  leaves_dispatch(g, partial, groups, st);
+  SB_LAUNCH(k_reduce_groups, blocks_for(3 * n, 256), 256, 0, st, partial, groups, 3 * n, 3 * n, vout);
 }
 
 void launch_ssw_forcing(int leaves, int q, int type, double omega, const double* time, const double* x,

@@ -118,6 +118,7 @@ void launch_sources_from_disp(const StepGeom& g, const double* dx, const double*
                               const double* source, double4* src, cudaStream_t st);
 void launch_copy_strength(const StepGeom& g, const double4* src, double* out, cudaStream_t st);
 
+int direct_leaf_groups(int leaves, int q);
 // Stand-alone direct sums (no tree).
 int direct_groups(long n_targets, long n_sources);
 void launch_direct_bve(long nt, const double* tx, const double* ty, const double* tz, long ns, const double* sx,

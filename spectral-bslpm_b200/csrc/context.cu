@@ -250,8 +250,7 @@ sbslpm_status allocate_workspace(sbslpm_ctx* c) {
   SB_TRY(dalloc(&c->newvor, ln));
   if (c->cfg.tracer_count > 0) SB_TRY(dalloc(&c->newtr, ln * c->cfg.tracer_count));
   if (c->cfg.velocity == SBSLPM_VEL_DIRECT) {
-    long g = (148L * 64) / c->A;
-    c->groups = (int)(g < 1 ? 1 : (g > 64 ? 64 : g));
+    c->groups = direct_leaf_groups(c->A, c->q);
     SB_TRY(dalloc(&c->partial, (size_t)c->groups * 3 * ln));
   }
   SB_TRY(alloc_error_word(&c->err, &c->h_err));

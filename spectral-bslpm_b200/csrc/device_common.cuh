@@ -213,8 +213,11 @@ __device__ __forceinline__ void store_packed(float4* srcf, int q, long panel, in
   store_packed_w(srcf, q, panel, j, (float)w);
 }
 
-// Nodes per direction of a panel of q = n^2 nodes: the length to which loops
-// over a panel of more than 25 sources are unrolled (whole rounds at any q).
+// Nodes per direction of a panel of q = n^2 nodes: the length to which float64
+// loops over a panel of more than 25 sources are unrolled (whole rounds at any
+// q).  Three or four sources, with remainders, hid too little latency where a
+// tree has few panels: lists of a step at levels 3, us, 49 points 190 / 147, 64
+// 239 / 184, 100 461 / 382; two fields of 36 points at levels 4 1,006 / 706.
 constexpr int row_of(int q) {
   int n = 1;
   while (n * n < q) n++;

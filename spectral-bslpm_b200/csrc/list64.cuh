@@ -1,6 +1,6 @@
 // Float64 proxy interactions over a target panel's list of source panels
-// (CSR list, or every leaf of a group), for one source field (BVE) or two
-// (shallow water), q <= 25.
+// (CSR list, or, for the shallow-water direct velocity, every leaf of a group),
+// for one source field (BVE) or two (shallow water), q <= 25.
 //
 // The FP64 pipe bounds the pairs (13 operations each; about 1.2e12 pairs/s
 // with the operands that a pair reads from registers).  What kept the kernels
