@@ -1388,8 +1388,8 @@ void launch_direct_bve(long nt, const double* tx, const double* ty, const double
 // Source groups of a grid's direct sum by panels: blocks of four warps for
 // about 12 per SM, no fewer leaves in a group than a warp has source splits (a
 // warp's rounds are then full).  us of a step's sums with 64 * 148 / leaves
-// groups and with this rule: shallow water, q = 9 at levels 3 77 / 41, q = 16 74
-// / 45, q = 25 189 / 83 (float64), 70 / 36, 60 / 35, 84 / 57 (mixed).
+// groups and with this rule: shallow water, q = 9 at levels 3 77 / 37, q = 16 74
+// / 44, q = 25 189 / 83 (float64), 70 / 34, 60 / 35, 84 / 57 (mixed).
 int direct_leaf_groups(int leaves, int q) {
   const int most = 64;
   if (q > 25) return std::max(1, std::min(most, 148 * 64 / leaves));
@@ -1403,8 +1403,8 @@ int direct_leaf_groups(int leaves, int q) {
 // The grid's direct velocity.  In float64, and mixed up to nine points a panel,
 // as a direct sum over points (mixed pairs need a panel's common centre, which
 // costs more than they save on few points); else by panels, in source groups.
-// us per step by panels / by points, float64 at levels 5, 4 points a panel 475 /
-// 185, levels 4, 9 points 154 / 96, 49 points 1,710 / 1,323.
+// us per step by panels, one target per lane / by points, float64 at levels 5, 4
+// points a panel 471 / 185, levels 4, 9 points 132 / 96, 49 points 1,865 / 1,323.
 void launch_direct_leaves(const StepGeom& g, int precision, const double4* src, double* vout, double* partial,
                           int groups, cudaStream_t st) {
   const long n = (long)g.leaves * g.q, pn = (long)g.panels * g.q, off = (long)g.offset * g.q;
