@@ -1386,16 +1386,18 @@ void launch_direct_bve(long nt, const double* tx, const double* ty, const double
 }
 
 // Source groups of a grid's direct sum by panels: blocks of four warps for
-// about 12 per SM, no fewer leaves in a group than a warp has source splits (a
-// warp's rounds are then full).  us of a step's sums with 64 * 148 / leaves
-// groups and with this rule: shallow water, q = 9 at levels 3 77 / 37, q = 16 74
-// / 44, q = 25 189 / 83 (float64), 70 / 34, 60 / 35, 84 / 57 (mixed).
+// about 10 per SM and six groups at least (short last rounds on large grids),
+// each a whole number of a warp's source splits (its rounds are then full).  us
+// of a step's sums with 64 * 148 / leaves groups and with this rule: shallow
+// water at levels 3, 9 points a panel 77 / 37, 16 74 / 44, 25 189 / 83
+// (float64), 70 / 34, 60 / 35, 84 / 57 (mixed); mixed velocity, 16 points at
+// levels 5 1,183 / 1,183, levels 6 19,160 / 17,290.
 int direct_leaf_groups(int leaves, int q) {
   const int most = 64;
   if (q > 25) return std::max(1, std::min(most, 148 * 64 / leaves));
   const int splits = q <= 1 ? ListShape<1, 1>::S : q <= 4 ? ListShape<4, 1>::S : q <= 9 ? ListShape<9, 1>::S
                      : q <= 16 ? ListShape<16, 1>::S : ListShape<25, 1>::S;
-  const int want = std::max(1, std::min(most, 148 * 48 / leaves)), per = (leaves + want - 1) / want;
+  const int want = std::max(6, std::min(most, 148 * 40 / leaves)), per = (leaves + want - 1) / want;
   const int full = (per + splits - 1) / splits * splits;
   return (leaves + full - 1) / full;
 }

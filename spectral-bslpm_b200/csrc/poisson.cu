@@ -24,8 +24,9 @@ constexpr double kInvLapConst = -0.07957747154594767;  // -1/(4 pi), as the refe
 // splits' source panels brought in by cp.async one ahead, partial sums added
 // in a fixed order.  One block of 128 threads per panel, a thread per node,
 // left 112 of them idle at 16 nodes: 98,304 points, theta 0.7, 922 us; this
-// organisation 310 us with CUDA's log, 207 us with table_log, bound by the
-// FP64 pipe (about 25 operations a pair).
+// organisation 310 us with CUDA's log, 207 us with table_log (about 25 FP64
+// operations a pair): the FP64 pipe is 54% busy, and what holds the warps is
+// the table's reads from shared memory (45% of their stalled cycles).
 template <int Q, int WPT>
 __global__ void __launch_bounds__(32 * dev::ListShape<Q, 1>::NW)
     k_poisson_interact(StepGeom g, const double* __restrict__ table, const double* __restrict__ src,
