@@ -910,7 +910,7 @@ def direct_sum_bve(tx, ty, tz, sx, sy, sz, strength, eps, precision=FP64, out=No
 
 def direct_sum_bve_noalloc(tx, ty, tz, sx, sy, sz, strength, eps, precision=FP64, out=None):
     """direct_sum_bve through the entry point that allocates no device memory
-    (fixed scratch inside the library; at most 699,050 targets)."""
+    (at most 699,050 targets)."""
     import torch
 
     nt, ns = tx.numel(), sx.numel()
