@@ -45,7 +45,9 @@ enum { SBSLPM_VEL_FMM = 0, SBSLPM_VEL_DIRECT = 1 };
 /* Arithmetic of the pair kernels.  FP64: everything in float64.  MIXED: the
  * pair kernels evaluate in float32 on panel-relative coordinates and
  * accumulate per source panel in float32, then in float64; positions,
- * projections, BLI weights, the RK4 update and the remap stay float64. */
+ * projections, BLI weights, the RK4 update and the remap stay float64, and so
+ * do the pairs of the BVE's direct velocity on panels of at most nine points
+ * (interp_degree <= 2), where float32 is slower. */
 enum { SBSLPM_FP64 = 0, SBSLPM_MIXED = 1 };
 
 /* Mirrors the hot-path fields of the reference's RunConfig
